@@ -373,7 +373,7 @@ KoszulCtx::~KoszulCtx() {
     i8_destroy();
     for (auto& g : graphs)
         if (g) cudaGraphExecDestroy(g);
-    for (void* p : allocations) cudaFree(p);
+    for (auto& a : allocations) cudaFree(a.first);
     if (ev_join) cudaEventDestroy(ev_join);
     if (own_stream) cudaStreamDestroy(own_stream);
 }
@@ -383,7 +383,7 @@ T* KoszulCtx::alloc(uint64_t count) {
     void* p = nullptr;
     const uint64_t bytes = std::max<uint64_t>(count, 1) * sizeof(T);
     BW_CUDA(cudaMalloc(&p, bytes));
-    allocations.push_back(p);
+    allocations.emplace_back(p, bytes);
     device_bytes += bytes;
     return static_cast<T*>(p);
 }
@@ -484,21 +484,26 @@ KoszulCtx* KoszulCtx::create(const bw_koszul_desc& d, int dev) {
                 coef_fwd[(static_cast<size_t>(i) * c->ci + b) * c->co8 + cc] = bal;
                 coef_bwd[(static_cast<size_t>(i) * c->co + cc) * c->ci8 + b] = bal;
             }
-    std::vector<uint32_t> fwd, bwd;
-    build_tables(c->r, c->k, fwd, bwd);
-
     cudaStream_t st = c->own_stream;
-    c->d_coef_fwd = c->alloc<int32_t>(coef_fwd.size());
-    c->d_coef_bwd = c->alloc<int32_t>(coef_bwd.size());
-    c->d_fwd = c->alloc<uint32_t>(fwd.size());
-    c->d_bwd = c->alloc<uint32_t>(bwd.size());
-    BW_CUDA(cudaMemcpyAsync(c->d_coef_fwd, coef_fwd.data(), coef_fwd.size() * 4, cudaMemcpyHostToDevice, st));
-    BW_CUDA(cudaMemcpyAsync(c->d_coef_bwd, coef_bwd.data(), coef_bwd.size() * 4, cudaMemcpyHostToDevice, st));
-    BW_CUDA(cudaMemcpyAsync(c->d_fwd, fwd.data(), fwd.size() * 4, cudaMemcpyHostToDevice, st));
-    BW_CUDA(cudaMemcpyAsync(c->d_bwd, bwd.data(), bwd.size() * 4, cudaMemcpyHostToDevice, st));
+    // plain form only (the INT8 form builds its own tables on the device)
+    std::vector<uint32_t> fwd, bwd;
+    if (c->form == BW_FORM_PLAIN) {
+        build_tables(c->r, c->k, fwd, bwd);
+        c->d_coef_fwd = c->alloc<int32_t>(coef_fwd.size());
+        c->d_coef_bwd = c->alloc<int32_t>(coef_bwd.size());
+        c->d_fwd = c->alloc<uint32_t>(fwd.size());
+        c->d_bwd = c->alloc<uint32_t>(bwd.size());
+        BW_CUDA(cudaMemcpyAsync(c->d_coef_fwd, coef_fwd.data(), coef_fwd.size() * 4, cudaMemcpyHostToDevice, st));
+        BW_CUDA(cudaMemcpyAsync(c->d_coef_bwd, coef_bwd.data(), coef_bwd.size() * 4, cudaMemcpyHostToDevice, st));
+        BW_CUDA(cudaMemcpyAsync(c->d_fwd, fwd.data(), fwd.size() * 4, cudaMemcpyHostToDevice, st));
+        BW_CUDA(cudaMemcpyAsync(c->d_bwd, bwd.data(), bwd.size() * 4, cudaMemcpyHostToDevice, st));
+    }
 
     c->d_diag = c->alloc<int32_t>(c->n_src);
     if (d.diag_on_device) {
+        // after everything issued on the legacy stream, where the caller may just have written the diagonal
+        BW_CUDA(cudaEventRecord(c->ev_join, cudaStreamLegacy));
+        BW_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
         c->launch_to_balanced(d.diag, c->d_diag, c->n_src, st);
     } else {
         uint32_t* tmp = c->alloc<uint32_t>(c->n_src);
@@ -609,9 +614,10 @@ template uint32_t* KoszulCtx::alloc<uint32_t>(uint64_t);
 template int4* KoszulCtx::alloc<int4>(uint64_t);
 
 void KoszulCtx::release(void* p) {
-    auto it = std::find(allocations.begin(), allocations.end(), p);
+    auto it = std::find_if(allocations.begin(), allocations.end(), [p](const auto& a) { return a.first == p; });
     if (it != allocations.end()) {
         cudaFree(p);
+        device_bytes -= it->second;
         allocations.erase(it);
     }
 }

@@ -6,6 +6,7 @@
 
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace bw {
@@ -24,7 +25,7 @@ struct KoszulCtx {
     // device state
     cudaStream_t own_stream = nullptr;
     cudaEvent_t ev_join = nullptr;     // orders NULL-stream calls with the legacy stream
-    std::vector<void*> allocations;
+    std::vector<std::pair<void*, uint64_t>> allocations;   // pointer, bytes
     uint64_t device_bytes = 0, scratch_bytes = 0;
     int32_t *d_coef_fwd = nullptr, *d_coef_bwd = nullptr;
     uint32_t *d_fwd = nullptr, *d_bwd = nullptr;

@@ -49,6 +49,8 @@
 // timeout the kernel records an error code, all roles wind down, in-flight
 // copies and MMAs are drained and TMEM is freed.
 #include "bw_koszul.cuh"
+#include "bw_koszul_i8_dev.cuh"
+#include "bw_koszul_i8_union.cuh"
 #include "tc_sm100.cuh"
 
 #include <cuda.h>   // CUtensorMap and cuTensorMapEncodeTiled's types (the function is reached through the runtime)
@@ -67,26 +69,8 @@ namespace bw {
 
 namespace {
 
-constexpr uint32_t kAbsent = 0xFFFFFFFFu;
 constexpr int kEpilogueWarps = 8;                 // hybrid kernel; per TMEM lane quadrant: kEpilogueWarps / 4
-
-// Warp roles of the cp.async gather kernel with PW producer warps: PW = 8
-// (eight epilogue warps, 17 in all) or PW = 16 (four epilogue warps, 21 in
-// all; more copy streams for the same register budget of 96 a thread).
-template <int PW>
-struct GatherWarps {
-    static_assert(PW == 8 || PW == 16, "8 or 16 producer warps");
-    static constexpr int producers = PW;
-    static constexpr int mma = PW;                        // allocates TMEM, issues the MMAs
-    static constexpr int epilogue0 = PW + 1;
-    static constexpr int epilogue = PW == 16 ? 4 : 8;     // per TMEM lane quadrant: epilogue / 4
-    static constexpr int threads = (PW + 1 + epilogue) * 32;
-};
-constexpr int kMaxSmem = 227 * 1024;
 constexpr int kMaxRowTable = 2048;    // bytes of the K'-row -> generator table
-
-// Plane index inside a four-plane block array.
-enum : int { PL_LO = 0, PL_HI = 1, PL_NLO = 2, PL_NHI = 3 };
 
 struct I8Dir {
     const int8_t* in[4];      // input planes lo, hi, -lo, -hi: [blk][h][inner][16]
@@ -118,30 +102,6 @@ struct I8Dir {
     uint32_t tx_full, tx_last;   // bytes a full / the last stage of a tile receives
 };
 
-// Position in a ring of pipeline slots: slot index and the parity of its
-// current phase, advanced without dividing (a 64-bit division per stage would
-// sit on the producers' and the MMA thread's critical paths).
-struct SlotRing {
-    int slot = 0, n = 1;
-    uint32_t phase = 0;
-    __device__ explicit SlotRing(int count) : n(count) {}
-    __device__ void next() {
-        if (++slot == n) {
-            slot = 0;
-            phase ^= 1u;
-        }
-    }
-};
-
-// ll + 255 (lh + hl) + 255^2 hh mod p (balanced); c1 = 255, c2 = 255^2 mod p, balanced.
-__device__ __forceinline__ int32_t combine(int32_t ll, int32_t lhhl, int32_t hh, const Mod& mod, int32_t c1,
-                                           int32_t c2) {
-    const int32_t a = reduce_partial(ll, mod);
-    const int32_t b = reduce_partial(lhhl, mod);
-    const int32_t c = reduce_partial(hh, mod);
-    return reduce_balanced(a + c1 * b + c2 * c, mod);
-}
-
 // The gather-GEMM epilogue's value of one output, balanced: ll + 255 (lh + hl)
 // + 255^2 hh, times the diagonal entry dg when scaling (d^T).  The sum before
 // the last reduction stays below 1.11e9 in magnitude: |ll| <= 1024 * 127^2
@@ -152,47 +112,6 @@ __device__ __forceinline__ int32_t epilogue_value(int32_t ll, int32_t lhhl, int3
                                                   bool scale, int32_t dg) {
     const int32_t t = ll + 255 * reduce_partial(lhhl, mod) + c2 * reduce_partial(hh, mod);
     return reduce_balanced_fast(scale ? reduce_partial(t, mod) * dg : t, mod);
-}
-
-__host__ __device__ __forceinline__ void split_limbs(int32_t v, int8_t& lo, int8_t& hi) {
-    // v in [-16383, 16383]: q = floor((v + 127) / 255), lo = v - 255 q in [-127, 127]
-    const int32_t q = static_cast<int32_t>(static_cast<uint32_t>(v + 127 + 255 * 128) / 255u) - 128;
-    lo = static_cast<int8_t>(v - 255 * q);
-    hi = static_cast<int8_t>(q);
-}
-
-// 16 x 16 byte transpose inside each half-warp.  On entry lane L (L = lane & 15)
-// holds row L as four words (byte b of word q = element 4q + b); on exit it
-// holds column L the same way.  Two butterfly stages exchange words (lane bits
-// 2 and 3 against word-index bits), two exchange bytes (lane bits 0 and 1
-// against byte-index bits, recombined with byte permutes).
-__device__ __forceinline__ void transpose16(uint32_t (&w)[4], int lane) {
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const bool upper = (lane >> (k + 2)) & 1;
-        const int step = 1 << k;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (q & step) continue;   // the pair (q, q + step)
-            const uint32_t send = upper ? w[q] : w[q + step];
-            const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 4 << k);
-            if (upper) w[q] = recv;
-            else w[q + step] = recv;
-        }
-    }
-    const bool b0 = lane & 1, b1 = (lane >> 1) & 1;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        uint32_t r = __shfl_xor_sync(0xffffffffu, w[q], 1);
-        w[q] = __byte_perm(w[q], r, b0 ? 0x3715 : 0x6240);
-        r = __shfl_xor_sync(0xffffffffu, w[q], 2);
-        w[q] = __byte_perm(w[q], r, b1 ? 0x3276 : 0x5410);
-    }
-}
-
-// Byte offset of element (row = blk * dim + u, column j) in a plane of width NB.
-__host__ __device__ __forceinline__ long long plane_offset(long long blk, int u, int j, int dim, int NB) {
-    return blk * (static_cast<long long>(NB) * dim) + static_cast<long long>(j >> 4) * dim * 16 + u * 16 + (j & 15);
 }
 
 template <int NB, int PW>
@@ -895,7 +814,7 @@ __global__ void from_limbs_kernel(const int8_t* __restrict__ lo, const int8_t* _
         const int j = static_cast<int>(i - row * w_out);
         const long long blk = row / dim;
         const long long off = plane_offset(blk, static_cast<int>(row - blk * dim), j, dim, NB);
-        out[i] = to_canonical(255 * static_cast<int32_t>(hi[off]) + lo[off], mod);
+        out[i] = to_canonical(reduce_balanced(255 * static_cast<int32_t>(hi[off]) + lo[off], mod), mod);
     }
 }
 
@@ -1175,6 +1094,14 @@ struct KoszulCtx::I8State {
         int pw = 8;                // cp.async producer warps (8 or 16)
         size_t smem = 0;
         unsigned grid = 0;
+        // union kernel (bw_koszul_i8_union.cuh); the dense producers' tables above are then not built
+        bool use_union = false;
+        I8Union u{};
+        int8_t* maps = nullptr;
+        std::vector<uint32_t> mask;      // [tile] union of its blocks' generators
+        uint32_t* d_mask = nullptr;
+        uint32_t *start = nullptr, *words = nullptr, *steps = nullptr;   // stage list of list_gs generators a stage
+        int list_gs = 0;
     } fwd, bwd;
     // Y_a, Y_b, Z: lo, hi, -lo, -hi; each -plane directly follows its +plane in
     // memory, so that one tensor map covers both signs of a limb
@@ -1200,10 +1127,10 @@ struct TuneKey {
     }
 };
 struct TuneChoice {
-    bool gather4 = false;   // the hybrid producer
+    int kind = 0;           // 0 dense cp.async, 1 dense hybrid, 2 union
     int pw = 8;             // cp.async producer warps
-    int gps = 0;            // generators per stage
-    int t_tma = 0;          // hybrid: blocks of a tile gathered by TMA
+    int gps = 0;            // generators per stage (dense and union kernels)
+    int t_tma = 0;          // hybrid: blocks of a tile gathered by TMA; union: producer groups
     double ms = 0;
 };
 std::mutex g_tune_mutex;
@@ -1348,28 +1275,199 @@ bool plan_direction(KoszulCtx& c, KoszulCtx::I8State::Dir& D, int inner, int out
     return true;
 }
 
+// Binomial coefficients for the table kernels: C(n, k), n, k <= 31 (below 2^32).
+struct BinomTable {
+    uint32_t c[32][32];
+};
+
+BinomTable binom_table() {
+    BinomTable t;
+    for (int n = 0; n < 32; ++n)
+        for (int k = 0; k < 32; ++k) t.c[n][k] = static_cast<uint32_t>(k <= n ? binom(n, k) : 0);
+    return t;
+}
+
+// Dense incidence table [blk][r]: neighbour rank | negative << 31, or kAbsent.
+//   forward : blk = T, a (k-1)-subset; neighbour S = T u {i} for every i not in T
+//   backward: blk = S, a k-subset; neighbour T = S \ {i} for every i in S
+// with rank(S) = C(r,k) - 1 - sum_pos C(r-1-S_pos, k-pos) (lexicographic) and
+// the sign (-1)^pos of i's position in S.  One thread unranks a subset and
+// walks the generators; `before` and `after` hold the neighbour's rank terms of
+// the elements below and above i.
+__global__ void incidence_kernel(uint32_t* __restrict__ inc, long long n_blk, int r, int k, bool forward,
+                                 const __grid_constant__ BinomTable B) {
+    const long long blk = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (blk >= n_blk) return;
+    const int size = forward ? k - 1 : k, other = forward ? k : k - 1;   // of blk, of its neighbours
+    uint32_t set = 0, rem = B.c[r][size] - 1 - static_cast<uint32_t>(blk);
+    for (int pos = 0, v = 0; pos < size; ++pos, ++v) {
+        while (B.c[r - 1 - v][size - pos] > rem) ++v;
+        rem -= B.c[r - 1 - v][size - pos];
+        set |= 1u << v;
+    }
+    // an element at position j counts C(r-1-v, other - j) below i; above i its
+    // position in the neighbour is j + 1 (forward) or j - 1 (backward)
+    const int shift = forward ? 1 : -1;
+    uint32_t before = 0, after = 0;
+    for (int v = 0, j = 0; v < r; ++v)
+        if (set >> v & 1) {
+            after += other - j - shift >= 0 ? B.c[r - 1 - v][other - j - shift] : 0u;
+            ++j;
+        }
+    uint32_t* out = inc + blk * r;
+    for (int i = 0, pos = 0; i < r; ++i) {
+        const bool in = (set >> i & 1) != 0;
+        const uint32_t sign = (pos & 1) ? 0x80000000u : 0u;
+        uint32_t e = kAbsent;
+        if (in) after -= other - pos - shift >= 0 ? B.c[r - 1 - i][other - pos - shift] : 0u;
+        if (in != forward)
+            e = (B.c[r][other] - 1 - before - after - (forward ? B.c[r - 1 - i][k - pos] : 0u)) | sign;
+        if (in) {
+            before += other - pos >= 0 ? B.c[r - 1 - i][other - pos] : 0u;
+            ++pos;
+        }
+        out[i] = e;
+    }
+}
+
 // Rows of the TMA gathers: for output block blk and group g (generators
 // 4g..4g+3), the plane row of each generator's neighbour run at h = 0:
 // neg * n_blk_in * HG + nbr * HG, or one past the last row (zero-filled) for an
 // absent generator or one past r.
-std::vector<int4> gather_rows(const std::vector<uint32_t>& inc, uint64_t n_blk, int r, uint64_t n_blk_in, int hg) {
-    const int groups = (r + 3) / 4;
-    const int64_t oob = static_cast<int64_t>(2 * n_blk_in * hg);
-    BW_REQUIRE(oob + hg < (1ll << 31), "INT8 form: plane rows above the TMA coordinate range");
-    std::vector<int4> out(n_blk * groups);
-    for (uint64_t b = 0; b < n_blk; ++b)
-        for (int g = 0; g < groups; ++g) {
-            int32_t v[4];
-            for (int q = 0; q < 4; ++q) {
-                const int i = 4 * g + q;
-                const uint32_t e = i < r ? inc[b * r + i] : kAbsent;
-                v[q] = static_cast<int32_t>(e == kAbsent ? oob
-                                                         : static_cast<int64_t>(e >> 31) * n_blk_in * hg +
-                                                               static_cast<int64_t>(e & 0x7FFFFFFFu) * hg);
+__global__ void gather_rows_kernel(const uint32_t* __restrict__ inc, int4* __restrict__ rows, long long n_blk, int r,
+                                   int groups, long long n_blk_in, int hg) {
+    const long long q = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (q >= n_blk * groups) return;
+    const long long blk = q / groups;
+    const int g = static_cast<int>(q - blk * groups);
+    int32_t v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int i = 4 * g + j;
+        const uint32_t e = i < r ? inc[blk * r + i] : kAbsent;
+        v[j] = static_cast<int32_t>(e == kAbsent ? 2 * n_blk_in * hg
+                                                 : (e >> 31) * n_blk_in * hg + (e & 0x7FFFFFFFu) * static_cast<long long>(hg));
+    }
+    rows[q] = make_int4(v[0], v[1], v[2], v[3]);
+}
+
+// Per tile of bt blocks, the generators that any of its blocks has.
+__global__ void union_mask_kernel(const uint32_t* __restrict__ inc, uint32_t* __restrict__ mask, long long n_tiles,
+                                  long long n_blk, int r, int bt) {
+    const long long tile = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (tile >= n_tiles) return;
+    uint32_t m = 0;
+    for (long long blk = tile * bt; blk < min(n_blk, (tile + 1) * bt); ++blk)
+        for (int i = 0; i < r; ++i)
+            if (inc[blk * r + i] != kAbsent) m |= 1u << i;
+    mask[tile] = m;
+}
+
+unsigned blocks_of(uint64_t items, unsigned threads) { return static_cast<unsigned>((items + threads - 1) / threads); }
+
+// Plans one direction of the union kernel with gs generators a stage and pw
+// producer warps in groups; false when it does not fit (shared memory for the
+// resident maps and at least two slots, one table word and one step word a
+// lane, kUnionPasses passes).
+bool plan_union(KoszulCtx& c, KoszulCtx::I8State::Dir& D, int inner, int outer, bool transpose_dir, int gs, int pw,
+                int groups) {
+    I8Union& U = D.u;
+    const int bt = 128 / c.nbi, run = (c.nbi / 16) * inner;
+    U.r = c.r;
+    U.inner = inner;
+    U.outer = outer;
+    U.ho = (outer + 7) / 8 * 8;
+    U.cpg = (2 * inner + 15) / 16;
+    U.gs = gs;
+    U.groups = groups;
+    U.row = ((gs * U.cpg + 1) / 2 + 3) / 4 * 4;
+    // Without a reduction of hi on its own the epilogue's first sum is lo + 255
+    // hi over at most n = incident generators x inner pairs of rows, each below
+    // 127 * (127 + 127) in lo and 64 * (127 + 127) in hi (the maps' hi limbs are
+    // at most 64): 4.18e6 n, which must stay within the range near_shifted()
+    // brings back below 255 * 127 + 127, 0.49 * 2^32 at p = 32749: n <= 500.
+    U.wide = (transpose_dir ? c.k : c.r - c.k + 1) * inner > 500;
+    const bool odd = (U.cpg & 1) != 0;
+    if (gs < 1 || (odd && gs % 2 != 0) || gs * bt > 32 || U.row > kUnionSteps) return false;
+    if (gs * bt * run > pw / groups * 32 * kUnionPasses) return false;
+    const size_t b = (static_cast<size_t>(c.r) * U.cpg + (odd ? 1 : 0)) * 2 * U.ho * 16;
+    const size_t slot = static_cast<size_t>(gs) * U.cpg * 16 * 128;
+    const size_t extra = (2 * 8 + 2 * 2 + 2) * 8 + 16;
+    if (b + 2 * slot + extra > static_cast<size_t>(kMaxSmem)) return false;
+    U.b_bytes = static_cast<uint32_t>(b);
+    U.slot_bytes = static_cast<uint32_t>(slot);
+    U.slots = static_cast<int>(std::min<size_t>(8, (kMaxSmem - b - extra) / slot));
+    if (U.slots < groups) return false;
+    U.mod = c.mod;
+    U.maps = D.maps;
+    D.pw = pw;
+    D.smem = b + U.slots * slot + extra;
+    return true;
+}
+
+// The maps as the union kernel's B operand, in their shared-memory layout.
+std::vector<int8_t> union_maps(const KoszulCtx& c, int inner, int outer, bool transpose_maps) {
+    const int cpg = (2 * inner + 15) / 16, ho = (outer + 7) / 8 * 8, N = 2 * ho;
+    std::vector<int8_t> maps((static_cast<size_t>(c.r) * cpg + (cpg & 1)) * N * 16, 0);
+    for (int i = 0; i < c.r; ++i)
+        for (int row = 0; row < 2 * inner; ++row) {
+            const int limb = row / inner, u = row - limb * inner;
+            for (int o = 0; o < outer; ++o) {
+                // forward: coefficient M_i[o][u]; transpose: M_i[u][o]; times 255 for the hi rows
+                const uint64_t raw = transpose_maps
+                                         ? c.maps_canonical[(static_cast<size_t>(i) * c.co + u) * c.ci + o]
+                                         : c.maps_canonical[(static_cast<size_t>(i) * c.co + o) * c.ci + u];
+                const uint32_t v = static_cast<uint32_t>((limb ? 255u : 1u) * raw % c.p);
+                int8_t lo, hi;
+                split_limbs(to_balanced(v, c.mod), lo, hi);
+                int8_t* at = maps.data() + (static_cast<size_t>(i) * cpg + row / 16) * N * 16 + row % 16;
+                at[static_cast<size_t>(o) * 16] = lo;
+                at[static_cast<size_t>(ho + o) * 16] = hi;
             }
-            out[b * groups + g] = make_int4(v[0], v[1], v[2], v[3]);
         }
-    return out;
+    return maps;
+}
+
+// Builds the stage list for D.u's generators a stage: CTA c's tiles are c,
+// c + grid, ..., their stages one after the other.
+void build_stage_list(KoszulCtx& c, KoszulCtx::I8State::Dir& D, uint64_t n_blk, uint64_t n_in, int inner) {
+    I8Union& U = D.u;
+    if (D.list_gs != U.gs) {
+        for (uint32_t** p : {&D.start, &D.words, &D.steps})
+            if (*p) {
+                c.release(*p);
+                *p = nullptr;
+            }
+        const uint64_t tiles = D.mask.size();
+        const int bt = 128 / c.nbi;
+        std::vector<uint32_t> start(D.grid + 1, 0u), tile_stage(tiles);
+        uint32_t at = 0;
+        for (unsigned cta = 0; cta < D.grid; ++cta) {
+            start[cta] = at;
+            for (uint64_t t = cta; t < tiles; t += D.grid) {
+                tile_stage[t] = at;
+                at += static_cast<uint32_t>((__builtin_popcount(D.mask[t]) + U.gs - 1) / U.gs);
+            }
+        }
+        start[D.grid] = at;
+        D.start = c.alloc<uint32_t>(start.size());
+        D.words = c.alloc<uint32_t>(static_cast<uint64_t>(at) * U.gs * bt);
+        D.steps = c.alloc<uint32_t>(static_cast<uint64_t>(at) * U.row);
+        uint32_t* d_ts = c.alloc<uint32_t>(tiles);
+        BW_CUDA(cudaMemcpyAsync(D.start, start.data(), start.size() * 4, cudaMemcpyHostToDevice, c.own_stream));
+        BW_CUDA(cudaMemcpyAsync(d_ts, tile_stage.data(), tiles * 4, cudaMemcpyHostToDevice, c.own_stream));
+        const uint32_t run16 = static_cast<uint32_t>((c.nbi / 16) * inner);
+        union_tables_kernel<<<blocks_of(tiles, 128), 128, 0, c.own_stream>>>(
+            D.inc, D.d_mask, d_ts, D.words, D.steps, static_cast<long long>(tiles), static_cast<long long>(n_blk), c.r,
+            bt, U.gs, U.cpg, 2 * U.ho, U.row, run16, static_cast<uint32_t>(n_in * run16));
+        BW_CHECK_LAUNCH();
+        BW_CUDA(cudaStreamSynchronize(c.own_stream));
+        c.release(d_ts);
+        D.list_gs = U.gs;
+    }
+    U.start = D.start;
+    U.words = D.words;
+    U.steps = D.steps;
 }
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1455,6 +1553,17 @@ void plan_projection(KoszulCtx& c, KoszulCtx::I8State& S) {
 
 template <int NB>
 void launch_i8(KoszulCtx& c, KoszulCtx::I8State::Dir& D, const CUtensorMap* maps, cudaStream_t st) {
+    if (D.use_union) {
+        BW_REQUIRE(D.u.start != nullptr && D.u.words != nullptr && D.u.steps != nullptr && D.u.maps != nullptr,
+                   "internal: INT8 stage list missing for the union kernel");
+        if (D.pw == 16)
+            i8_union_gemm_kernel<NB, 16><<<D.grid, GatherWarps<16>::threads, D.smem, st>>>(D.u);
+        else
+            i8_union_gemm_kernel<NB, 8><<<D.grid, GatherWarps<8>::threads, D.smem, st>>>(D.u);
+        BW_CHECK_LAUNCH();
+        ++c.launches;
+        return;
+    }
     BW_REQUIRE(D.p.inc != nullptr && (!D.gather4 || D.p.rows4 != nullptr) && D.p.b_tiles != nullptr,
                "internal: INT8 gather tables missing for the chosen producer");
     if (D.gather4)
@@ -1485,29 +1594,6 @@ void KoszulCtx::i8_setup() {
     BW_REQUIRE(major == 10, "INT8 form needs an sm_100 GPU (tcgen05)");
     i8 = new I8State();
     I8State& S = *i8;
-    // dense incidence tables: fwd[T][i] (S = T u i), bwd[S][i] (T = S \ i)
-    std::vector<uint32_t> fwd(n_t * r, kAbsent), bwd(n_s * r, kAbsent);
-    int T[64], Sx[64];
-    for (uint64_t t = 0; t < n_t; ++t) {
-        lex_unrank(t, r, k - 1, T);
-        int pos = 0;
-        for (int i = 0; i < r; ++i) {
-            if (pos < k - 1 && T[pos] == i) {
-                ++pos;
-                continue;
-            }
-            for (int qq = 0, w = 0; qq < k; ++qq) Sx[qq] = (qq == pos) ? i : T[w++];
-            fwd[t * r + i] = static_cast<uint32_t>(lex_rank(Sx, r, k)) | ((pos & 1) ? 0x80000000u : 0u);
-        }
-    }
-    for (uint64_t s = 0; s < n_s; ++s) {
-        lex_unrank(s, r, k, Sx);
-        for (int pos = 0; pos < k; ++pos) {
-            for (int qq = 0, w = 0; qq < k; ++qq)
-                if (qq != pos) T[w++] = Sx[qq];
-            bwd[s * r + Sx[pos]] = static_cast<uint32_t>(lex_rank(T, r, k - 1)) | ((pos & 1) ? 0x80000000u : 0u);
-        }
-    }
     // each limb's -plane directly after its +plane (one tensor map covers both signs)
     for (int b = 0; b < 3; ++b) {
         const uint64_t plane = (b < 2 ? n_src : n_tgt) * nbi;
@@ -1523,25 +1609,103 @@ void KoszulCtx::i8_setup() {
     BW_CUDA(cudaMemsetAsync(S.err, 0, sizeof(int), own_stream));
     plan_projection(*this, S);
     const int hg = nbi / 16;
-    // Both gather tables (TMA rows per group of four generators, and the
-    // per-generator words of the cp.async producer) until the plans are chosen.
-    auto upload_rows = [&](const std::vector<uint32_t>& inc, uint64_t n_out, uint64_t n_in) {
-        const std::vector<int4> rows = gather_rows(inc, n_out, r, n_in, hg);
-        int4* d = alloc<int4>(rows.size());
-        BW_CUDA(cudaMemcpyAsync(d, rows.data(), rows.size() * sizeof(int4), cudaMemcpyHostToDevice, own_stream));
-        BW_CUDA(cudaStreamSynchronize(own_stream));
-        return d;
+    // The producers that may be used.  BW_I8_PRODUCER=union, =cpasync or
+    // =hybrid restricts the choice to one.
+    bool allow_union = true, allow_g4 = true, allow_cp = true, tune = true;
+    if (const char* e = std::getenv("BW_I8_PRODUCER")) {
+        const std::string want = e;
+        allow_union = want != "cpasync" && want != "hybrid";
+        allow_g4 = want != "cpasync" && want != "union";
+        allow_cp = want != "hybrid" && want != "union";
+    }
+    if (const char* e = std::getenv("BW_I8_TUNE")) tune = std::string(e) != "0";
+    // BW_I8_PRODUCER_WARPS=8 or =16 restricts the cp.async producers' warp count
+    std::vector<int> pws{8, 16};
+    if (const char* e = std::getenv("BW_I8_PRODUCER_WARPS")) {
+        const int v = std::atoi(e);
+        if (v == 8 || v == 16) pws = {v};
+    }
+    // Plans of a direction (see Cand): the union kernel's, and the dense
+    // producers' only where the union kernel's resident maps leave room for
+    // fewer than eight generators in flight (maps of 2 r inner rows: r * inner
+    // * outer above about 32,000).  With more room the union kernel won at every
+    // shape timed (us, dense against union: r=19 k=9 20->28 n=16 179/130 d and
+    // 228/156 d^T; r=21 k=10 32->40 n=32 1726/1190 and 2429/1411).
+    struct Cand {
+        int kind;               // 0 dense cp.async, 1 dense hybrid, 2 union
+        int gps, t_tma, pw;     // as in TuneChoice
     };
-    auto upload_inc = [&](const std::vector<uint32_t>& inc) {
-        uint32_t* d = alloc<uint32_t>(inc.size());
-        BW_CUDA(cudaMemcpyAsync(d, inc.data(), inc.size() * 4, cudaMemcpyHostToDevice, own_stream));
-        BW_CUDA(cudaStreamSynchronize(own_stream));
-        return d;
-    };
-    S.fwd.rows4 = upload_rows(fwd, n_t, n_s);
-    S.bwd.rows4 = upload_rows(bwd, n_s, n_t);
-    S.fwd.inc = upload_inc(fwd);
-    S.bwd.inc = upload_inc(bwd);
+    std::vector<Cand> cands[2];
+    TuneKey keys[2];
+    const BinomTable binoms = binom_table();
+    for (int dir = 0; dir < 2; ++dir) {
+        I8State::Dir& D = dir == 0 ? S.fwd : S.bwd;
+        const uint64_t n_out = dir == 0 ? n_t : n_s, n_in = dir == 0 ? n_s : n_t;
+        const int inner = dir == 0 ? ci : co, outer = dir == 0 ? co : ci, bt = 128 / nbi;
+        int in_flight = 0;      // generators, of the roomiest union plan
+        // four to eight generators a stage (fewer, where those do not fit, pay a
+        // hand-over between the roles for less work), warps in 2 or 4 groups
+        for (const auto& sizes : {std::vector<int>{4, 6, 8}, std::vector<int>{3, 2}})
+            for (int g : sizes)
+                for (int pw : pws)
+                    for (int groups : {2, 4}) {
+                        if (!allow_union || !plan_union(*this, D, inner, outer, dir == 1, g, pw, groups)) continue;
+                        if (g < 4 && !cands[dir].empty() && cands[dir][0].gps >= 4) continue;
+                        cands[dir].push_back({2, g, groups, pw});
+                        in_flight = std::max(in_flight, D.u.slots * g);
+                    }
+        const bool dense = (allow_g4 || allow_cp) && in_flight < 8;
+        BW_REQUIRE(!cands[dir].empty() || dense, "INT8 form: no union plan fits in shared memory");
+        if (dense) {
+            if (allow_cp)
+                // the fill heuristic's stage, and fewer or more generators a stage
+                // (smaller stages leave room for more pipeline slots)
+                for (int pw : pws) {
+                    cands[dir].push_back({0, 0, 0, pw});
+                    for (int g : {4, 6, 8, 12})
+                        if (g < r) cands[dir].push_back({0, g, 0, pw});
+                }
+            if (allow_g4)
+                for (int gs = 1; gs <= std::min(3, (r + 3) / 4); ++gs)
+                    for (int qt = 1; qt <= 3; ++qt) cands[dir].push_back({1, 4 * gs, qt * bt / 4, 8});
+        }
+        keys[dir] = TuneKey{r, k, inner, outer, nbi, dir, sms,
+                            (allow_g4 ? 1 : 0) | (allow_cp ? 2 : 0) | (pws.size() == 1 ? pws[0] * 4 : 0) |
+                                (allow_union ? 128 : 0)};
+        TuneChoice known{};
+        // a shape tuned earlier in this process: its choice alone
+        if (tune && tune_lookup(keys[dir], known))
+            cands[dir] = {{known.kind, known.gps, known.t_tma, known.pw}};
+        // the tables that the candidates read
+        bool any_union = false, any_rows = false;
+        for (const Cand& c : cands[dir]) {
+            any_union = any_union || c.kind == 2;
+            any_rows = any_rows || c.kind == 1;
+        }
+        D.inc = alloc<uint32_t>(n_out * r);
+        incidence_kernel<<<blocks_of(n_out, 128), 128, 0, own_stream>>>(D.inc, static_cast<long long>(n_out), r, k,
+                                                                         dir == 0, binoms);
+        if (any_rows) {
+            const int groups = (r + 3) / 4;
+            BW_REQUIRE(2 * n_in * hg + hg < (1ull << 31), "INT8 form: plane rows above the TMA coordinate range");
+            D.rows4 = alloc<int4>(n_out * groups);
+            gather_rows_kernel<<<blocks_of(n_out * groups, 256), 256, 0, own_stream>>>(
+                D.inc, D.rows4, static_cast<long long>(n_out), r, groups, static_cast<long long>(n_in), hg);
+        }
+        if (any_union) {
+            const uint64_t tiles = (n_out + bt - 1) / bt;
+            D.d_mask = alloc<uint32_t>(tiles);
+            union_mask_kernel<<<blocks_of(tiles, 128), 128, 0, own_stream>>>(
+                D.inc, D.d_mask, static_cast<long long>(tiles), static_cast<long long>(n_out), r, bt);
+            D.mask.resize(tiles);
+            BW_CUDA(cudaMemcpyAsync(D.mask.data(), D.d_mask, tiles * 4, cudaMemcpyDeviceToHost, own_stream));
+            const std::vector<int8_t> maps = union_maps(*this, inner, outer, dir == 1);
+            D.maps = alloc<int8_t>(maps.size());
+            BW_CUDA(cudaMemcpyAsync(D.maps, maps.data(), maps.size(), cudaMemcpyHostToDevice, own_stream));
+            BW_CUDA(cudaStreamSynchronize(own_stream));
+        }
+        BW_CHECK_LAUNCH();
+    }
     for (int b = 0; b < 3; ++b) {
         const uint64_t n_blk = b < 2 ? n_s : n_t;
         const int dim = b < 2 ? ci : co;
@@ -1561,10 +1725,12 @@ void KoszulCtx::i8_setup() {
     int hold = 0;
     if (const char* e = std::getenv("BW_TEST_HOLD_FIRST_STAGE")) hold = (*e && std::string(e) != "0") ? 1 : 0;
     S.proj.wait_limit = wait_limit;
-    int cap_g = 0, cap_4 = 0;
+    int cap_g = 0, cap_4 = 0, cap_u = 0;
     dispatch_i8_nb(nbi, [&](auto NBc) {
         cap_g = std::min(allow_dynamic_smem(i8_gather_gemm_kernel<decltype(NBc)::value, 8>, device),
                          allow_dynamic_smem(i8_gather_gemm_kernel<decltype(NBc)::value, 16>, device));
+        cap_u = std::min(allow_dynamic_smem(i8_union_gemm_kernel<decltype(NBc)::value, 8>, device),
+                         allow_dynamic_smem(i8_union_gemm_kernel<decltype(NBc)::value, 16>, device));
         cap_4 = allow_dynamic_smem(i8_gather_hybrid_kernel<decltype(NBc)::value>, device);
         const int cap_p = allow_dynamic_smem(i8_project_tc_kernel<decltype(NBc)::value>, device);
         BW_REQUIRE(static_cast<int>(S.proj_smem) <= cap_p, "INT8 form: shared-memory plan above the device limit");
@@ -1577,37 +1743,35 @@ void KoszulCtx::i8_setup() {
     S.fwd.grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((n_t + bt - 1) / bt, sms)));
     S.bwd.grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((n_s + bt - 1) / bt, sms)));
 
-    // Stage plans.  Each direction's producer (TMA gathers or cp.async warps)
-    // and stage size are chosen by timing every candidate that fits in shared
-    // memory on this device, at set-up, on the context's own buffers (the
-    // kernels' work does not depend on the values); the choice is cached per
-    // shape for the life of the process.  BW_I8_TUNE=0 takes the fill
-    // heuristic instead; BW_I8_PRODUCER=cpasync or =hybrid restricts the
-    // producer.
-    bool allow_g4 = true, allow_cp = true, tune = true;
-    if (const char* e = std::getenv("BW_I8_PRODUCER")) {
-        allow_g4 = std::string(e) != "cpasync";
-        allow_cp = std::string(e) != "hybrid";
-    }
-    if (const char* e = std::getenv("BW_I8_TUNE")) tune = std::string(e) != "0";
-    // BW_I8_PRODUCER_WARPS=8 or =16 restricts the cp.async producer's warp count
-    std::vector<int> pws{8, 16};
-    if (const char* e = std::getenv("BW_I8_PRODUCER_WARPS")) {
-        const int v = std::atoi(e);
-        if (v == 8 || v == 16) pws = {v};
-    }
+    // Stage plans.  Each direction's plan is chosen by timing every candidate
+    // that fits in shared memory on this device, at set-up, on the context's
+    // own buffers (the kernels' work does not depend on the values); the choice
+    // is cached per shape for the life of the process.  BW_I8_TUNE=0 takes the
+    // first candidate that fits instead.
     std::string text;
     for (int dir = 0; dir < 2; ++dir) {
         I8State::Dir& D = dir == 0 ? S.fwd : S.bwd;
         const int inner = dir == 0 ? ci : co, outer = dir == 0 ? co : ci;
         const int in_buf = dir == 0 ? I8_YA : I8_Z, out_buf = dir == 0 ? I8_Z : I8_YB;
-        auto plan = [&](bool g4, int gps, int t_tma, int pw) {
+        auto plan = [&](const Cand& c) {
+            D.use_union = c.kind == 2;
+            if (D.use_union) {
+                if (!plan_union(*this, D, inner, outer, dir == 1, c.gps, c.pw, c.t_tma) ||
+                    static_cast<int>(D.smem) > cap_u)
+                    return false;
+                build_stage_list(*this, D, dir == 0 ? n_t : n_s, dir == 0 ? n_s : n_t, inner);
+                D.u.err = S.err;
+                D.u.wait_limit = wait_limit;
+                D.u.hold_first_stage = 0;
+                return true;
+            }
+            const bool g4 = c.kind == 1;
             if (D.b_tiles) release(D.b_tiles);
             D.b_tiles = nullptr;
-            if (!plan_direction(*this, D, inner, outer, dir == 1, g4, gps)) return false;
+            if (!plan_direction(*this, D, inner, outer, dir == 1, g4, c.gps)) return false;
             if (static_cast<int>(D.smem) > (g4 ? cap_4 : cap_g)) return false;
-            D.pw = g4 ? 8 : pw;
-            D.p.t_tma = g4 ? t_tma : 0;
+            D.pw = g4 ? 8 : c.pw;
+            D.p.t_tma = g4 ? c.t_tma : 0;
             D.p.err = S.err;
             D.p.wait_limit = wait_limit;
             D.p.hold_first_stage = 0;
@@ -1615,60 +1779,45 @@ void KoszulCtx::i8_setup() {
             D.p.rows4 = D.rows4;
             return true;
         };
-        const TuneKey key{r, k, inner, outer, nbi, dir, sms,
-                          (allow_g4 ? 1 : 0) | (allow_cp ? 2 : 0) | (pws.size() == 1 ? pws[0] * 4 : 0)};
-        TuneChoice choice{};
-        bool have = tune && tune_lookup(key, choice);
         std::string tried;
-        if (!have && tune) {
-            // candidates: the cp.async producer with its heuristic stage; the
-            // hybrid producer with 1..3 groups of four generators a stage and a
-            // quarter, half or three quarters of a tile's blocks gathered by TMA
-            struct Cand {
-                bool g4;
-                int gps, t_tma, pw;
-            };
-            std::vector<Cand> cands;
-            if (allow_cp) {
-                // the fill heuristic's stage, and fewer or more generators a stage
-                // (smaller stages leave room for more pipeline slots), each with 8
-                // and with 16 producer warps
-                for (int pw : pws) {
-                    cands.push_back({false, 0, 0, pw});
-                    for (int g : {4, 6, 8, 12})
-                        if (g < r) cands.push_back({false, g, 0, pw});
+        Cand choice = cands[dir][0];
+        if (!tune) {
+            for (const Cand& cand : cands[dir])
+                if (plan(cand)) {
+                    choice = cand;
+                    break;
                 }
-            }
-            if (allow_g4)
-                for (int gs = 1; gs <= std::min(3, (r + 3) / 4); ++gs)
-                    for (int qt = 1; qt <= 3; ++qt) cands.push_back({true, 4 * gs, qt * bt / 4, 8});
+        } else if (cands[dir].size() > 1) {
             double best = 1e30;
-            for (const Cand& cand : cands) {
-                if (!plan(cand.g4, cand.gps, cand.t_tma, cand.pw)) continue;
+            for (const Cand& cand : cands[dir]) {
+                if (!plan(cand)) continue;
                 const double ms = i8_time_direction(dir == 0, in_buf, out_buf);
                 char buf[96];
-                if (cand.g4)
-                    std::snprintf(buf, sizeof buf, "%shybrid stage=%d tma=%d/%d: %.4f ms", tried.empty() ? "" : ", ",
-                                  D.p.gi, cand.t_tma, bt, ms);
+                const char* sep = tried.empty() ? "" : ", ";
+                if (cand.kind == 2)
+                    std::snprintf(buf, sizeof buf, "%sunion stage=%d warps=%d/%d: %.4f ms", sep, cand.gps, cand.pw,
+                                  cand.t_tma, ms);
+                else if (cand.kind == 1)
+                    std::snprintf(buf, sizeof buf, "%shybrid stage=%d tma=%d/%d: %.4f ms", sep, D.p.gi, cand.t_tma, bt,
+                                  ms);
                 else
-                    std::snprintf(buf, sizeof buf, "%scp.async stage=%d warps=%d: %.4f ms", tried.empty() ? "" : ", ",
-                                  D.p.gi, cand.pw, ms);
+                    std::snprintf(buf, sizeof buf, "%scp.async stage=%d warps=%d: %.4f ms", sep, D.p.gi, cand.pw, ms);
                 tried += buf;
                 if (ms < best) {
                     best = ms;
-                    choice = TuneChoice{cand.g4, cand.pw, D.p.gi, cand.t_tma, ms};
+                    choice = {cand.kind, cand.kind == 2 ? cand.gps : D.p.gi, cand.t_tma, cand.pw};
                 }
             }
             BW_REQUIRE(best < 1e30, "INT8 form: no stage plan fits in shared memory");
-            tune_store(key, choice);
-            have = true;
+            tune_store(keys[dir], TuneChoice{choice.kind, choice.pw, choice.gps, choice.t_tma, best});
         }
-        bool ok = false;
-        if (have) ok = plan(choice.gather4, choice.gps, choice.t_tma, choice.pw);
-        if (!ok) ok = (allow_cp && plan(false, 0, 0, pws[0])) || (allow_g4 && plan(true, 0, bt / 2, 8));
-        BW_REQUIRE(ok, "INT8 form: maps too large for shared memory");
+        BW_REQUIRE(plan(choice), "INT8 form: maps too large for shared memory");
+        D.gather4 = !D.use_union && D.gather4;
         char buf[192];
-        if (D.gather4)
+        if (D.use_union)
+            std::snprintf(buf, sizeof buf, "%s: union stage=%d generators, %d producer warps in %d groups, %d slots, "
+                          "%zu B shared", dir == 0 ? "d" : "d^T", D.u.gs, D.pw, D.u.groups, D.u.slots, D.smem);
+        else if (D.gather4)
             std::snprintf(buf, sizeof buf, "%s: hybrid (TMA gathers for %d of %d blocks) stage=%d generators, %d slots, "
                           "%zu B shared", dir == 0 ? "d" : "d^T", D.p.t_tma, bt, D.p.gi, D.p.slots, D.smem);
         else
@@ -1677,13 +1826,25 @@ void KoszulCtx::i8_setup() {
         text += (text.empty() ? "" : "; ") + std::string(buf);
         if (!tried.empty()) text += " (tuned: " + tried + ")";
     }
-    // the TMA rows are freed when the cp.async producer alone was chosen (the
-    // hybrid producer reads both tables)
+    // the tables of the producers that were not chosen are freed: the union
+    // kernel reads its stage list only, the hybrid producer both dense tables
     for (I8State::Dir* D : {&S.fwd, &S.bwd}) {
-        if (!D->gather4) {
-            release(D->rows4);
-            D->rows4 = nullptr;
+        auto drop = [&](auto*& p) {
+            if (p) release(p);
+            p = nullptr;
+        };
+        if (D->use_union) {
+            drop(D->inc);
+        } else {
+            drop(D->start);
+            drop(D->words);
+            drop(D->steps);
+            drop(D->maps);
         }
+        if (!D->gather4) drop(D->rows4);
+        drop(D->d_mask);
+        D->mask = std::vector<uint32_t>();
+        D->u.hold_first_stage = hold;
         D->p.inc = D->inc;
         D->p.rows4 = D->rows4;
         D->p.hold_first_stage = hold;
@@ -1720,6 +1881,13 @@ uint64_t KoszulCtx::i8_kernels_per_step() const { return 3; }
 
 void KoszulCtx::i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cudaStream_t st) {
     I8State::Dir& D = forward_dir ? i8->fwd : i8->bwd;
+    if (D.use_union) {
+        D.u.in[0] = i8->planes[in_buf][PL_LO];
+        D.u.in[1] = i8->planes[in_buf][PL_HI];
+        for (int pl = 0; pl < 4; ++pl) D.u.out[pl] = i8->planes[out_buf][pl];
+        D.u.n_blk = D.p.n_blk;
+        D.u.diag = (!forward_dir && scale) ? d_diag : nullptr;
+    }
     for (int pl = 0; pl < 4; ++pl) {
         D.p.in[pl] = i8->planes[in_buf][pl];
         D.p.out[pl] = i8->planes[out_buf][pl];

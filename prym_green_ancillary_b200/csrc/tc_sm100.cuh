@@ -77,6 +77,30 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     return false;
 }
 
+// The same wait made by a whole converged warp (bar, a shared-memory address,
+// and parity uniform): the outcome comes from warp votes, so every branch on
+// it is uniform.  With one lane waiting (or lanes branching on their own
+// outcome) a wait on a phase that is already complete costs about 230-330
+// cycles of divergence handling; voted, about 70.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort, int* err, int code,
+                                          uint32_t limit = kWaitLimit) {
+    for (uint32_t i = 0; i < limit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (__all_sync(0xffffffffu, ok != 0)) return true;
+        if (abort != nullptr && __any_sync(0xffffffffu, *abort != 0)) return false;
+    }
+    if (abort != nullptr) *abort = 1;
+    atomicCAS(err, ERR_NONE, code);
+    return false;
+}
+
 // Bulk copy of `bytes` (multiple of 16, both addresses 16-byte aligned) from
 // global to this CTA's shared memory, completing on `bar` (tx bytes).
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -126,6 +150,10 @@ __device__ __forceinline__ void cp_async16_zfill(uint32_t dst_smem, const void* 
 // (the arrival is one of the barrier's expected arrivals).
 __device__ __forceinline__ void cp_async_arrive_noinc(uint64_t* bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {   // bar: a shared-memory address
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // Wait until every cp.async issued by this thread has completed.
@@ -190,10 +218,35 @@ __device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_
         : "memory");
 }
 
+// The same issued by one elected lane of a converged warp.  The operands have
+// to be values the compiler can prove warp-uniform (kernel parameters, warp
+// votes and shuffles): from such values an MMA issues at the tensor pipe's
+// rate, from others it costs about 100 cycles more.
+__device__ __forceinline__ void mma_i8_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                             uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
 // Arrive on `bar` once all tcgen05 operations issued so far by this thread complete.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
+}
+
+// The same by one elected lane of a converged warp (the lane that
+// mma_i8_elect() elects), the barrier as a shared-memory address.
+__device__ __forceinline__ void mma_commit_elect(uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar)
+        : "memory");
 }
 
 // 32 lanes x 16 consecutive 32-bit columns (lane = warp quadrant base + lane id).
