@@ -142,6 +142,12 @@ __host__ __device__ __forceinline__ int32_t reduce_balanced_fast(int32_t x, cons
     return s - (s >= m.p ? m.p + m.half : m.half);
 }
 
+// x mod p in [0, p) for any 32-bit x: floor(x * barrett / 2^32) is floor(x / p) or one below.
+__host__ __device__ __forceinline__ uint32_t reduce_u32(uint32_t x, const Mod& m) {
+    const uint32_t p = static_cast<uint32_t>(m.p), r = x - mulhi_u32(x, static_cast<uint32_t>(m.barrett)) * p;
+    return r >= p ? r - p : r;
+}
+
 // Bytewise negation of four signed bytes in [-127, 127] (SWAR: 0x80 - the low
 // seven bits never borrows across a byte; the sign bit is then fixed up).
 __host__ __device__ __forceinline__ uint32_t neg_bytes4(uint32_t w) {
@@ -155,6 +161,31 @@ __host__ __device__ __forceinline__ int32_t to_balanced(uint32_t canonical, cons
 
 __host__ __device__ __forceinline__ uint32_t to_canonical(int32_t balanced, const Mod& m) {
     return static_cast<uint32_t>(balanced < 0 ? balanced + m.p : balanced);
+}
+
+#if defined(__CUDACC__)
+// Four consecutive residues of a caller's buffer: one 16-byte access where the
+// buffer is 16-byte aligned (the offset is a multiple of four), else four.
+__device__ __forceinline__ uint4 load_quad(const uint32_t* p, bool aligned) {
+    if (aligned) return __ldg(reinterpret_cast<const uint4*>(p));
+    return make_uint4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+__device__ __forceinline__ void store_quad(uint32_t* p, const uint4& v, bool aligned) {
+    if (aligned) {
+        *reinterpret_cast<uint4*>(p) = v;
+    } else {
+        p[0] = v.x;
+        p[1] = v.y;
+        p[2] = v.z;
+        p[3] = v.w;
+    }
+}
+#endif
+inline bool quad_aligned(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+// Grid of 256-thread blocks for a quad-per-thread pass, at most a full GPU's worth.
+inline unsigned quad_grid(uint64_t quads, int sms) {
+    const uint64_t want = (quads + 255) / 256, most = static_cast<uint64_t>(sms) * 8;
+    return static_cast<unsigned>(want < 1 ? 1 : want < most ? want : most);
 }
 
 // ------------------------------------------------------------ seeded data

@@ -248,36 +248,49 @@ __global__ void __launch_bounds__(256) project_kernel(
     }
 }
 
-__global__ void to_balanced_kernel(const uint32_t* __restrict__ in, int32_t* __restrict__ out,
-                                   long long count, Mod mod) {
-    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-    for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride)
-        out[i] = to_balanced(in[i] % static_cast<uint32_t>(mod.p), mod);
+// Four residues a thread; the last count % 4 go to the first threads one by one.
+__global__ void __launch_bounds__(256) to_balanced_kernel(const uint32_t* __restrict__ in, int32_t* __restrict__ out,
+                                                          long long count, bool aligned, Mod mod) {
+    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x, quads = count / 4;
+    const long long first = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (long long i = first; i < quads; i += stride) {
+        const uint4 v = load_quad(in + i * 4, aligned);
+        reinterpret_cast<int4*>(out)[i] =
+            make_int4(to_balanced(reduce_u32(v.x, mod), mod), to_balanced(reduce_u32(v.y, mod), mod),
+                      to_balanced(reduce_u32(v.z, mod), mod), to_balanced(reduce_u32(v.w, mod), mod));
+    }
+    if (first < count % 4) out[quads * 4 + first] = to_balanced(reduce_u32(in[quads * 4 + first], mod), mod);
 }
 
-__global__ void to_canonical_kernel(const int32_t* __restrict__ in, uint32_t* __restrict__ out,
-                                    long long count, Mod mod) {
-    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-    for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride)
-        out[i] = to_canonical(in[i], mod);
+__global__ void __launch_bounds__(256) to_canonical_kernel(const int32_t* __restrict__ in, uint32_t* __restrict__ out,
+                                                           long long count, bool aligned, Mod mod) {
+    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x, quads = count / 4;
+    const long long first = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (long long i = first; i < quads; i += stride) {
+        const int4 v = __ldg(reinterpret_cast<const int4*>(in) + i);
+        store_quad(out + i * 4, make_uint4(to_canonical(v.x, mod), to_canonical(v.y, mod), to_canonical(v.z, mod),
+                                           to_canonical(v.w, mod)), aligned);
+    }
+    if (first < count % 4) out[quads * 4 + first] = to_canonical(in[quads * 4 + first], mod);
 }
 
 }  // namespace
 
 // ------------------------------------------------------------ host helpers
 
+// The engine's side of either conversion is one of its own allocations (16-byte aligned).
 void KoszulCtx::launch_to_balanced(const uint32_t* in, int32_t* out, uint64_t count, cudaStream_t st) {
     if (count == 0) return;
-    unsigned grid = static_cast<unsigned>(std::min<uint64_t>((count + 255) / 256, static_cast<uint64_t>(sms) * 8));
-    to_balanced_kernel<<<grid, 256, 0, st>>>(in, out, static_cast<long long>(count), mod);
+    to_balanced_kernel<<<quad_grid(count / 4, sms), 256, 0, st>>>(in, out, static_cast<long long>(count),
+                                                                  quad_aligned(in), mod);
     BW_CHECK_LAUNCH();
     ++launches;
 }
 
 void KoszulCtx::launch_to_canonical(const int32_t* in, uint32_t* out, uint64_t count, cudaStream_t st) {
     if (count == 0) return;
-    unsigned grid = static_cast<unsigned>(std::min<uint64_t>((count + 255) / 256, static_cast<uint64_t>(sms) * 8));
-    to_canonical_kernel<<<grid, 256, 0, st>>>(in, out, static_cast<long long>(count), mod);
+    to_canonical_kernel<<<quad_grid(count / 4, sms), 256, 0, st>>>(in, out, static_cast<long long>(count),
+                                                                   quad_aligned(out), mod);
     BW_CHECK_LAUNCH();
     ++launches;
 }

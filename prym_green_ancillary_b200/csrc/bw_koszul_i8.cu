@@ -782,39 +782,74 @@ __global__ void __launch_bounds__(kHyThreads, 1)
 }
 
 // ---- limb conversions and the projection on limb planes
+//
+// Memory-bound: a thread takes four columns of a row (16 bytes of residues, 4
+// bytes of each plane), so a warp's loads and stores are whole lines; one
+// byte a thread with 64-bit divisions ran at a sixth of the copy bandwidth
+// (genus-20-like Y, 1.85 M x 16, with the call around d: 514 us against 254).
 
-// canonical row-major (rows = n_blk * dim, w_in columns) -> four planes of NB
-// columns (columns w_in..NB-1 are zero)
+// Offset of the four columns 4 q .. 4 q + 3 of a row in a plane of NB columns.
 template <int NB>
-__global__ void to_limbs_kernel(const uint32_t* __restrict__ in, int8_t* __restrict__ lo, int8_t* __restrict__ hi,
-                                int8_t* __restrict__ nlo, int8_t* __restrict__ nhi, long long count, int dim,
-                                int w_in, Mod mod) {
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < count;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const long long row = i / NB;
-        const int j = static_cast<int>(i - row * NB);
-        int8_t a = 0, b = 0;
-        if (j < w_in) split_limbs(to_balanced(in[row * w_in + j] % static_cast<uint32_t>(mod.p), mod), a, b);
-        const long long blk = row / dim;
-        const long long off = plane_offset(blk, static_cast<int>(row - blk * dim), j, dim, NB);
-        lo[off] = a;
-        hi[off] = b;
-        nlo[off] = static_cast<int8_t>(-a);
-        nhi[off] = static_cast<int8_t>(-b);
+__device__ __forceinline__ size_t quad_offset(uint32_t row, uint32_t q, uint32_t dim) {
+    if constexpr (NB == 16) {
+        return static_cast<size_t>(row) * 16 + q * 4;   // one column group: a block's rows are its plane rows
+    } else {
+        const uint32_t blk = row / dim, u = row - blk * dim;
+        return (static_cast<size_t>(blk) * (NB / 16) + (q >> 2)) * dim * 16 + u * 16 + (q & 3) * 4;
+    }
+}
+
+// Four residues as packed limb bytes (any 32-bit values; reduced mod p).
+__device__ __forceinline__ void limbs4(const uint4& x, const Mod& mod, uint32_t& lo, uint32_t& hi) {
+    const uint32_t v[4] = {x.x, x.y, x.z, x.w};
+    int32_t l[4], h[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        split_limbs(to_balanced(reduce_u32(v[j], mod), mod), l[j], h[j]);
+    }
+    lo = pack_bytes(l[0], l[1], l[2], l[3]);
+    hi = pack_bytes(h[0], h[1], h[2], h[3]);
+}
+
+// canonical row-major (rows x w_in) -> four planes of NB columns (columns
+// w_in..NB-1 are zero); rows below 2^32
+template <int NB>
+__global__ void __launch_bounds__(256) to_limbs_kernel(const uint32_t* __restrict__ in, int8_t* __restrict__ lo,
+                                                       int8_t* __restrict__ hi, int8_t* __restrict__ nlo,
+                                                       int8_t* __restrict__ nhi, long long quads, uint32_t dim,
+                                                       uint32_t w_in, bool aligned, Mod mod) {
+    constexpr uint32_t Q = NB / 4;
+    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < quads; i += stride) {
+        const uint32_t row = static_cast<uint32_t>(i / Q), q = static_cast<uint32_t>(i) % Q;
+        uint32_t a = 0, b = 0;
+        if (q * 4 < w_in) limbs4(load_quad(in + static_cast<size_t>(row) * w_in + q * 4, aligned), mod, a, b);
+        const size_t off = quad_offset<NB>(row, q, dim);
+        *reinterpret_cast<uint32_t*>(lo + off) = a;
+        *reinterpret_cast<uint32_t*>(hi + off) = b;
+        *reinterpret_cast<uint32_t*>(nlo + off) = neg_bytes4(a);
+        *reinterpret_cast<uint32_t*>(nhi + off) = neg_bytes4(b);
     }
 }
 
 // four planes of NB columns -> canonical row-major with the first w_out columns
 template <int NB>
-__global__ void from_limbs_kernel(const int8_t* __restrict__ lo, const int8_t* __restrict__ hi,
-                                  uint32_t* __restrict__ out, long long count, int dim, int w_out, Mod mod) {
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < count;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const long long row = i / w_out;
-        const int j = static_cast<int>(i - row * w_out);
-        const long long blk = row / dim;
-        const long long off = plane_offset(blk, static_cast<int>(row - blk * dim), j, dim, NB);
-        out[i] = to_canonical(reduce_balanced(255 * static_cast<int32_t>(hi[off]) + lo[off], mod), mod);
+__global__ void __launch_bounds__(256) from_limbs_kernel(const int8_t* __restrict__ lo, const int8_t* __restrict__ hi,
+                                                         uint32_t* __restrict__ out, long long quads, uint32_t dim,
+                                                         uint32_t w_shift, bool aligned, Mod mod) {
+    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < quads; i += stride) {
+        const uint32_t row = static_cast<uint32_t>(i >> w_shift), q = static_cast<uint32_t>(i) & ((1u << w_shift) - 1);
+        const size_t off = quad_offset<NB>(row, q, dim);
+        const uint32_t a = __ldg(reinterpret_cast<const uint32_t*>(lo + off));
+        const uint32_t b = __ldg(reinterpret_cast<const uint32_t*>(hi + off));
+        uint32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int32_t x = 255 * static_cast<int8_t>(b >> (8 * j)) + static_cast<int8_t>(a >> (8 * j));
+            v[j] = to_canonical(reduce_balanced_fast(x, mod), mod);
+        }
+        store_quad(out + i * 4, make_uint4(v[0], v[1], v[2], v[3]), aligned);
     }
 }
 
@@ -1048,27 +1083,24 @@ __global__ void __launch_bounds__(kProjThreads, 1) i8_project_tc_kernel(I8Proj P
 // X (canonical, rows x m) -> the projection's A tiles [stage][2 MG][KP][16]:
 // group g < MG holds the lo limbs of columns 16 g .. 16 g + 15, group MG + g
 // their hi limbs; rows past the stage's SB * dim, past the last row or columns
-// past m are zero.
-__global__ void x_tiles_kernel(const uint32_t* __restrict__ X, int8_t* __restrict__ xt, long long rows, int m,
-                               int mg, int dim, int sb, int kp, long long n_units, Mod mod) {
-    for (long long q = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; q < n_units;
-         q += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const long long per_stage = 2LL * mg * kp;
-        const long long st = q / per_stage;
-        const int rem = static_cast<int>(q - st * per_stage);
-        const int g = rem / kp, kr = rem - (rem / kp) * kp;
+// past m are zero.  A thread takes four columns of one row, both limbs.
+__global__ void __launch_bounds__(256) x_tiles_kernel(const uint32_t* __restrict__ X, int8_t* __restrict__ xt,
+                                                      long long rows, int m, int mg, int dim, int sb, int kp,
+                                                      long long quads, bool aligned, Mod mod) {
+    const uint32_t per_stage = static_cast<uint32_t>(mg) * kp * 4;   // quads
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < quads;
+         i += static_cast<long long>(gridDim.x) * blockDim.x) {
+        const long long st = i / per_stage;
+        const uint32_t rem = static_cast<uint32_t>(i - st * per_stage);
+        const uint32_t q = rem % 4, gk = rem / 4, g = gk / kp, kr = gk - g * kp;
         const long long row = st * sb * dim + kr;
-        const bool valid = kr < sb * dim && row < rows;
-        const int limb = g / mg, x0 = (g % mg) * 16;
-        uint32_t packed[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int xi = 0; xi < 16; ++xi) {
-            const int x = x0 + xi;
-            int8_t lo = 0, hi = 0;
-            if (valid && x < m) split_limbs(to_balanced(X[row * m + x] % static_cast<uint32_t>(mod.p), mod), lo, hi);
-            packed[xi / 4] |= static_cast<uint32_t>(static_cast<uint8_t>(limb ? hi : lo)) << (8 * (xi % 4));
-        }
-        *reinterpret_cast<uint4*>(xt + q * 16) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        const int x0 = static_cast<int>(g) * 16 + static_cast<int>(q) * 4;
+        uint32_t a = 0, b = 0;
+        if (kr < static_cast<uint32_t>(sb * dim) && row < rows && x0 < m)
+            limbs4(load_quad(X + row * m + x0, aligned), mod, a, b);
+        int8_t* at = xt + ((st * 2 * mg + g) * kp + kr) * 16 + q * 4;
+        *reinterpret_cast<uint32_t*>(at) = a;
+        *reinterpret_cast<uint32_t*>(at + static_cast<size_t>(mg) * kp * 16) = b;
     }
 }
 
@@ -1112,7 +1144,8 @@ struct KoszulCtx::I8State {
     int8_t* xt = nullptr;
     size_t proj_smem = 0;
     unsigned proj_grid = 0;
-    int* err = nullptr;
+    int* err = nullptr;        // the kernels' error word (device address)
+    volatile int* h_err = nullptr;   // the same word: mapped host memory, written only when a kernel gives up
 };
 
 namespace {
@@ -1579,6 +1612,7 @@ void launch_i8(KoszulCtx& c, KoszulCtx::I8State::Dir& D, const CUtensorMap* maps
 }  // namespace
 
 void KoszulCtx::i8_destroy() {
+    if (i8 != nullptr && i8->h_err != nullptr) cudaFreeHost(const_cast<int*>(i8->h_err));
     delete i8;
     i8 = nullptr;
 }
@@ -1605,8 +1639,11 @@ void KoszulCtx::i8_setup() {
             S.planes[b][limb + 2] = pair + plane;
         }
     }
-    S.err = alloc<int>(1);
-    BW_CUDA(cudaMemsetAsync(S.err, 0, sizeof(int), own_stream));
+    void* word = nullptr;
+    BW_CUDA(cudaHostAlloc(&word, sizeof(int), cudaHostAllocMapped));
+    S.h_err = static_cast<volatile int*>(word);
+    *S.h_err = 0;
+    BW_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&S.err), word, 0));
     plan_projection(*this, S);
     const int hg = nbi / 16;
     // The producers that may be used.  BW_I8_PRODUCER=union, =cpasync or
@@ -1898,10 +1935,9 @@ void KoszulCtx::i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cu
 }
 
 void KoszulCtx::i8_check_error() {
-    int err = 0;
-    BW_CUDA(cudaMemcpy(&err, i8->err, sizeof(int), cudaMemcpyDeviceToHost));
+    const int err = *i8->h_err;   // the caller has synchronised with the kernels
     if (err != 0) {
-        cudaMemset(i8->err, 0, sizeof(int));
+        *i8->h_err = 0;
         static const char* const names[] = {"", "ERR_WAIT_FULL: consumer waited for a loaded stage",
                                             "ERR_WAIT_EMPTY: producer waited for a free stage",
                                             "ERR_WAIT_ACCUM: epilogue waited for an accumulator",
@@ -1917,24 +1953,25 @@ int KoszulCtx::i8_dim(int buf) const { return buf == I8_Z ? co : ci; }
 uint64_t KoszulCtx::i8_rows(int buf) const { return buf == I8_Z ? n_tgt : n_src; }
 
 void KoszulCtx::i8_to_limbs(const uint32_t* in, int buf, cudaStream_t st) {
-    const uint64_t count = i8_rows(buf) * nbi;
-    unsigned grid = static_cast<unsigned>(std::min<uint64_t>((count + 255) / 256, static_cast<uint64_t>(sms) * 8));
+    const uint64_t quads = i8_rows(buf) * nbi / 4;
     int8_t** pl = i8->planes[buf];
     dispatch_i8_nb(nbi, [&](auto NBc) {
-        to_limbs_kernel<decltype(NBc)::value><<<std::max(grid, 1u), 256, 0, st>>>(
-            in, pl[0], pl[1], pl[2], pl[3], static_cast<long long>(count), i8_dim(buf), nb, mod);
+        to_limbs_kernel<decltype(NBc)::value><<<quad_grid(quads, sms), 256, 0, st>>>(
+            in, pl[0], pl[1], pl[2], pl[3], static_cast<long long>(quads), static_cast<uint32_t>(i8_dim(buf)),
+            static_cast<uint32_t>(nb), quad_aligned(in), mod);
     });
     BW_CHECK_LAUNCH();
     ++launches;
 }
 
 void KoszulCtx::i8_from_limbs(int buf, uint32_t* out, cudaStream_t st) {
-    const uint64_t count = i8_rows(buf) * nb;
-    unsigned grid = static_cast<unsigned>(std::min<uint64_t>((count + 255) / 256, static_cast<uint64_t>(sms) * 8));
+    const uint64_t quads = i8_rows(buf) * nb / 4;
+    const uint32_t w_shift = nb == 4 ? 0 : nb == 8 ? 1 : nb == 16 ? 2 : 3;
     int8_t** pl = i8->planes[buf];
     dispatch_i8_nb(nbi, [&](auto NBc) {
-        from_limbs_kernel<decltype(NBc)::value><<<std::max(grid, 1u), 256, 0, st>>>(
-            pl[0], pl[1], out, static_cast<long long>(count), i8_dim(buf), nb, mod);
+        from_limbs_kernel<decltype(NBc)::value><<<quad_grid(quads, sms), 256, 0, st>>>(
+            pl[0], pl[1], out, static_cast<long long>(quads), static_cast<uint32_t>(i8_dim(buf)), w_shift,
+            quad_aligned(out), mod);
     });
     BW_CHECK_LAUNCH();
     ++launches;
@@ -1942,10 +1979,9 @@ void KoszulCtx::i8_from_limbs(int buf, uint32_t* out, cudaStream_t st) {
 
 void KoszulCtx::i8_load_x(const uint32_t* x, cudaStream_t st) {
     const I8Proj& P = i8->proj;
-    const long long units = static_cast<long long>(P.n_stages) * 2 * P.mg * P.kp;
-    unsigned grid = static_cast<unsigned>(std::min<long long>((units + 255) / 256, static_cast<long long>(sms) * 8));
-    x_tiles_kernel<<<std::max(grid, 1u), 256, 0, st>>>(x, i8->xt, static_cast<long long>(n_src), m, P.mg, ci, P.sb,
-                                                        P.kp, units, mod);
+    const long long quads = static_cast<long long>(P.n_stages) * P.mg * P.kp * 4;
+    x_tiles_kernel<<<quad_grid(quads, sms), 256, 0, st>>>(x, i8->xt, static_cast<long long>(n_src), m, P.mg, ci, P.sb,
+                                                          P.kp, quads, quad_aligned(x), mod);
     BW_CHECK_LAUNCH();
     ++launches;
 }

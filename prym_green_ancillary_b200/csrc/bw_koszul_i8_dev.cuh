@@ -64,6 +64,11 @@ __host__ __device__ __forceinline__ void split_limbs(int32_t v, int8_t& lo, int8
     hi = static_cast<int8_t>(h);
 }
 
+// The low bytes of four values in one word.
+__device__ __forceinline__ uint32_t pack_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+}
+
 // 16 x 16 byte transpose inside each half-warp.  On entry lane L (L = lane & 15)
 // holds row L as four words (byte b of word q = element 4q + b); on exit it
 // holds column L the same way.  Two butterfly stages exchange words (lane bits

@@ -112,11 +112,6 @@ __device__ __forceinline__ int32_t union_value(int32_t lo, int32_t hi, const Mod
     return scale ? near_shifted((v - mod.half) * dg, mod) : v;
 }
 
-// The low bytes of four values in one word.
-__device__ __forceinline__ uint32_t pack_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
-}
-
 // The limbs of four values v - half as packed bytes: with x = v - half + 127 +
 // 255 * 128 (16 bits) and q = floor(x / 255), hi = q - 128 and lo = v - half -
 // 255 hi, whose low byte is that of v - half + hi.
