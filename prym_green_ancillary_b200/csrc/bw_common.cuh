@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <stdexcept>
 #include <string>
+#include <utility>
 
 namespace bw {
 
@@ -164,6 +165,32 @@ __host__ __device__ __forceinline__ uint32_t to_canonical(int32_t balanced, cons
 }
 
 #if defined(__CUDACC__)
+// Programmatic dependent launch.  A kernel launched by launch_dependent() may
+// begin (barriers, TMEM, constant tables) while the kernel before it on the
+// stream is still finishing; pdl_wait() blocks until that kernel has completed
+// and its writes are visible, so it comes before the first access to anything
+// an earlier kernel reads or writes.  pdl_trigger() lets the next kernel begin
+// early.  Every kernel launched this way calls pdl_wait(), so a kernel's
+// completion implies that of all kernels before it.  Without the attribute
+// both are no-ops.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    BW_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
+}
+
 // Four consecutive residues of a caller's buffer: one 16-byte access where the
 // buffer is 16-byte aligned (the offset is a multiple of four), else four.
 __device__ __forceinline__ uint4 load_quad(const uint32_t* p, bool aligned) {

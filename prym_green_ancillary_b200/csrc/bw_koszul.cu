@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(256) gather_mac_kernel(
     }
 }
 
-// Projection a = X^T W (m x n) of one block into seq[*seq_index].  Every CTA
+// Projection a = X^T W (m x n) of one block into state->seq[state->index].  Every CTA
 // adds its m x n balanced sums into one int32 accumulator with atomics (at
 // most 4 * 148 CTAs x (p-1)/2, far below 2^31: exact, and the same whatever
 // the order of the additions); the last CTA to finish reads and clears it.
@@ -169,7 +169,7 @@ template <int NB>
 __global__ void __launch_bounds__(256) project_kernel(
     const int32_t* __restrict__ X, const int32_t* __restrict__ W, long long rows, int m,
     int32_t* __restrict__ partials, unsigned int* __restrict__ counter,
-    uint32_t* __restrict__ seq, unsigned long long* __restrict__ seq_index, Mod mod) {
+    SeqState* __restrict__ state, Mod mod) {
     constexpr int JG = NB / 4;
     const int tps = m * JG;                       // threads per row slice
     const int slices = blockDim.x / tps;
@@ -236,15 +236,26 @@ __global__ void __launch_bounds__(256) project_kernel(
     __syncthreads();
     if (!am_last) return;
     __threadfence();
-    const unsigned long long pos = *reinterpret_cast<volatile unsigned long long*>(seq_index);
+    const unsigned long long pos = state->index;
+    uint32_t* seq = state->seq;
     const int entries = m * NB;
     for (int e = threadIdx.x; e < entries; e += blockDim.x)
         seq[pos * entries + e] = to_canonical(reduce_balanced(atomicExch(partials + e, 0), mod), mod);
     __syncthreads();
     if (threadIdx.x == 0) {
-        *seq_index = pos + 1;
+        state->index = pos + 1;
         *counter = 0;
         __threadfence();
+    }
+}
+
+// A session's start: the buffer, no entries, clear projection scratch.
+__global__ void seq_begin_kernel(SeqState* state, uint32_t* seq, unsigned int* counter, int32_t* partials, int n) {
+    for (int e = threadIdx.x; e < n; e += blockDim.x) partials[e] = 0;
+    if (threadIdx.x == 0) {
+        state->index = 0;
+        state->seq = seq;
+        *counter = 0;
     }
 }
 
@@ -322,7 +333,7 @@ void launch_gather(KoszulCtx& c, const int32_t* in, int32_t* out, const uint32_t
 template <int NB>
 void launch_project(KoszulCtx& c, const int32_t* W, cudaStream_t st) {
     project_kernel<NB><<<c.proj_grid, 256, 0, st>>>(c.d_xb, W, static_cast<long long>(c.n_src), c.m,
-                                                    c.d_partials, c.d_counter, c.d_seq, c.d_seq_index, c.mod);
+                                                    c.d_partials, c.d_counter, c.d_seq_state, c.mod);
     BW_CHECK_LAUNCH();
     ++c.launches;
 }
@@ -537,10 +548,8 @@ KoszulCtx* KoszulCtx::create(const bw_koszul_desc& d, int dev) {
     // per-CTA partial sums: the plain projection's grid, or up to one CTA per SM for the INT8 form
     c->d_partials = c->alloc<int32_t>(std::max<uint64_t>(c->proj_grid, c->sms) * c->m * std::max(c->nb, c->nbi));
     c->d_counter = c->alloc<unsigned int>(1);
-    c->d_seq_index = c->alloc<unsigned long long>(1);
+    c->d_seq_state = c->alloc<SeqState>(1);
     c->scratch_bytes = c->device_bytes - scratch_before;
-    BW_CUDA(cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned int), st));
-    BW_CUDA(cudaMemsetAsync(c->d_seq_index, 0, sizeof(unsigned long long), st));
     if (c->form == BW_FORM_INT8) c->i8_setup();
     if (c->form == BW_FORM_PLAIN) c->plain_setup();
     BW_CUDA(cudaStreamSynchronize(st));
@@ -620,6 +629,7 @@ void KoszulCtx::plain_setup() {
     g_plain_tiles[key] = {tile_fwd, tile_bwd};
 }
 
+template SeqState* KoszulCtx::alloc<SeqState>(uint64_t);
 template int8_t* KoszulCtx::alloc<int8_t>(uint64_t);
 template int16_t* KoszulCtx::alloc<int16_t>(uint64_t);
 template int* KoszulCtx::alloc<int>(uint64_t);
@@ -641,12 +651,11 @@ void KoszulCtx::seq_start(const uint32_t* x, const uint32_t* y0, uint32_t* seq, 
                           cudaStream_t st) {
     BW_ARG(x != nullptr && y0 != nullptr && seq != nullptr, "seq_start: null buffer");
     BW_REQUIRE(capacity >= 1, "seq_start: sequence capacity must be at least 1");
-    d_seq = seq;
     seq_capacity = capacity;
     cur_is_a = true;
-    BW_CUDA(cudaMemsetAsync(d_seq_index, 0, sizeof(unsigned long long), st));
-    BW_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(unsigned int), st));
-    BW_CUDA(cudaMemsetAsync(d_partials, 0, static_cast<size_t>(m) * std::max(nb, nbi) * sizeof(int32_t), st));
+    seq_begin_kernel<<<1, 256, 0, st>>>(d_seq_state, seq, d_counter, d_partials, m * std::max(nb, nbi));
+    BW_CHECK_LAUNCH();
+    ++launches;
     if (form == BW_FORM_INT8) {
         i8_load_x(x, st);
         i8_to_limbs(y0, I8_YA, st);
@@ -657,16 +666,6 @@ void KoszulCtx::seq_start(const uint32_t* x, const uint32_t* y0, uint32_t* seq, 
         project(d_ya, st);
     }
     seq_len = 1;
-    // The step graphs capture device pointers: all are the context's own but
-    // the sequence buffer, so a session with another buffer recaptures them.
-    if (seq != graph_seq) {
-        for (auto& g : graphs)
-            if (g) {
-                cudaGraphExecDestroy(g);
-                g = nullptr;
-            }
-        graph_seq = seq;
-    }
     in_session = true;
 }
 

@@ -11,6 +11,13 @@
 
 namespace bw {
 
+// Where the projection appends (device memory, so that captured steps serve
+// every session whatever its buffer): entries written so far, and the buffer.
+struct SeqState {
+    unsigned long long index;
+    uint32_t* seq;
+};
+
 struct KoszulCtx {
     // shape
     int device = 0, sms = 0;
@@ -37,15 +44,13 @@ struct KoszulCtx {
     unsigned proj_grid = 1;
     int32_t* d_partials = nullptr;
     unsigned int* d_counter = nullptr;
-    unsigned long long* d_seq_index = nullptr;
+    SeqState* d_seq_state = nullptr;
 
     // sequence session
     bool in_session = false, cur_is_a = true;
-    uint32_t* d_seq = nullptr;
     uint64_t seq_capacity = 0, seq_len = 0;
     static constexpr int kGraphPairs = 8;
     cudaGraphExec_t graphs[2] = {nullptr, nullptr};
-    const uint32_t* graph_seq = nullptr;   // the sequence buffer the step graphs write
     uint64_t graph_launch_kernels = 0;
     uint64_t launches = 0;
 

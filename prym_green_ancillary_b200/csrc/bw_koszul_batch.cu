@@ -42,14 +42,6 @@ struct KoszulBatch {
         if (own_stream) cudaStreamDestroy(own_stream);
     }
 
-    void drop_graphs() {
-        for (auto& g : graphs)
-            if (g) {
-                cudaGraphExecDestroy(g);
-                g = nullptr;
-            }
-    }
-
     bool parity() const { return sectors.front()->cur_is_a; }
 
     void step_direct(cudaStream_t st) {
@@ -185,7 +177,6 @@ extern "C" int bw_koszul_batch_seq_start(bw_koszul_batch* batch, const uint32_t*
         b.capacity = seq_capacity;
         b.seq_len = 1;
         b.in_session = true;
-        b.drop_graphs();   // new sequence buffers
     });
 }
 

@@ -872,7 +872,8 @@ __global__ void __launch_bounds__(256) from_limbs_kernel(const int8_t* __restric
 // Warps: 0 producer (bulk copies: the stage's X tile and W block runs), 1 MMA
 // issuer (allocates TMEM), 2-5 epilogue (tcgen05.ld + reduction mod p).  The
 // CTA's combined sums are added into an m x n int32 accumulator; the last CTA
-// to finish writes them to seq[*seq_index], clears them and advances the index.
+// to finish writes them to the session's buffer, clears them and advances the
+// index.
 constexpr int kProjThreads = 6 * 32;
 constexpr int kProjStageTarget = 32 * 1024;   // bytes of X tile + W runs per stage
 
@@ -881,8 +882,7 @@ struct I8Proj {
     const int8_t* w[2];         // W lo, hi planes: [blk][h][u][16]
     int32_t* partials;          // [m][NB] accumulator, zero between launches
     unsigned int* counter;
-    uint32_t* seq;
-    unsigned long long* seq_index;
+    SeqState* state;
     int* err;
     long long n_blk;
     int dim, m, mg, sb, kp, n_stages, slots, drain;
@@ -912,6 +912,7 @@ __global__ void __launch_bounds__(kProjThreads, 1) i8_project_tc_kernel(I8Proj P
     const long long n_my = blockIdx.x < P.n_stages ? (P.n_stages - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const long long n_chunks = (n_my + P.drain - 1) / P.drain;
     const uint32_t tmem_cols = 2 * N;   // two accumulators (64 or 128 columns)
+    pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.slots; ++s) {
             tc::mbar_init(&full[s], 1);
@@ -934,6 +935,7 @@ __global__ void __launch_bounds__(kProjThreads, 1) i8_project_tc_kernel(I8Proj P
     tc::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t run_bytes = static_cast<uint32_t>(P.dim) * 16;   // one (block, h) run of a plane
+    pdl_wait();
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
@@ -1064,17 +1066,18 @@ __global__ void __launch_bounds__(kProjThreads, 1) i8_project_tc_kernel(I8Proj P
     __syncthreads();
     if (!am_last) return;
     __threadfence();
-    const unsigned long long pos = *reinterpret_cast<volatile unsigned long long*>(P.seq_index);
+    const unsigned long long pos = P.state->index;
+    uint32_t* seq = P.state->seq;
     for (int e = threadIdx.x; e < entries; e += blockDim.x) {
         const int x = e / NB, j = e - (e / NB) * NB;
         const int32_t sum = atomicExch(P.partials + e, 0);
         if (j >= P.n_out) continue;
-        P.seq[pos * (static_cast<unsigned long long>(P.m) * P.n_out) + x * P.n_out + j] =
+        seq[pos * (static_cast<unsigned long long>(P.m) * P.n_out) + x * P.n_out + j] =
             to_canonical(reduce_balanced(sum, P.mod), P.mod);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        *P.seq_index = pos + 1;
+        P.state->index = pos + 1;
         *P.counter = 0;
         __threadfence();
     }
@@ -1590,9 +1593,9 @@ void launch_i8(KoszulCtx& c, KoszulCtx::I8State::Dir& D, const CUtensorMap* maps
         BW_REQUIRE(D.u.start != nullptr && D.u.words != nullptr && D.u.steps != nullptr && D.u.maps != nullptr,
                    "internal: INT8 stage list missing for the union kernel");
         if (D.pw == 16)
-            i8_union_gemm_kernel<NB, 16><<<D.grid, GatherWarps<16>::threads, D.smem, st>>>(D.u);
+            launch_dependent(i8_union_gemm_kernel<NB, 16>, D.grid, GatherWarps<16>::threads, D.smem, st, D.u);
         else
-            i8_union_gemm_kernel<NB, 8><<<D.grid, GatherWarps<8>::threads, D.smem, st>>>(D.u);
+            launch_dependent(i8_union_gemm_kernel<NB, 8>, D.grid, GatherWarps<8>::threads, D.smem, st, D.u);
         BW_CHECK_LAUNCH();
         ++c.launches;
         return;
@@ -1992,10 +1995,9 @@ void KoszulCtx::i8_project(int buf, cudaStream_t st) {
     P.w[1] = i8->planes[buf][1];
     P.partials = d_partials;
     P.counter = d_counter;
-    P.seq = d_seq;
-    P.seq_index = d_seq_index;
+    P.state = d_seq_state;
     dispatch_i8_nb(nbi, [&](auto NBc) {
-        i8_project_tc_kernel<decltype(NBc)::value><<<i8->proj_grid, kProjThreads, i8->proj_smem, st>>>(P);
+        launch_dependent(i8_project_tc_kernel<decltype(NBc)::value>, i8->proj_grid, kProjThreads, i8->proj_smem, st, P);
     });
     BW_CHECK_LAUNCH();
     ++launches;

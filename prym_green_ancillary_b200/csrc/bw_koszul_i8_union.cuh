@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(GatherWarps<PW>::threads, 1) i8_union_gemm_ker
     // the warp index through a shuffle, so that role and pass branches are uniform
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0), lane = threadIdx.x % 32;
     const long long n_tiles = (P.n_blk + BT - 1) / BT;
+    pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.slots; ++s) {
             tc::mbar_init(&full[s], W::producers / P.groups * 32);   // per thread: its copies have landed
@@ -217,6 +218,7 @@ __global__ void __launch_bounds__(GatherWarps<PW>::threads, 1) i8_union_gemm_ker
         uint32_t word0 = has_word && group < n_stages ? __ldg(tab) : kSkip;
         uint32_t word1 = has_word && group + P.groups < n_stages ? __ldg(tab + tab_step) : kSkip;
         tab += 2 * tab_step;
+        pdl_wait();   // the input planes; the maps and lists are constant
         for (int left = n_stages - group; left > 0; left -= P.groups) {
             const uint32_t word = word0;
             word0 = word1;
@@ -356,6 +358,7 @@ __global__ void __launch_bounds__(GatherWarps<PW>::threads, 1) i8_union_gemm_ker
                 for (int oo = 0; oo < 16; ++oo) dg[oo] = any && c * 16 + oo < P.outer ? __ldg(src + oo) : 0;
             }
         };
+        pdl_wait();   // the output planes may still be read, and the diagonal be written, by earlier kernels
         // a tile's first chunk is loaded one tile ahead (the diagonal streams from DRAM)
         int32_t dg_next[16];
         load_diag(dg_next, blockIdx.x, part);
