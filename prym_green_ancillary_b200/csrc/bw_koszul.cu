@@ -9,13 +9,14 @@
 //   X     : n_src x m
 // so one subset's block is one contiguous run of dim * n residues.
 //
-// Incidence tables (built once on the host):
+// Incidence tables (built once, on the device):
 //   fwd[T][q], q < r-k+1 : the subsets S = T u {i}, i not in T
 //   bwd[S][q], q < k     : the subsets T = S \ {i},  i in S
 // each entry = subset rank | i << 26 | negative << 31, with the entries of a
 // row ordered positive signs first so that a kernel flips its accumulator sign
 // at most once per output block.
 #include "bw_koszul.cuh"
+#include "bw_koszul_tables.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -33,21 +34,31 @@ namespace bw {
 
 namespace {
 
-// acc[o0 + a][j] += coef[a] * y[j] for the four coefficients of one int4
+// acc[o0 + a][j] += coef[a] * y[j] for the (at most four) rows of a tile that one int4 of coefficients covers
 template <int TO>
-__device__ __forceinline__ void mac4(int32_t (&acc)[TO][4], int o0, const int4& a, const int4& y) {
-    acc[o0][0] += a.x * y.x; acc[o0][1] += a.x * y.y; acc[o0][2] += a.x * y.z; acc[o0][3] += a.x * y.w;
-    acc[o0 + 1][0] += a.y * y.x; acc[o0 + 1][1] += a.y * y.y; acc[o0 + 1][2] += a.y * y.z; acc[o0 + 1][3] += a.y * y.w;
-    acc[o0 + 2][0] += a.z * y.x; acc[o0 + 2][1] += a.z * y.y; acc[o0 + 2][2] += a.z * y.z; acc[o0 + 2][3] += a.z * y.w;
-    acc[o0 + 3][0] += a.w * y.x; acc[o0 + 3][1] += a.w * y.y; acc[o0 + 3][2] += a.w * y.z; acc[o0 + 3][3] += a.w * y.w;
+__device__ __forceinline__ void mac4(int32_t (&acc)[TO][4], int o0, const int4& coef, const int4& y) {
+    const int32_t c[4] = {coef.x, coef.y, coef.z, coef.w};
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        if (o0 + a >= TO) break;
+        acc[o0 + a][0] += c[a] * y.x;
+        acc[o0 + a][1] += c[a] * y.y;
+        acc[o0 + a][2] += c[a] * y.z;
+        acc[o0 + a][3] += c[a] * y.w;
+    }
 }
 
+// Keeps the accumulators inside int32 between chunks of eight products:
+// x = (x mod 2^s) + (x >> s) c with c = 2^s mod p (balanced), one multiply-add
+// and two operations of the other integer pipe (a Barrett step is a
+// multiply-high and a multiply-add).  The host's choice of s leaves room for
+// eight more products (plan_fold).
 template <int TO>
-__device__ __forceinline__ void reduce_tile(int32_t (&acc)[TO][4], const Mod& mod) {
+__device__ __forceinline__ void reduce_tile(int32_t (&acc)[TO][4], const Fold& fold) {
 #pragma unroll
     for (int a = 0; a < TO; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = reduce_partial(acc[a][b], mod);
+        for (int b = 0; b < 4; ++b) acc[a][b] = (acc[a][b] & fold.mask) + (acc[a][b] >> fold.shift) * fold.c;
 }
 
 template <int TO>
@@ -65,29 +76,36 @@ __device__ __forceinline__ void negate_tile(int32_t (&acc)[TO][4]) {
 // d   : blk = T, o = c (dim_out), u = b (dim_in),  coef = M^T  (i x b x c)
 // d^T : blk = S, o = b (dim_in),  u = c (dim_out), coef = M    (i x c x b)
 //
-// A thread owns a TO (o) x 4 (j) register tile of one output block (TO = 4 or
-// 8: an 8-row tile does twice the multiply-adds per gathered 16-byte row); the
-// coefficient tiles of all r maps sit in shared memory ([i][u][o], rows of
-// `ostride` = outer rounded up to 8, zero-padded), the gathered input rows
-// stream from L2 as 16-byte loads.  Sums of 8 balanced products stay inside
-// int32 next to a partially reduced value, so the accumulator is reduced every
+// A thread owns a TO (o) x 4 (j) register tile of one output block (4 to 8
+// rows: more rows are more multiply-adds per gathered 16-byte row, and the
+// rows of a block are dealt evenly, so that 28 are four tiles of 7 and 17
+// three of 6, with little padding; measured at r = 19, k = 9, 20 -> 28, 16
+// columns: d 0.726 ms with 8 rows, 0.655 with 7); the coefficient tiles of all r maps sit in
+// shared memory ([i][u][tile][TO rounded up to 4], zero-padded), the gathered
+// input rows stream from L2 as 16-byte loads.  Sums of 8 balanced products
+// stay inside int32 next to a folded value, so the accumulator is folded every
 // 8 u-steps.
+//
+// Bound by the integer multiply pipe (64 IMADs a cycle and SM): 18.6 T/s, of
+// which r = 20, k = 9, 32 -> 40, 32 columns reaches 11.9 T products/s in d and
+// 12.6 in d^T (10.0 and 10.6 with a Barrett step for a fold).  Splitting a
+// thread's rows between IMADs and exact fp64 multiply-adds was slower (6.7
+// against 5.2 ms there).
 template <int NB, int TO>
-__global__ void __launch_bounds__(256) gather_mac_kernel(
+__global__ void __launch_bounds__(256, TO == 4 ? 3 : 1) gather_mac_kernel(
     const int32_t* __restrict__ in, int32_t* __restrict__ out,
-    const uint32_t* __restrict__ inc, const int32_t* __restrict__ coef,
+    const uint32_t* __restrict__ inc, const int4* __restrict__ coef,
     const int32_t* __restrict__ diag,   // nullptr: no scaling
-    long long n_blk, int width, int r, int inner, int outer, int ostride, Mod mod) {
-    extern __shared__ int4 smem_raw[];
-    int32_t* sm = reinterpret_cast<int32_t*>(smem_raw);
-    const int total = r * inner * ostride;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) sm[e] = coef[e];
+    long long n_blk, int width, int r, int inner, int outer, Mod mod, Fold fold) {
+    extern __shared__ int4 sm4[];
+    constexpr int JG = NB / 4;
+    constexpr int TQ = (TO + 3) / 4;               // int4 coefficient loads per u-step
+    const int OG = (outer + TO - 1) / TO;
+    const int row4 = OG * TQ;                      // int4 of one u
+    const int total = r * inner * row4;
+    for (int e = threadIdx.x; e < total; e += blockDim.x) sm4[e] = __ldg(coef + e);
     __syncthreads();
 
-    constexpr int JG = NB / 4;
-    constexpr int TQ = TO / 4;                     // int4 coefficient loads per u-step
-    const int OG = (outer + TO - 1) / TO;
-    const int OS4 = ostride / 4;
     const int tpb = OG * JG;                       // threads per output block
     const int bpc = blockDim.x / tpb;              // output blocks per CTA pass
     const int local = threadIdx.x / tpb;
@@ -96,7 +114,6 @@ __global__ void __launch_bounds__(256) gather_mac_kernel(
     const int jg = sub - og * JG;
     if (local >= bpc) return;                      // no barrier below this point
 
-    const int4* sm4 = reinterpret_cast<const int4*>(sm);
     for (long long blk = static_cast<long long>(blockIdx.x) * bpc + local; blk < n_blk;
          blk += static_cast<long long>(gridDim.x) * bpc) {
         int32_t acc[TO][4];
@@ -121,7 +138,7 @@ __global__ void __launch_bounds__(256) gather_mac_kernel(
                 neg_state = neg;
             }
             const int4* irow = reinterpret_cast<const int4*>(in + s * inner * NB) + jg;
-            const int4* crow = sm4 + static_cast<size_t>(i) * inner * OS4 + og * TQ;
+            const int4* crow = sm4 + static_cast<size_t>(i) * inner * row4 + og * TQ;
             for (int u0 = 0; u0 < inner; u0 += 8) {
                 int4 y[8];
 #pragma unroll
@@ -131,9 +148,9 @@ __global__ void __launch_bounds__(256) gather_mac_kernel(
                 for (int uu = 0; uu < 8; ++uu) {
                     if (u0 + uu >= inner) break;
 #pragma unroll
-                    for (int t = 0; t < TQ; ++t) mac4<TO>(acc, 4 * t, crow[(u0 + uu) * OS4 + t], y[uu]);
+                    for (int t = 0; t < TQ; ++t) mac4<TO>(acc, 4 * t, crow[(u0 + uu) * row4 + t], y[uu]);
                 }
-                reduce_tile<TO>(acc, mod);
+                reduce_tile<TO>(acc, fold);
             }
         }
         if (neg_state) negate_tile<TO>(acc);
@@ -161,72 +178,70 @@ __global__ void __launch_bounds__(256) gather_mac_kernel(
 
 // Projection a = X^T W (m x n) of one block into state->seq[state->index].  Every CTA
 // adds its m x n balanced sums into one int32 accumulator with atomics (at
-// most 4 * 148 CTAs x (p-1)/2, far below 2^31: exact, and the same whatever
+// most 2 * 148 CTAs x (p-1)/2, far below 2^31: exact, and the same whatever
 // the order of the additions); the last CTA to finish reads and clears it.
 //   partials : m x n int32 accumulator, left at 0 after every launch
 //   counter  : arrival counter, left at 0 after every launch
+// A thread owns a 4 x 4 tile of the m x n sums of its slice of rows, so a
+// row's two 16-byte loads feed sixteen multiply-adds (one scalar and one
+// 16-byte load for four of them were bound by the loads: 5.4 M rows of 32 x 32
+// 3.82 -> 0.64 ms, 1.85 M rows of 16 x 16 0.331 -> 0.082 ms; 18 T products/s
+// and 6.5 TB/s would be 0.34 and 0.036).  Eight rows' loads are in flight
+// together (hence two CTAs an SM), and eight products fit in int32 beside a
+// folded sum.
 template <int NB>
-__global__ void __launch_bounds__(256) project_kernel(
+__global__ void __launch_bounds__(256, 2) project_kernel(
     const int32_t* __restrict__ X, const int32_t* __restrict__ W, long long rows, int m,
-    int32_t* __restrict__ partials, unsigned int* __restrict__ counter,
-    SeqState* __restrict__ state, Mod mod) {
+    int32_t* __restrict__ partials, unsigned int* __restrict__ counter, SeqState* __restrict__ state, Mod mod,
+    Fold fold) {
     constexpr int JG = NB / 4;
-    const int tps = m * JG;                       // threads per row slice
+    const int tps = (m / 4) * JG;                 // threads per row slice, 1 to 64
     const int slices = blockDim.x / tps;
     const int slice = threadIdx.x / tps;
     const int sub = threadIdx.x - slice * tps;
-    const int x = sub / JG;
-    const int jg = sub - x * JG;
-    __shared__ int32_t red[256 * 4];
+    const int xg = sub / JG, jg = sub - xg * JG;
+    extern __shared__ int32_t red[];              // m x n sums of the CTA
     __shared__ bool am_last;
+    const int entries = m * NB;
+    for (int e = threadIdx.x; e < entries; e += blockDim.x) red[e] = 0;
+    __syncthreads();
 
-    int32_t acc[4] = {0, 0, 0, 0};
-    if (slice < slices) {
-        // four rows a pass, their loads in flight together; eight products of
-        // balanced residues beside a partially reduced value stay inside int32
+    int32_t acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = 0;
+    {   // 256 is a multiple of tps: every thread has a slice
+        const int4* x4 = reinterpret_cast<const int4*>(X) + xg;
+        const int4* w4 = reinterpret_cast<const int4*>(W) + jg;
+        const long long xs = m / 4;
         const long long stride = static_cast<long long>(gridDim.x) * slices;
         long long row = static_cast<long long>(blockIdx.x) * slices + slice;
-        for (; row + 3 * stride < rows; row += 4 * stride) {
-            int32_t xv[4];
-            int4 w[4];
+        for (; row + 7 * stride < rows; row += 8 * stride) {
+            int4 x[8], w[8];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                xv[q] = __ldg(X + (row + q * stride) * m + x);
-                w[q] = __ldg(reinterpret_cast<const int4*>(W + (row + q * stride) * NB) + jg);
+            for (int q = 0; q < 8; ++q) {
+                x[q] = __ldg(x4 + (row + q * stride) * xs);
+                w[q] = __ldg(w4 + (row + q * stride) * JG);
             }
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                acc[0] += xv[q] * w[q].x; acc[1] += xv[q] * w[q].y; acc[2] += xv[q] * w[q].z; acc[3] += xv[q] * w[q].w;
+            for (int q = 0; q < 8; ++q) mac4<4>(acc, 0, x[q], w[q]);
+            reduce_tile<4>(acc, fold);
+        }
+        for (; row < rows; row += stride) mac4<4>(acc, 0, __ldg(x4 + row * xs), __ldg(w4 + row * JG));   // at most 7
+        // the balanced sums of a warp's slices, then of the CTA's warps (at
+        // most 256 (p-1)/2: far below 2^31); tps is a power of two
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                int32_t v = reduce_balanced(acc[a][b], mod);
+                for (int off = 16; off >= tps; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                if ((threadIdx.x & 31) < tps) atomicAdd(&red[(xg * 4 + a) * NB + jg * 4 + b], v);
             }
-#pragma unroll
-            for (int a = 0; a < 4; ++a) acc[a] = reduce_partial(acc[a], mod);
-        }
-        for (; row < rows; row += stride) {
-            const int32_t xv = __ldg(X + row * m + x);
-            const int4 w = __ldg(reinterpret_cast<const int4*>(W + row * NB) + jg);
-            acc[0] += xv * w.x; acc[1] += xv * w.y; acc[2] += xv * w.z; acc[3] += xv * w.w;
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a) acc[a] = reduce_balanced(acc[a], mod);
     }
-#pragma unroll
-    for (int a = 0; a < 4; ++a) red[threadIdx.x * 4 + a] = acc[a];
     __syncthreads();
-    // Fold the slices: thread t < tps sums column t of the slice table.
-    if (threadIdx.x < tps) {
-        int32_t s[4] = {0, 0, 0, 0};
-        for (int sl = 0; sl < slices; ++sl) {
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                s[a] += red[(sl * tps + threadIdx.x) * 4 + a];
-                if ((sl & 7) == 7) s[a] = reduce_partial(s[a], mod);
-            }
-        }
-        const int xx = threadIdx.x / JG, jj = threadIdx.x - xx * JG;
-        int32_t* dst = partials + (static_cast<size_t>(xx) * NB + jj * 4);
-#pragma unroll
-        for (int a = 0; a < 4; ++a) atomicAdd(dst + a, reduce_balanced(s[a], mod));
-    }
+    for (int e = threadIdx.x; e < entries; e += blockDim.x) atomicAdd(partials + e, reduce_balanced(red[e], mod));
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -238,7 +253,6 @@ __global__ void __launch_bounds__(256) project_kernel(
     __threadfence();
     const unsigned long long pos = state->index;
     uint32_t* seq = state->seq;
-    const int entries = m * NB;
     for (int e = threadIdx.x; e < entries; e += blockDim.x)
         seq[pos * entries + e] = to_canonical(reduce_balanced(atomicExch(partials + e, 0), mod), mod);
     __syncthreads();
@@ -247,6 +261,21 @@ __global__ void __launch_bounds__(256) project_kernel(
         *counter = 0;
         __threadfence();
     }
+}
+
+// The plain gathers' incidence rows [blk][width]: rank | i << 26 | negative <<
+// 31, positive signs first (a row flips its accumulators' sign at most once).
+__global__ void plain_incidence_kernel(uint32_t* __restrict__ inc, long long n_blk, int width, int r, int k,
+                                       bool forward, const __grid_constant__ BinomTable B) {
+    const long long blk = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (blk >= n_blk) return;
+    int negatives = 0;
+    for_each_neighbour(static_cast<uint32_t>(blk), r, k, forward, B,
+                       [&](int, uint32_t, bool negative) { negatives += negative; });
+    uint32_t *pos = inc + blk * width, *neg = pos + width - negatives;
+    for_each_neighbour(static_cast<uint32_t>(blk), r, k, forward, B, [&](int i, uint32_t rank, bool negative) {
+        *(negative ? neg++ : pos++) = rank | (static_cast<uint32_t>(i) << 26) | (negative ? 0x80000000u : 0u);
+    });
 }
 
 // A session's start: the buffer, no entries, clear projection scratch.
@@ -309,12 +338,11 @@ void KoszulCtx::launch_to_canonical(const int32_t* in, uint32_t* out, uint64_t c
 namespace {
 
 template <int NB, int TO>
-void launch_gather(KoszulCtx& c, const int32_t* in, int32_t* out, const uint32_t* inc, const int32_t* coef,
-                   const int32_t* diag, uint64_t n_blk, int width, int inner, int outer, int ostride,
-                   cudaStream_t st) {
-    const size_t smem = static_cast<size_t>(c.r) * inner * ostride * sizeof(int32_t);
+void launch_gather(KoszulCtx& c, const int32_t* in, int32_t* out, const uint32_t* inc, const int4* coef,
+                   const int32_t* diag, uint64_t n_blk, int width, int inner, int outer, cudaStream_t st) {
     auto kern = gather_mac_kernel<NB, TO>;
-    const int tpb = (outer + TO - 1) / TO * (NB / 4);
+    const int tiles = (outer + TO - 1) / TO, tpb = tiles * (NB / 4);
+    const size_t smem = static_cast<size_t>(c.r) * inner * tiles * ((TO + 3) / 4) * sizeof(int4);
     BW_REQUIRE(tpb <= 256, "dimension too large for the plain gather kernel (dim/4 * n/4 > 256)");
     const int bpc = 256 / tpb;
     BW_REQUIRE(static_cast<int>(smem) <= allow_dynamic_smem(kern, c.device),
@@ -324,16 +352,34 @@ void launch_gather(KoszulCtx& c, const int32_t* in, int32_t* out, const uint32_t
     BW_REQUIRE(occ > 0, "plain gather kernel does not fit on an SM");
     const uint64_t groups = (n_blk + bpc - 1) / bpc;
     const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(groups, static_cast<uint64_t>(c.sms) * occ));
-    kern<<<grid, 256, smem, st>>>(in, out, inc, coef, diag, static_cast<long long>(n_blk), width, c.r,
-                                  inner, outer, ostride, c.mod);
+    kern<<<grid, 256, smem, st>>>(in, out, inc, coef, diag, static_cast<long long>(n_blk), width, c.r, inner, outer,
+                                  c.mod, c.fold);
     BW_CHECK_LAUNCH();
     ++c.launches;
 }
 
 template <int NB>
+void launch_rows(int rows, KoszulCtx& c, const int32_t* in, int32_t* out, const uint32_t* inc, const int4* coef,
+                 const int32_t* diag, uint64_t n_blk, int width, int inner, int outer, cudaStream_t st) {
+    switch (rows) {
+        case 4: return launch_gather<NB, 4>(c, in, out, inc, coef, diag, n_blk, width, inner, outer, st);
+        case 5: return launch_gather<NB, 5>(c, in, out, inc, coef, diag, n_blk, width, inner, outer, st);
+        case 6: return launch_gather<NB, 6>(c, in, out, inc, coef, diag, n_blk, width, inner, outer, st);
+        case 7: return launch_gather<NB, 7>(c, in, out, inc, coef, diag, n_blk, width, inner, outer, st);
+        default: return launch_gather<NB, 8>(c, in, out, inc, coef, diag, n_blk, width, inner, outer, st);
+    }
+}
+
+// Rows a tile when a block's rows are dealt evenly to as many tiles of at most eight as they need.
+int even_rows(int outer) {
+    const int tiles = (outer + 7) / 8;
+    return std::max(4, (outer + tiles - 1) / tiles);
+}
+
+template <int NB>
 void launch_project(KoszulCtx& c, const int32_t* W, cudaStream_t st) {
-    project_kernel<NB><<<c.proj_grid, 256, 0, st>>>(c.d_xb, W, static_cast<long long>(c.n_src), c.m,
-                                                    c.d_partials, c.d_counter, c.d_seq_state, c.mod);
+    project_kernel<NB><<<c.proj_grid, 256, c.m * NB * sizeof(int32_t), st>>>(
+        c.d_xb, W, static_cast<long long>(c.n_src), c.m, c.d_partials, c.d_counter, c.d_seq_state, c.mod, c.fold);
     BW_CHECK_LAUNCH();
     ++c.launches;
 }
@@ -353,22 +399,14 @@ void dispatch_nb(int nb, F&& f) {
 
 void KoszulCtx::plain_forward(const int32_t* y, int32_t* z, cudaStream_t st) {
     dispatch_nb(nb, [&](auto NBc) {
-        constexpr int NB = decltype(NBc)::value;
-        if (tile_fwd == 8)
-            launch_gather<NB, 8>(*this, y, z, d_fwd, d_coef_fwd, nullptr, n_t, r - k + 1, ci, co, co8, st);
-        else
-            launch_gather<NB, 4>(*this, y, z, d_fwd, d_coef_fwd, nullptr, n_t, r - k + 1, ci, co, co8, st);
+        launch_rows<decltype(NBc)::value>(tile_fwd, *this, y, z, d_fwd, d_coef_fwd, nullptr, n_t, r - k + 1, ci, co, st);
     });
 }
 
 void KoszulCtx::plain_transpose(const int32_t* z, int32_t* w, bool scale, cudaStream_t st) {
     dispatch_nb(nb, [&](auto NBc) {
-        constexpr int NB = decltype(NBc)::value;
-        const int32_t* dg = scale ? d_diag : nullptr;
-        if (tile_bwd == 8)
-            launch_gather<NB, 8>(*this, z, w, d_bwd, d_coef_bwd, dg, n_s, k, co, ci, ci8, st);
-        else
-            launch_gather<NB, 4>(*this, z, w, d_bwd, d_coef_bwd, dg, n_s, k, co, ci, ci8, st);
+        launch_rows<decltype(NBc)::value>(tile_bwd, *this, z, w, d_bwd, d_coef_bwd, scale ? d_diag : nullptr, n_s, k, co,
+                                          ci, st);
     });
 }
 
@@ -412,45 +450,23 @@ T* KoszulCtx::alloc(uint64_t count) {
     return static_cast<T*>(p);
 }
 
-static void build_tables(int r, int k, std::vector<uint32_t>& fwd, std::vector<uint32_t>& bwd) {
-    const uint64_t n_t = binom(r, k - 1), n_s = binom(r, k);
-    const int fw = r - k + 1;
-    fwd.assign(n_t * fw, 0);
-    bwd.assign(n_s * k, 0);
-    int T[64], S[64];
-    for (uint64_t t = 0; t < n_t; ++t) {
-        lex_unrank(t, r, k - 1, T);
-        uint32_t pos_list[64], neg_list[64];
-        int np = 0, nn = 0, pos = 0;
-        for (int i = 0; i < r; ++i) {
-            if (pos < k - 1 && T[pos] == i) {
-                ++pos;
-                continue;
-            }
-            for (int q = 0, w = 0; q < k; ++q) S[q] = (q == pos) ? i : T[w++];
-            const uint32_t e = static_cast<uint32_t>(lex_rank(S, r, k)) | (static_cast<uint32_t>(i) << 26);
-            if (pos & 1) neg_list[nn++] = e | 0x80000000u;
-            else pos_list[np++] = e;
-        }
-        uint32_t* row = fwd.data() + t * fw;
-        std::memcpy(row, pos_list, sizeof(uint32_t) * np);
-        std::memcpy(row + np, neg_list, sizeof(uint32_t) * nn);
+// The shift of the accumulators' fold: the least bound 2^s + (2^(31-s) + 1)
+// |2^s mod p| on a folded value.  It fits in int32 beside eight products of
+// balanced residues for every odd prime below 2^15: up to 32,500 some s near 22
+// has room, and above that 2^15 mod p is below 268.
+Fold plan_fold(uint32_t p) {
+    const Mod m = make_mod(p);
+    Fold best{};
+    int64_t least = INT64_MAX;
+    for (int s = 1; s < 30; ++s) {
+        const int32_t c = to_balanced((1u << s) % p, m);
+        const int64_t bound = (int64_t{1} << s) + ((int64_t{1} << (31 - s)) + 1) * (c < 0 ? -c : c);
+        if (bound >= least) continue;
+        least = bound;
+        best = Fold{c, s, static_cast<int32_t>((1u << s) - 1)};
     }
-    for (uint64_t s = 0; s < n_s; ++s) {
-        lex_unrank(s, r, k, S);
-        uint32_t* row = bwd.data() + s * k;
-        int np = 0;
-        uint32_t neg_list[64];
-        int nn = 0;
-        for (int pos = 0; pos < k; ++pos) {
-            for (int q = 0, w = 0; q < k; ++q)
-                if (q != pos) T[w++] = S[q];
-            const uint32_t e = static_cast<uint32_t>(lex_rank(T, r, k - 1)) | (static_cast<uint32_t>(S[pos]) << 26);
-            if (pos & 1) neg_list[nn++] = e | 0x80000000u;
-            else row[np++] = e;
-        }
-        std::memcpy(row + np, neg_list, sizeof(uint32_t) * nn);
-    }
+    BW_REQUIRE(least + int64_t{8} * m.half * m.half < (int64_t{1} << 31), "internal: no fold of the sums fits int32");
+    return best;
 }
 
 KoszulCtx* KoszulCtx::create(const bw_koszul_desc& d, int dev) {
@@ -476,13 +492,12 @@ KoszulCtx* KoszulCtx::create(const bw_koszul_desc& d, int dev) {
     c->k = static_cast<int>(d.k);
     c->ci = static_cast<int>(d.dim_in);
     c->co = static_cast<int>(d.dim_out);
-    c->ci8 = (c->ci + 7) / 8 * 8;
-    c->co8 = (c->co + 7) / 8 * 8;
     c->nb = static_cast<int>(d.block_width);
     c->nbi = d.form == BW_FORM_INT8 ? (c->nb <= 16 ? 16 : 32) : c->nb;
     c->m = static_cast<int>(d.proj_width);
     c->p = d.prime;
     c->mod = make_mod(d.prime);
+    c->fold = plan_fold(d.prime);
     c->form = d.form;
     c->n_s = binom(c->r, c->k);
     c->n_t = binom(c->r, c->k - 1);
@@ -491,36 +506,23 @@ KoszulCtx* KoszulCtx::create(const bw_koszul_desc& d, int dev) {
     BW_CUDA(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));
     BW_CUDA(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
 
-    const size_t smem_fwd = static_cast<size_t>(c->r) * c->ci * c->co8 * sizeof(int32_t);
-    const size_t smem_bwd = static_cast<size_t>(c->r) * c->co * c->ci8 * sizeof(int32_t);
+    const size_t smem_fwd = static_cast<size_t>(c->r) * c->ci * ((c->co + 7) / 8 * 8) * sizeof(int32_t);
+    const size_t smem_bwd = static_cast<size_t>(c->r) * c->co * ((c->ci + 7) / 8 * 8) * sizeof(int32_t);
     BW_REQUIRE(smem_fwd <= 200 * 1024 && smem_bwd <= 200 * 1024,
                "maps too large for shared memory staging (r * dim_in * dim_out * 4 > 200 KiB)");
 
-    // Coefficient tiles (balanced): forward uses M^T [i][b][c8], transpose M [i][c][b8] (rows zero-padded to 8).
-    std::vector<int32_t> coef_fwd(static_cast<size_t>(c->r) * c->ci * c->co8, 0);
-    std::vector<int32_t> coef_bwd(static_cast<size_t>(c->r) * c->co * c->ci8, 0);
     c->maps_canonical.assign(d.maps, d.maps + static_cast<size_t>(c->r) * c->co * c->ci);
-    for (int i = 0; i < c->r; ++i)
-        for (int cc = 0; cc < c->co; ++cc)
-            for (int b = 0; b < c->ci; ++b) {
-                const uint32_t v = d.maps[(static_cast<size_t>(i) * c->co + cc) * c->ci + b] % c->p;
-                const int32_t bal = to_balanced(v, c->mod);
-                coef_fwd[(static_cast<size_t>(i) * c->ci + b) * c->co8 + cc] = bal;
-                coef_bwd[(static_cast<size_t>(i) * c->co + cc) * c->ci8 + b] = bal;
-            }
     cudaStream_t st = c->own_stream;
-    // plain form only (the INT8 form builds its own tables on the device)
-    std::vector<uint32_t> fwd, bwd;
-    if (c->form == BW_FORM_PLAIN) {
-        build_tables(c->r, c->k, fwd, bwd);
-        c->d_coef_fwd = c->alloc<int32_t>(coef_fwd.size());
-        c->d_coef_bwd = c->alloc<int32_t>(coef_bwd.size());
-        c->d_fwd = c->alloc<uint32_t>(fwd.size());
-        c->d_bwd = c->alloc<uint32_t>(bwd.size());
-        BW_CUDA(cudaMemcpyAsync(c->d_coef_fwd, coef_fwd.data(), coef_fwd.size() * 4, cudaMemcpyHostToDevice, st));
-        BW_CUDA(cudaMemcpyAsync(c->d_coef_bwd, coef_bwd.data(), coef_bwd.size() * 4, cudaMemcpyHostToDevice, st));
-        BW_CUDA(cudaMemcpyAsync(c->d_fwd, fwd.data(), fwd.size() * 4, cudaMemcpyHostToDevice, st));
-        BW_CUDA(cudaMemcpyAsync(c->d_bwd, bwd.data(), bwd.size() * 4, cudaMemcpyHostToDevice, st));
+    if (c->form == BW_FORM_PLAIN) {   // the INT8 form has tables of its own
+        const int fw = c->r - c->k + 1;
+        const BinomTable binoms = binom_table();
+        c->d_fwd = c->alloc<uint32_t>(c->n_t * fw);
+        c->d_bwd = c->alloc<uint32_t>(c->n_s * c->k);
+        plain_incidence_kernel<<<blocks_of(c->n_t, 128), 128, 0, st>>>(c->d_fwd, static_cast<long long>(c->n_t), fw,
+                                                                        c->r, c->k, true, binoms);
+        plain_incidence_kernel<<<blocks_of(c->n_s, 128), 128, 0, st>>>(c->d_bwd, static_cast<long long>(c->n_s), c->k,
+                                                                        c->r, c->k, false, binoms);
+        BW_CHECK_LAUNCH();
     }
 
     c->d_diag = c->alloc<int32_t>(c->n_src);
@@ -542,7 +544,7 @@ KoszulCtx* KoszulCtx::create(const bw_koszul_desc& d, int dev) {
         c->d_z = c->alloc<int32_t>(c->n_tgt * c->nb);
         c->d_xb = c->alloc<int32_t>(c->n_src * c->m);
     }
-    c->proj_grid = static_cast<unsigned>(std::min<uint64_t>(static_cast<uint64_t>(c->sms) * 4,
+    c->proj_grid = static_cast<unsigned>(std::min<uint64_t>(static_cast<uint64_t>(c->sms) * 2,
                                                             std::max<uint64_t>(1, (c->n_src + 255) / 256)));
     const uint64_t scratch_before = c->device_bytes;
     // per-CTA partial sums: the plain projection's grid, or up to one CTA per SM for the INT8 form
@@ -561,29 +563,55 @@ namespace {
 // context of the process.
 std::mutex g_plain_mutex;
 std::map<std::tuple<int, int, int, int, int, int>, std::pair<int, int>> g_plain_tiles;
+
 }  // namespace
 
-// The plain gathers hold a 4- or 8-row output tile per thread (8 rows: twice
-// the multiply-adds per gathered row, more registers, and the rows padded to
-// a multiple of 8).  Each direction's height is timed at set-up on the
-// context's own buffers (one warm-up and two launches; the kernels' work does
-// not depend on the values) and the faster kept; BW_PLAIN_TILE=4 or =8 forces
-// one height.
+// The coefficients of one direction's gathers for tiles of `rows` output rows
+// (balanced, [i][u][tile][rows rounded up to 4]; d uses M_i^T, d^T M_i),
+// replacing the direction's earlier ones.
+void KoszulCtx::plain_coefficients(bool transpose_dir, int rows) {
+    const int inner = transpose_dir ? co : ci, outer = transpose_dir ? ci : co;
+    const int tiles = (outer + rows - 1) / rows, pad = (rows + 3) / 4 * 4;
+    std::vector<int4> host(static_cast<size_t>(r) * inner * tiles * pad / 4, make_int4(0, 0, 0, 0));
+    int32_t* cell = reinterpret_cast<int32_t*>(host.data());
+    for (int i = 0; i < r; ++i)
+        for (int u = 0; u < inner; ++u)
+            for (int o = 0; o < outer; ++o) {
+                const size_t at = transpose_dir ? (static_cast<size_t>(i) * co + u) * ci + o
+                                                : (static_cast<size_t>(i) * co + o) * ci + u;
+                cell[((static_cast<size_t>(i) * inner + u) * tiles + o / rows) * pad + o % rows] =
+                    to_balanced(maps_canonical[at] % p, mod);
+            }
+    int4*& d = transpose_dir ? d_coef_bwd : d_coef_fwd;
+    if (d) release(d);
+    d = alloc<int4>(host.size());
+    BW_CUDA(cudaMemcpyAsync(d, host.data(), host.size() * sizeof(int4), cudaMemcpyHostToDevice, own_stream));
+    BW_CUDA(cudaStreamSynchronize(own_stream));
+    (transpose_dir ? tile_bwd : tile_fwd) = rows;
+}
+
+// Output rows a thread of each direction's gathers: 4, 8 or the even height
+// (5 to 7, see even_rows), timed at set-up on the context's own buffers (one
+// warm-up and two launches; the kernels' work does not depend on the values),
+// the fastest kept; BW_PLAIN_TILE=4 to =8 forces one height.
 void KoszulCtx::plain_setup() {
     int forced = 0;
     if (const char* e = std::getenv("BW_PLAIN_TILE")) forced = std::atoi(e);
-    if (forced == 4 || forced == 8) {
-        tile_fwd = tile_bwd = forced;
+    if (forced >= 4 && forced <= 8) {
+        plain_coefficients(false, forced);
+        plain_coefficients(true, forced);
         plain_plan = "plain: " + std::to_string(forced) + " output rows a thread (forced)";
         return;
     }
     const auto key = std::make_tuple(r, k, ci, co, nb, sms);
     {
-        std::lock_guard<std::mutex> lock(g_plain_mutex);
+        std::unique_lock<std::mutex> lock(g_plain_mutex);
         const auto it = g_plain_tiles.find(key);
         if (it != g_plain_tiles.end()) {
-            tile_fwd = it->second.first;
-            tile_bwd = it->second.second;
+            const auto tiles = it->second;
+            lock.unlock();
+            plain_coefficients(false, tiles.first);
+            plain_coefficients(true, tiles.second);
             plain_plan = "plain: d " + std::to_string(tile_fwd) + ", d^T " + std::to_string(tile_bwd) +
                          " output rows a thread (tuned earlier in this process)";
             return;
@@ -595,36 +623,46 @@ void KoszulCtx::plain_setup() {
     cudaEvent_t e0, e1;
     BW_CUDA(cudaEventCreate(&e0));
     BW_CUDA(cudaEventCreate(&e1));
-    auto time_it = [&](bool fwd, int tile) {
-        (fwd ? tile_fwd : tile_bwd) = tile;
-        auto run = [&] {
-            if (fwd)
-                plain_forward(d_ya, d_z, st);
-            else
-                plain_transpose(d_z, d_yb, true, st);
-        };
-        run();
-        BW_CUDA(cudaEventRecord(e0, st));
-        run();
-        run();
-        BW_CUDA(cudaEventRecord(e1, st));
-        BW_CUDA(cudaEventSynchronize(e1));
-        float ms = 0;
-        BW_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        return ms / 2;
+    std::string tried;
+    auto choose = [&](bool fwd) {
+        const int outer = fwd ? co : ci;
+        std::vector<int> heights{4, 8};
+        if (even_rows(outer) > 4 && even_rows(outer) < 8) heights.push_back(even_rows(outer));
+        int best = 0;
+        float least = 0;
+        for (int rows : heights) {
+            plain_coefficients(!fwd, rows);
+            auto run = [&] {
+                if (fwd)
+                    plain_forward(d_ya, d_z, st);
+                else
+                    plain_transpose(d_z, d_yb, true, st);
+            };
+            run();
+            BW_CUDA(cudaEventRecord(e0, st));
+            run();
+            run();
+            BW_CUDA(cudaEventRecord(e1, st));
+            BW_CUDA(cudaEventSynchronize(e1));
+            float ms = 0;
+            BW_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+            ms /= 2;
+            char buf[64];
+            std::snprintf(buf, sizeof buf, "%s%s %d rows %.4f ms", tried.empty() ? "" : ", ", fwd ? "d" : "d^T", rows, ms);
+            tried += buf;
+            if (best == 0 || ms < least) {
+                best = rows;
+                least = ms;
+            }
+        }
+        if ((fwd ? tile_fwd : tile_bwd) != best) plain_coefficients(!fwd, best);
     };
-    char buf[256];
-    const float f4 = time_it(true, 4), f8 = time_it(true, 8);
-    const float b4 = time_it(false, 4), b8 = time_it(false, 8);
+    choose(true);
+    choose(false);
     BW_CUDA(cudaEventDestroy(e0));
     BW_CUDA(cudaEventDestroy(e1));
-    tile_fwd = f8 < f4 ? 8 : 4;
-    tile_bwd = b8 < b4 ? 8 : 4;
-    std::snprintf(buf, sizeof buf,
-                  "plain: d %d, d^T %d output rows a thread (tuned: d 4 rows %.4f ms, 8 rows %.4f ms; d^T 4 rows %.4f "
-                  "ms, 8 rows %.4f ms)",
-                  tile_fwd, tile_bwd, f4, f8, b4, b8);
-    plain_plan = buf;
+    plain_plan = "plain: d " + std::to_string(tile_fwd) + ", d^T " + std::to_string(tile_bwd) +
+                 " output rows a thread (tuned: " + tried + ")";
     std::lock_guard<std::mutex> lock(g_plain_mutex);
     g_plain_tiles[key] = {tile_fwd, tile_bwd};
 }

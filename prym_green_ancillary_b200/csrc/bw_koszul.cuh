@@ -18,15 +18,21 @@ struct SeqState {
     uint32_t* seq;
 };
 
+// x = (x & mask) + (x >> shift) * c (mod p), c = 2^shift mod p.
+struct Fold {
+    int32_t c, shift, mask;
+};
+
 struct KoszulCtx {
     // shape
     int device = 0, sms = 0;
-    int r = 0, k = 0, ci = 0, co = 0, ci8 = 0, co8 = 0, nb = 0, m = 0;
-    // plain form: output rows per thread of the d and d^T gathers (4 or 8)
+    int r = 0, k = 0, ci = 0, co = 0, nb = 0, m = 0;
+    // plain form: output rows per thread of the d and d^T gathers (4 to 8)
     int tile_fwd = 4, tile_bwd = 4;
     int nbi = 0;   // block width inside the INT8 form (nb, or 16 for nb = 4 / 8: zero columns appended)
     uint32_t p = 0, form = BW_FORM_PLAIN;
     Mod mod{};
+    Fold fold{};   // plain gathers
     uint64_t n_s = 0, n_t = 0, n_src = 0, n_tgt = 0;
 
     // device state
@@ -34,7 +40,7 @@ struct KoszulCtx {
     cudaEvent_t ev_join = nullptr;     // orders NULL-stream calls with the legacy stream
     std::vector<std::pair<void*, uint64_t>> allocations;   // pointer, bytes
     uint64_t device_bytes = 0, scratch_bytes = 0;
-    int32_t *d_coef_fwd = nullptr, *d_coef_bwd = nullptr;
+    int4 *d_coef_fwd = nullptr, *d_coef_bwd = nullptr;   // plain gathers (plain_coefficients)
     uint32_t *d_fwd = nullptr, *d_bwd = nullptr;
     int32_t* d_diag = nullptr;
     int32_t *d_ya = nullptr, *d_yb = nullptr, *d_z = nullptr, *d_xb = nullptr;
@@ -85,6 +91,7 @@ struct KoszulCtx {
     void ensure_host_staging(uint64_t nlen);
 
     // INT8-limb form
+    void plain_coefficients(bool transpose_dir, int rows);
     void plain_setup();            // chooses the plain gathers' tile heights (tile_fwd, tile_bwd)
     std::string plain_plan;        // the choice and its timings
     void i8_setup();

@@ -50,6 +50,7 @@
 // copies and MMAs are drained and TMEM is freed.
 #include "bw_koszul.cuh"
 #include "bw_koszul_i8_dev.cuh"
+#include "bw_koszul_tables.cuh"
 #include "bw_koszul_i8_union.cuh"
 #include "tc_sm100.cuh"
 
@@ -1311,59 +1312,17 @@ bool plan_direction(KoszulCtx& c, KoszulCtx::I8State::Dir& D, int inner, int out
     return true;
 }
 
-// Binomial coefficients for the table kernels: C(n, k), n, k <= 31 (below 2^32).
-struct BinomTable {
-    uint32_t c[32][32];
-};
-
-BinomTable binom_table() {
-    BinomTable t;
-    for (int n = 0; n < 32; ++n)
-        for (int k = 0; k < 32; ++k) t.c[n][k] = static_cast<uint32_t>(k <= n ? binom(n, k) : 0);
-    return t;
-}
-
-// Dense incidence table [blk][r]: neighbour rank | negative << 31, or kAbsent.
-//   forward : blk = T, a (k-1)-subset; neighbour S = T u {i} for every i not in T
-//   backward: blk = S, a k-subset; neighbour T = S \ {i} for every i in S
-// with rank(S) = C(r,k) - 1 - sum_pos C(r-1-S_pos, k-pos) (lexicographic) and
-// the sign (-1)^pos of i's position in S.  One thread unranks a subset and
-// walks the generators; `before` and `after` hold the neighbour's rank terms of
-// the elements below and above i.
+// Dense incidence table [blk][r]: neighbour rank | negative << 31, or kAbsent
+// (forward: blk = T; backward: blk = S; see for_each_neighbour).
 __global__ void incidence_kernel(uint32_t* __restrict__ inc, long long n_blk, int r, int k, bool forward,
                                  const __grid_constant__ BinomTable B) {
     const long long blk = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (blk >= n_blk) return;
-    const int size = forward ? k - 1 : k, other = forward ? k : k - 1;   // of blk, of its neighbours
-    uint32_t set = 0, rem = B.c[r][size] - 1 - static_cast<uint32_t>(blk);
-    for (int pos = 0, v = 0; pos < size; ++pos, ++v) {
-        while (B.c[r - 1 - v][size - pos] > rem) ++v;
-        rem -= B.c[r - 1 - v][size - pos];
-        set |= 1u << v;
-    }
-    // an element at position j counts C(r-1-v, other - j) below i; above i its
-    // position in the neighbour is j + 1 (forward) or j - 1 (backward)
-    const int shift = forward ? 1 : -1;
-    uint32_t before = 0, after = 0;
-    for (int v = 0, j = 0; v < r; ++v)
-        if (set >> v & 1) {
-            after += other - j - shift >= 0 ? B.c[r - 1 - v][other - j - shift] : 0u;
-            ++j;
-        }
     uint32_t* out = inc + blk * r;
-    for (int i = 0, pos = 0; i < r; ++i) {
-        const bool in = (set >> i & 1) != 0;
-        const uint32_t sign = (pos & 1) ? 0x80000000u : 0u;
-        uint32_t e = kAbsent;
-        if (in) after -= other - pos - shift >= 0 ? B.c[r - 1 - i][other - pos - shift] : 0u;
-        if (in != forward)
-            e = (B.c[r][other] - 1 - before - after - (forward ? B.c[r - 1 - i][k - pos] : 0u)) | sign;
-        if (in) {
-            before += other - pos >= 0 ? B.c[r - 1 - i][other - pos] : 0u;
-            ++pos;
-        }
-        out[i] = e;
-    }
+    for (int i = 0; i < r; ++i) out[i] = kAbsent;
+    for_each_neighbour(static_cast<uint32_t>(blk), r, k, forward, B, [&](int i, uint32_t rank, bool negative) {
+        out[i] = rank | (negative ? 0x80000000u : 0u);
+    });
 }
 
 // Rows of the TMA gathers: for output block blk and group g (generators
@@ -1398,8 +1357,6 @@ __global__ void union_mask_kernel(const uint32_t* __restrict__ inc, uint32_t* __
             if (inc[blk * r + i] != kAbsent) m |= 1u << i;
     mask[tile] = m;
 }
-
-unsigned blocks_of(uint64_t items, unsigned threads) { return static_cast<unsigned>((items + threads - 1) / threads); }
 
 // Plans one direction of the union kernel with gs generators a stage and pw
 // producer warps in groups; false when it does not fit (shared memory for the
