@@ -19,6 +19,8 @@
 
 #include <algorithm>
 #include <cstring>
+#include <system_error>
+#include <thread>
 #include <iostream>
 
 namespace bw {
@@ -284,55 +286,59 @@ __global__ void cyc_rowmix_kernel(const uint32_t* __restrict__ pairs, long long 
 
 __device__ __forceinline__ int tri_index(int row, int col) { return row * (2 * 4 - row + 1) / 2 + (col - row); }
 
-// Gram moments of one half-round: G1 = A1^t C1 and (count == 2) G2 = A2^t C2,
-// upper triangles packed into seq at positions *seq_index (+1), canonical.
-// partials: gridDim.x x 20 int32; counter left at 0.
-__global__ void __launch_bounds__(kThreads) cyc_gram_kernel(
-    const int32_t* __restrict__ A1, const int32_t* __restrict__ C1, const int32_t* __restrict__ A2,
-    const int32_t* __restrict__ C2, int count, long long rows, int32_t* __restrict__ partials,
-    unsigned int* __restrict__ counter, uint32_t* __restrict__ seq, unsigned long long* __restrict__ seq_index,
-    Mod mod) {
+// Gram moments of one half-round: B^t D and (count == 2) O^t O, where O is the
+// newer of the two, upper triangles packed into seq at positions *seq_index
+// (+1), canonical.
+// partials: 20 accumulators, left at 0; counter left at 0.
+// Bound by the row loads where a thread has enough rows to spread the reduction
+// of its 20 sums over: four CTAs an SM and one warp instruction a sum (eight
+// CTAs an SM and five shuffles a sum spent half of their instructions there:
+// an application at genus 24 57.2 -> 53.9 us, at genus 26 165.4 -> 161.5).
+__global__ void __launch_bounds__(kThreads, 4) cyc_gram_kernel(
+    const int32_t* __restrict__ B, const int32_t* __restrict__ D, int b_is_newer, int count, long long rows,
+    int32_t* __restrict__ partials, unsigned int* __restrict__ counter, uint32_t* __restrict__ seq,
+    unsigned long long* __restrict__ seq_index, Mod mod) {
     cyc::pdl_trigger();
     cyc::pdl_wait();
     int32_t acc[20];
 #pragma unroll
     for (int e = 0; e < 20; ++e) acc[e] = 0;
-    int cnt = 0;
-    for (long long row = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; row < rows;
-         row += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int4 a1 = ld4(A1, row), c1 = ld4(C1, row);
-        const int av[4] = {a1.x, a1.y, a1.z, a1.w}, cv[4] = {c1.x, c1.y, c1.z, c1.w};
+    auto add = [&](const int4& b, const int4& d) {
+        const int4 o = b_is_newer ? b : d;
+        const int bv[4] = {b.x, b.y, b.z, b.w}, dv[4] = {d.x, d.y, d.z, d.w}, ov[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
         for (int r0 = 0; r0 < 4; ++r0)
 #pragma unroll
-            for (int c0 = r0; c0 < 4; ++c0) acc[tri_index(r0, c0)] += av[r0] * cv[c0];
-        if (count == 2) {
-            const int4 a2 = ld4(A2, row), c2 = ld4(C2, row);
-            const int bv[4] = {a2.x, a2.y, a2.z, a2.w}, dv[4] = {c2.x, c2.y, c2.z, c2.w};
+            for (int c0 = r0; c0 < 4; ++c0) {
+                acc[tri_index(r0, c0)] += bv[r0] * dv[c0];
+                acc[10 + tri_index(r0, c0)] += ov[r0] * ov[c0];
+            }
+    };
+    // four rows in flight, eight products beside a partially reduced sum
+    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+    long long row = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    for (; row + 3 * stride < rows; row += 4 * stride) {
+        int4 b[4], d[4];
 #pragma unroll
-            for (int r0 = 0; r0 < 4; ++r0)
-#pragma unroll
-                for (int c0 = r0; c0 < 4; ++c0) acc[10 + tri_index(r0, c0)] += bv[r0] * dv[c0];
+        for (int q = 0; q < 4; ++q) {
+            b[q] = ld4(B, row + q * stride);
+            d[q] = ld4(D, row + q * stride);
         }
-        if (++cnt == 8) {
-            cnt = 0;
 #pragma unroll
-            for (int e = 0; e < 20; ++e) acc[e] = reduce_partial(acc[e], mod);
-        }
+        for (int q = 0; q < 4; ++q) add(b[q], d[q]);
+#pragma unroll
+        for (int e = 0; e < 20; ++e) acc[e] = reduce_partial(acc[e], mod);
     }
+    for (; row < rows; row += stride) add(ld4(B, row), ld4(D, row));
     __shared__ int32_t red[kThreads / 32][20];
     __shared__ bool am_last;
-    // warp reduction (values below 2p; 32 of them stay far inside int32)
+    // warp sums of balanced values
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 #pragma unroll
     for (int e = 0; e < 20; ++e) {
-        int32_t v = reduce_balanced(acc[e], mod);
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        acc[e] = v;
+        const int32_t v = __reduce_add_sync(0xffffffffu, reduce_balanced(acc[e], mod));
+        if (lane == 0) red[warp][e] = reduce_balanced(v, mod);
     }
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    if (lane == 0)
-#pragma unroll
-        for (int e = 0; e < 20; ++e) red[warp][e] = reduce_balanced(acc[e], mod);
     __syncthreads();
     int32_t mine = 0, total = 0;
     if (threadIdx.x < 20) {
@@ -435,6 +441,11 @@ CyclicCtx::~CyclicCtx() {
     for (auto& g : graphs)
         if (g) cudaGraphExecDestroy(g);
     for (void* p : allocations) cudaFree(p);
+    if (h_err) cudaFreeHost(const_cast<int*>(h_err));
+    for (auto& lane : out_lanes) {
+        cudaFreeHost(lane.pinned);
+        cudaStreamDestroy(lane.stream);
+    }
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -552,6 +563,7 @@ CyclicCtx* CyclicCtx::open(const std::string& instance_path, const std::string& 
         c->initial_block = cyclic::random_vector(ncols * num_v, c->p, gen, false);
     }
     c->plan = cyclic::generate_rowmix_plan(es.target_rows, op, sector, c->p, rowmix_rounds, rowmix_seed);
+    c->plan_hash = cyclic::rowmix_plan_hash(c->plan);
     if (rowmix_rounds > 0) {
         c->precond = cyclic::composite_target_preconditioner(c->plan, c->row_precond, c->p);
     } else {
@@ -687,7 +699,7 @@ CyclicCtx* CyclicCtx::open(const std::string& instance_path, const std::string& 
     c->d_u = c->alloc<int32_t>(std::max<size_t>(es.target_rows, 1) * v);
     c->d_u2 = c->alloc<int32_t>(std::max<size_t>(es.target_rows, 1) * v);
     c->gram_grid = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>((nc + kThreads - 1) / kThreads,
-                                                                                static_cast<size_t>(c->sms) * 8)));
+                                                                                static_cast<size_t>(c->sms) * 4)));
     c->d_partials = c->alloc<int32_t>(20);   // grid-sum accumulators (zero between launches)
     BW_CUDA(cudaMemsetAsync(c->d_partials, 0, 20 * sizeof(int32_t), c->stream));
     c->d_counter = c->alloc<unsigned int>(1);
@@ -704,7 +716,9 @@ CyclicCtx* CyclicCtx::open(const std::string& instance_path, const std::string& 
     BW_CUDA(cudaMemsetAsync(c->d_seq_index, 0, sizeof(unsigned long long), c->stream));
     // the initial block (canonical -> balanced)
     uint32_t* tmp = c->upload(c->initial_block);
-    c->to_balanced(tmp, c->d_b, nc * v);
+    c->d_initial = c->alloc<int32_t>(nc * v);
+    c->to_balanced(tmp, c->d_initial, nc * v);
+    BW_CUDA(cudaMemcpyAsync(c->d_b, c->d_initial, nc * v * 4, cudaMemcpyDeviceToDevice, c->stream));
     BW_CUDA(cudaStreamSynchronize(c->stream));
     return c.release();
 }
@@ -801,9 +815,10 @@ void CyclicCtx::apply_square(const int32_t* in, int32_t* out) {
     backward(d_u2, out, true);
 }
 
-void CyclicCtx::gram(const int32_t* a1, const int32_t* c1, const int32_t* a2, const int32_t* c2, int count) {
-    launch_pdl(cyc_gram_kernel, gram_grid, 0, a1, c1, a2 ? a2 : a1, c2 ? c2 : c1, count,
-               static_cast<long long>(op_cols), d_partials, d_counter, d_seq, d_seq_index, mod);
+// count 2: B^t D and O^t O of the newer block O; count 1: b^t d.
+void CyclicCtx::gram(const int32_t* b, const int32_t* d, bool b_is_newer, int count) {
+    launch_pdl(cyc_gram_kernel, gram_grid, 0, b, d, b_is_newer ? 1 : 0, count, static_cast<long long>(op_cols), d_partials,
+               d_counter, d_seq, d_seq_index, mod);
     BW_CHECK_LAUNCH();
     ++launches;
 }
@@ -812,9 +827,9 @@ void CyclicCtx::gram(const int32_t* a1, const int32_t* c1, const int32_t* a2, co
 // D = S B; push B^t D, D^t D; B = S D; push B^t D, B^t B.
 void CyclicCtx::round() {
     apply_square(d_b, d_d);
-    gram(d_b, d_d, d_d, d_d, 2);
+    gram(d_b, d_d, false, 2);
     apply_square(d_d, d_b);
-    gram(d_b, d_d, d_b, d_b, 2);
+    gram(d_b, d_d, true, 2);
 }
 
 void CyclicCtx::generate(size_t nlen_target, float* device_ms) {
@@ -834,16 +849,15 @@ void CyclicCtx::generate(size_t nlen_target, float* device_ms) {
     }
     BW_CUDA(cudaMemsetAsync(d_seq_index, 0, sizeof(unsigned long long), stream));
     BW_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(unsigned int), stream));
-    // restart from the initial block
-    uint32_t* tmp = scratch_canonical();
-    BW_CUDA(cudaMemcpyAsync(tmp, initial_block.data(), nc * num_v * 4, cudaMemcpyHostToDevice, stream));
-    to_balanced(tmp, d_b, nc * num_v);
-    gram(d_b, d_b, nullptr, nullptr, 1);
+    // restart from the initial block (open() left it on the device)
+    if (d_b == xs_for) xs_for = nullptr;
+    BW_CUDA(cudaMemcpyAsync(d_b, d_initial, nc * num_v * 4, cudaMemcpyDeviceToDevice, stream));
+    gram(d_b, d_b, true, 1);
     // the first application's source, outside the round graph: every later
     // source is written by the backward kernels of the application before
     if (subset_path && rounds > 0) subset_source16(d_b, d_dc);
     if (rounds > 0) {
-        if (!graphs[0]) {
+        if (!persistent && !graphs[0]) {
             const uint64_t l0 = launches;
             cudaGraph_t graph;
             BW_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
@@ -865,9 +879,13 @@ void CyclicCtx::generate(size_t nlen_target, float* device_ms) {
             BW_CUDA(cudaEventCreate(&e1));
             BW_CUDA(cudaEventRecord(e0, stream));
         }
-        for (size_t r = 0; r < rounds; ++r) {
-            BW_CUDA(cudaGraphLaunch(graphs[0], stream));
-            launches += graph_kernels;
+        if (persistent) {
+            subset_rounds(rounds);
+        } else {
+            for (size_t r = 0; r < rounds; ++r) {
+                BW_CUDA(cudaGraphLaunch(graphs[0], stream));
+                launches += graph_kernels;
+            }
         }
         if (device_ms) {
             BW_CUDA(cudaEventRecord(e1, stream));
@@ -881,6 +899,12 @@ void CyclicCtx::generate(size_t nlen_target, float* device_ms) {
     }
     seq_len = 1 + 4 * rounds;
     BW_CUDA(cudaStreamSynchronize(stream));
+    if (persistent && *h_err != 0) {
+        *h_err = 0;
+        seq_len = 0;
+        BW_CUDA(cudaMemset(d_partials, 0, 20 * sizeof(int32_t)));
+        throw Error("the sequence's kernel gave up waiting (grid barrier between its phases)", 2);
+    }
 }
 
 uint32_t* CyclicCtx::scratch_canonical() {
@@ -888,15 +912,67 @@ uint32_t* CyclicCtx::scratch_canonical() {
     return d_canon;
 }
 
-void CyclicCtx::download_state(std::vector<uint32_t>& current, std::vector<uint32_t>& packed) {
-    const size_t nc = op_cols;
-    uint32_t* tmp = scratch_canonical();
-    to_canonical(d_b, tmp, nc * num_v);
-    current.resize(nc * num_v);
-    packed.resize(seq_len * 10);
-    BW_CUDA(cudaMemcpyAsync(current.data(), tmp, current.size() * 4, cudaMemcpyDeviceToHost, stream));
-    BW_CUDA(cudaMemcpyAsync(packed.data(), d_seq, packed.size() * 4, cudaMemcpyDeviceToHost, stream));
+// Device to pageable host memory.  A large block goes through a few pinned
+// chunks, each with a host thread and a stream of its own: the time is in
+// writing (and first touching) the destination's pages, which the threads
+// share (18 MB: 12 ms by one copy call).
+void CyclicCtx::copy_out(void* dst, const void* src, size_t bytes) {
+    constexpr size_t kChunk = size_t{1} << 20;
+    const size_t chunks = (bytes + kChunk - 1) / kChunk;
+    const size_t workers = std::min<size_t>({4, std::max(1u, std::thread::hardware_concurrency()), chunks / 2});
+    if (workers < 2) {
+        BW_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream));
+        BW_CUDA(cudaStreamSynchronize(stream));
+        return;
+    }
+    BW_CUDA(cudaStreamSynchronize(stream));   // src is complete
+    while (out_lanes.size() < workers) {
+        OutLane lane;
+        BW_CUDA(cudaHostAlloc(&lane.pinned, kChunk, cudaHostAllocDefault));
+        const cudaError_t made = cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking);
+        if (made != cudaSuccess) cudaFreeHost(lane.pinned);
+        BW_CUDA(made);
+        out_lanes.push_back(lane);
+    }
+    std::vector<cudaError_t> result(workers, cudaSuccess);
+    auto run = [&](size_t w) {
+        const OutLane& lane = out_lanes[w];
+        cudaError_t e = cudaSetDevice(device);
+        for (size_t c = w; c < chunks && e == cudaSuccess; c += workers) {
+            const size_t at = c * kChunk, n = std::min(kChunk, bytes - at);
+            e = cudaMemcpyAsync(lane.pinned, static_cast<const char*>(src) + at, n, cudaMemcpyDeviceToHost, lane.stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(lane.stream);
+            if (e == cudaSuccess) std::memcpy(static_cast<char*>(dst) + at, lane.pinned, n);
+        }
+        result[w] = e;
+    };
+    std::vector<std::thread> pool;
+    size_t started = 1;
+    try {
+        for (; started < workers; ++started) pool.emplace_back(run, started);
+    } catch (const std::system_error&) {   // no more threads: the caller does the rest
+    }
+    run(0);
+    for (size_t w = started; w < workers; ++w) run(w);
+    for (auto& t : pool) t.join();
+    for (cudaError_t e : result) BW_CUDA(e);
+}
+
+void CyclicCtx::download_into(uint32_t* current, uint32_t* packed) {
+    const size_t count = op_cols * num_v;
+    if (current) {
+        uint32_t* tmp = scratch_canonical();
+        to_canonical(d_b, tmp, count);
+        copy_out(current, tmp, count * 4);
+    }
+    if (packed) BW_CUDA(cudaMemcpyAsync(packed, d_seq, seq_len * 10 * 4, cudaMemcpyDeviceToHost, stream));
     BW_CUDA(cudaStreamSynchronize(stream));
+}
+
+void CyclicCtx::download_state(std::vector<uint32_t>& current, std::vector<uint32_t>& packed) {
+    current.resize(op_cols * num_v);
+    packed.resize(seq_len * 10);
+    download_into(current.data(), packed.data());
 }
 
 // Host-buffer operator applications (validation and tests).

@@ -62,7 +62,7 @@ struct SubsetDev {
     const uint32_t* u_pos;                 // compact u row -> its position in u (row-mixing locality order)
     const uint32_t* e_col;                 // folded target preconditioner, ELL (rows: padded u2 slots; columns: u positions)
     const int16_t* e_val;
-    uint32_t ell;                          // slots a row (a multiple of four)
+    uint32_t ell;                          // slots a row (six, or a multiple of four)
     const int32_t *blob_f, *blob_t;
     int blob_words;
     int o_R, o_B, o_a0off, o_a0idx, o_a1off, o_a1idx, o_koff, o_kidx, o_ych;
@@ -99,6 +99,7 @@ struct CyclicCtx {
     cyclic::EliminatedSector es;
     std::vector<uint32_t> row_precond, col_precond, initial_block;
     cyclic::RowMixPlan plan;
+    uint64_t plan_hash = 0;      // of the plan, which open() fixes (16 ms at genus 26)
     cyclic::Csr precond;
     // source columns: base_cols = x + z; op_cols = the operator's (the vectors' rows)
     size_t base_cols = 0, op_cols = 0, kept_cols = 0;
@@ -112,6 +113,7 @@ struct CyclicCtx {
     int32_t* d_dc = nullptr;
     uint32_t *d_p_ptr = nullptr, *d_p_col = nullptr;
     int32_t* d_p_val = nullptr;
+    int32_t* d_initial = nullptr;         // the initial block, balanced
     int32_t *d_b = nullptr, *d_d = nullptr, *d_xs = nullptr, *d_y = nullptr, *d_h = nullptr, *d_u = nullptr,
             *d_u2 = nullptr, *d_t = nullptr;
     bool small = false;          // int32 accumulation is exact for this sector
@@ -140,6 +142,15 @@ struct CyclicCtx {
     uint32_t* d_seq = nullptr;
     size_t seq_alloc = 0, seq_capacity = 0, seq_len = 0;
     cudaGraphExec_t graphs[1] = {nullptr};
+    // whole rounds in one cooperative launch (small sectors; bw_cyclic_subset.cu)
+    bool persistent = false;
+    unsigned rounds_grid = 0;
+    int rounds_threads = 0, rounds_hold = 0;
+    size_t rounds_smem = 0;
+    uint32_t rounds_wait_limit = 1u << 22;
+    uint32_t* d_barrier = nullptr;
+    int* d_err = nullptr;                 // mapped host memory (h_err)
+    volatile int* h_err = nullptr;
     // validation path (explicit rowmix rounds)
     uint32_t* d_pairs = nullptr;
     int32_t* d_dr = nullptr;
@@ -180,6 +191,8 @@ struct CyclicCtx {
     void forward(const int32_t* in, int32_t* u, bool precondition);
     // subset-major path (bw_cyclic_subset.cu): in -> d_u16, d_u16 -> d_u2_16, d_u2_16 -> out
     void setup_subset_path();
+    void setup_rounds();
+    void subset_rounds(size_t rounds);                              // d_b -> d_b, moments appended
     void subset_source16(const int32_t* in, const int32_t* dc);   // d_xs16 / d_zs = dc (.) in
     void subset_forward16();                                        // d_xs16 / d_zs -> d_u16
     void subset_precondition16();
@@ -191,9 +204,16 @@ struct CyclicCtx {
     void target_precondition(const int32_t* u, int32_t* u2);
     void backward(const int32_t* u2, int32_t* out, bool precondition);
     void apply_square(const int32_t* in, int32_t* out);
-    void gram(const int32_t* a1, const int32_t* c1, const int32_t* a2, const int32_t* c2, int count);
+    void gram(const int32_t* b, const int32_t* d, bool b_is_newer, int count);
     void round();
     void generate(size_t nlen_target, float* device_ms = nullptr);
+    struct OutLane {
+        void* pinned = nullptr;
+        cudaStream_t stream = nullptr;
+    };
+    std::vector<OutLane> out_lanes;       // copy_out's pinned chunks and streams (first large download)
+    void copy_out(void* dst, const void* src, size_t bytes);
+    void download_into(uint32_t* current, uint32_t* packed);   // host buffers, either may be null
     void download_state(std::vector<uint32_t>& current, std::vector<uint32_t>& packed);
     void apply_host(int what, const uint32_t* in, uint32_t* out);
     // kernel-vector recovery (bw_cyclic_recover.cu)

@@ -41,7 +41,7 @@ extern "C" int bw_cyclic_info_get(const bw_cyclic* ctx, bw_cyclic_info* out) {
         out->default_nlen = (2 * c.op_cols) / c.num_v + 50;
         out->seq_len = c.seq_len;
         out->rowmix_realized_seed = c.plan.realized_seed;
-        out->rowmix_hash = cyclic::rowmix_plan_hash(c.plan);
+        out->rowmix_hash = c.plan_hash;
         out->device_bytes = c.device_bytes;
         out->genus = static_cast<uint32_t>(c.inst.genus);
         out->prime = c.p;
@@ -92,13 +92,8 @@ extern "C" int bw_cyclic_download(bw_cyclic* ctx, uint32_t* packed_seq, uint64_t
         c.require_device();
         BW_REQUIRE(c.seq_len > 0, "bw_cyclic_download: no sequence generated");
         BW_CUDA(cudaSetDevice(c.device));
-        std::vector<uint32_t> cur, packed;
-        c.download_state(cur, packed);
-        if (packed_seq) {
-            BW_REQUIRE(seq_capacity >= c.seq_len, "bw_cyclic_download: sequence buffer too small");
-            std::memcpy(packed_seq, packed.data(), packed.size() * sizeof(uint32_t));
-        }
-        if (current) std::memcpy(current, cur.data(), cur.size() * sizeof(uint32_t));
+        if (packed_seq) BW_REQUIRE(seq_capacity >= c.seq_len, "bw_cyclic_download: sequence buffer too small");
+        c.download_into(current, packed_seq);
     });
 }
 

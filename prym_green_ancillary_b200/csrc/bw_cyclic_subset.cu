@@ -44,6 +44,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr uint32_t kLow26 = (1u << 26) - 1;
+constexpr int kResidentThreads = 512, kMomentThreads = 128, kResidentChunks = 4;   // sub_rounds_kernel: threads a CTA, chunks a gather, at most
 
 using cyc::Acc4;
 using cyc::ld4;
@@ -64,19 +65,13 @@ __device__ __forceinline__ void st_block(uint4* v, uint32_t s, const int4& r0, c
     v[s] = make_uint4(a.x, a.y, b.x, b.y);
 }
 
-// Views of the staged shared-memory tables.
+// Views of the shared-memory tables.
 struct Tables {
     const int4* coef;
     const int32_t *R, *B, *a0off, *a0idx, *a1off, *a1idx, *koff, *kidx, *ych;
 };
 
-// Staging reads only the constant tables, so it overlaps the end of the kernel
-// before (programmatic dependent launch); the wait follows it.
-__device__ __forceinline__ Tables stage(const SubsetDev& D, const int32_t* __restrict__ blob, int32_t* sm) {
-    cyc::pdl_trigger();
-    for (int w = threadIdx.x; w < D.blob_words; w += blockDim.x) sm[w] = __ldg(blob + w);
-    __syncthreads();
-    cyc::pdl_wait();
+__device__ __forceinline__ Tables views(const SubsetDev& D, const int32_t* sm) {
     Tables t;
     t.coef = reinterpret_cast<const int4*>(sm);
     t.R = sm + D.o_R;
@@ -89,6 +84,16 @@ __device__ __forceinline__ Tables stage(const SubsetDev& D, const int32_t* __res
     t.kidx = sm + D.o_kidx;
     t.ych = sm + D.o_ych;
     return t;
+}
+
+// Staging reads only the constant tables, so it overlaps the end of the kernel
+// before (programmatic dependent launch); the wait follows it.
+__device__ __forceinline__ Tables stage(const SubsetDev& D, const int32_t* __restrict__ blob, int32_t* sm) {
+    cyc::pdl_trigger();
+    for (int w = threadIdx.x; w < D.blob_words; w += blockDim.x) sm[w] = __ldg(blob + w);
+    __syncthreads();
+    cyc::pdl_wait();
+    return views(D, sm);
 }
 
 // Streamed table words: evict-first when the sector's tables exceed the L2
@@ -295,11 +300,17 @@ __global__ void __launch_bounds__(kThreads) sub_d2_forward_kernel(SubsetDev D, c
 // u2 = P u for the folded target preconditioner P = T^t Dr T in ELL form
 // ([slot][row] over the padded u2 slots, `ell` slots a row, coalesced across
 // threads; columns are positions of u in the locality order; empty slots hold
-// value 0).  Four slots at a time: their rows are
-// gathered together, and the next four slots' words are loaded meanwhile.
-template <bool SMALL, bool STREAM>
-__global__ void __launch_bounds__(kThreads) sub_ell_kernel(SubsetDev D, const uint2* __restrict__ u,
+// value 0).  SIX: a row of two rounds' pairings M1, M2 has the columns i, M1 i,
+// M2 i, M1 M2 i, M2 M1 i and M1 M2 M1 i, so `ell` is six and a row's words and
+// then its six rows of u are loaded together.  Otherwise four slots at a time:
+// their rows are gathered together, and the next four slots' words are loaded
+// meanwhile.  Bound by the latency of those loads: registers for all of them
+// (four CTAs an SM) are worth more than occupancy (an application at genus 26
+// 177.7 -> 165.4 us; with eight slots and eight CTAs 171.8).
+template <bool SMALL, bool STREAM, bool SIX>
+__global__ void __launch_bounds__(kThreads, 4) sub_ell_kernel(SubsetDev D, const uint2* __restrict__ u,
                                                            uint2* __restrict__ u2) {
+    constexpr int U = SIX ? 6 : 4;
     cyc::pdl_trigger();
     cyc::pdl_wait();
     const long long rows = 2 * static_cast<long long>(D.n2);
@@ -307,31 +318,32 @@ __global__ void __launch_bounds__(kThreads) sub_ell_kernel(SubsetDev D, const ui
         Acc4<SMALL> acc;
         const uint32_t* c = D.e_col + row;
         const int16_t* v = D.e_val + row;
-        uint32_t cc[4];
-        int32_t vv[4];
+        uint32_t cc[U];
+        int32_t vv[U];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < U; ++q) {
             cc[q] = ld_table<STREAM>(c + q * rows);
             vv[q] = ld_table<STREAM>(v + q * rows);
         }
-        for (uint32_t k = 0; k < D.ell; k += 4) {
-            uint2 x[4];
+        for (uint32_t k = 0; k < (SIX ? 1u : D.ell); k += U) {
+            uint2 x[U];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) x[q] = __ldg(u + cc[q]);
-            uint32_t nc[4];
-            int32_t nv[4];
-            if (k + 4 < D.ell) {
+            for (int q = 0; q < U; ++q) x[q] = __ldg(u + cc[q]);
+            uint32_t nc[U];
+            int32_t nv[U];
+            const bool more = !SIX && k + U < D.ell;
+            if (more) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    nc[q] = ld_table<STREAM>(c + (k + 4 + q) * rows);
-                    nv[q] = ld_table<STREAM>(v + (k + 4 + q) * rows);
+                for (int q = 0; q < U; ++q) {
+                    nc[q] = ld_table<STREAM>(c + (k + U + q) * rows);
+                    nv[q] = ld_table<STREAM>(v + (k + U + q) * rows);
                 }
             }
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc.mac(vv[q], unpack_row(x[q].x, x[q].y));
-            if (k + 4 < D.ell) {
+            for (int q = 0; q < U; ++q) acc.mac(vv[q], unpack_row(x[q].x, x[q].y));
+            if (more) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
+                for (int q = 0; q < U; ++q) {
                     cc[q] = nc[q];
                     vv[q] = nv[q];
                 }
@@ -500,6 +512,337 @@ __global__ void __launch_bounds__(kThreads) sub_dense_t_kernel(SubsetDev D, cons
         *counter = 0;
         __threadfence();
     }
+}
+
+// ----- whole rounds in one launch
+//
+// An application is five kernels, and on a small sector each costs about 4 us
+// whatever it does: the launch, the wait for the kernel before, and a chain of
+// dependent loads (a subset's word, its incidence words, its blocks chunk
+// after chunk).  Where every subset has a thread of its own and the tables fit
+// in shared memory, one cooperative launch runs many rounds instead: a
+// thread's incidence words and preconditioner entries stay in shared memory
+// and its coefficients in registers, so a phase is one round of gathers, all
+// in flight together, between two grid-wide barriers; the Gram moments of an
+// application are added up beside the next one's first phase.
+//
+// Microseconds an application, kernel by kernel -> so: genus 12 15.4 -> 7.8, 16
+// 20.3 -> 10.7, 20 24.1 -> 13.4, 22 34.5 -> 19.2, of which the five barriers
+// take 3.6 (one CTA pair) to 6.7.  (With the tables read from L2 it was 17.5,
+// 18.2, 22.7 and 29.1: the chain, not the launches, is what a phase costs.)
+struct RoundsArgs {
+    uint4 *xs, *y, *t_adj, *u2;
+    uint2* u;
+    int32_t *zs, *b, *d;          // scaled source's compact rows; the two compact blocks
+    const int32_t* dc;
+    long long rows;               // of the compact blocks
+    int32_t* sums;                // 20 accumulators, zero between launches
+    uint32_t* seq;
+    unsigned long long* seq_index;
+    unsigned int* arrivals;       // of all CTAs at all barriers (zero at launch)
+    int* err;                     // mapped host memory, written only on a give-up
+    unsigned int wait_limit;
+    int hold;                     // failure test: CTA 0 never arrives
+    int rounds;
+};
+
+// All CTAs of a cooperative launch meet (the `count`-th time); `threads` of
+// every CTA take part at hardware barrier `id`, the subset threads here and the
+// others in grid_barrier_join.  Thread 0 releases its CTA's writes and acquires
+// the others'; data written in this launch is read at L2 (__ldcg).  One counter
+// that one thread a CTA polls: 1.0 to 1.2 us (148 flags polled side by side by
+// every CTA: 3.5 us).  The wait is bounded: a CTA that runs out of tries
+// reports it and returns, and so do then the others.
+__device__ __forceinline__ void cta_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ bool grid_barrier(const RoundsArgs& A, unsigned int count, int id, int threads,
+                                             volatile int* gave_up /* shared */) {
+    cta_sync(id, threads);
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(A.arrivals) : "memory");
+        const unsigned int target = count * gridDim.x;
+        unsigned int tries = 0, v;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(A.arrivals) : "memory");
+        } while (v < target && ++tries < A.wait_limit);
+        if (v < target) {
+            *gave_up = 1;
+            *reinterpret_cast<volatile int*>(A.err) = 1;
+        }
+    }
+    cta_sync(id, threads);
+    return *gave_up == 0;
+}
+
+// The part in it of threads that only wait for the CTA's polling threads.
+__device__ __forceinline__ bool grid_barrier_join(volatile int* gave_up, int all) {
+    cta_sync(0, all);
+    cta_sync(0, all);
+    return *gave_up == 0;
+}
+
+__device__ __forceinline__ int tri(int row, int col) { return row * (2 * 4 - row + 1) / 2 + (col - row); }
+
+// Adds the packed upper triangles of B^t D and O^t O (O: the newer of the two)
+// over all rows to A.sums, by the kMomentThreads threads that call it in every
+// CTA (t: the thread's number among them).
+__device__ __forceinline__ void add_moments(const RoundsArgs& A, bool b_is_newer, const Mod& mod, int t) {
+    int32_t acc[20];
+#pragma unroll
+    for (int e = 0; e < 20; ++e) acc[e] = 0;
+    int cnt = 0;
+    for (long long row = static_cast<long long>(blockIdx.x) * kMomentThreads + t; row < A.rows;
+         row += static_cast<long long>(gridDim.x) * kMomentThreads) {
+        const int4 b = __ldcg(reinterpret_cast<const int4*>(A.b) + row);
+        const int4 d = __ldcg(reinterpret_cast<const int4*>(A.d) + row), o = b_is_newer ? b : d;
+        const int bv[4] = {b.x, b.y, b.z, b.w}, dv[4] = {d.x, d.y, d.z, d.w}, ov[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+        for (int r0 = 0; r0 < 4; ++r0)
+#pragma unroll
+            for (int c0 = r0; c0 < 4; ++c0) {
+                acc[tri(r0, c0)] += bv[r0] * dv[c0];
+                acc[10 + tri(r0, c0)] += ov[r0] * ov[c0];
+            }
+        if (++cnt == 8) {
+            cnt = 0;
+#pragma unroll
+            for (int e = 0; e < 20; ++e) acc[e] = reduce_partial(acc[e], mod);
+        }
+    }
+    const int lane = t % 32;
+    int32_t mine = 0;
+#pragma unroll
+    for (int e = 0; e < 20; ++e) {
+        const int32_t v = __reduce_add_sync(0xffffffffu, reduce_balanced(acc[e], mod));
+        if (lane == e) mine = v;
+    }
+    // at most 148 * 4 warps of 32 balanced values: far below 2^31
+    if (lane < 20) atomicAdd(A.sums + lane, mine);
+}
+
+// Gathers of one subset whose words lie in shared memory ([position][thread],
+// padded to chunks of four with words of the zero block): eight blocks are in
+// flight before their products.
+template <bool SMALL>
+__device__ __forceinline__ void gather_resident(const uint32_t* words, int stride, int chunks, const int4* coef, int r,
+                                                int ch, const uint4* in, Acc4<SMALL>& acc0, Acc4<SMALL>& acc1) {
+#pragma unroll
+    for (int c0 = 0; c0 < kResidentChunks; c0 += 2) {
+        if (c0 >= chunks) break;
+        const bool two = c0 + 1 < chunks;
+        uint32_t w[8];
+        uint4 b[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (u < 4 || two) {
+                w[u] = words[(4 * c0 + u) * stride];
+                b[u] = __ldcg(in + (w[u] & kLow26));
+            }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (u < 4 || two) mac_block<SMALL>(coef[static_cast<int>(w[u] >> 26) * r + ch], b[u], acc0, acc1);
+    }
+}
+
+// Shared memory: the two coefficient blobs, then per subset thread (stride T)
+// the padded words of the four gathers and the columns and values of its two
+// preconditioner rows.  Subset thread t of the grid owns the t-th m-, (m-1)-
+// and (m-2)-subset; each CTA's last kMomentThreads threads add up the moments
+// of the application before, beside the first three phases (in the subset
+// threads that took 3.5 us an application).
+template <bool SMALL>
+__global__ void __launch_bounds__(kResidentThreads, 1) sub_rounds_kernel(SubsetDev D, RoundsArgs A) {
+    extern __shared__ int32_t sm[];
+    __shared__ int gave_up;
+    const int all = blockDim.x, T = all - kMomentThreads, tid = threadIdx.x;
+    const int blob4 = (D.blob_words + 3) / 4 * 4;
+    for (int w = tid; w < D.blob_words; w += all) {
+        sm[w] = __ldg(D.blob_f + w);
+        sm[blob4 + w] = __ldg(D.blob_t + w);
+    }
+    if (tid == 0) gave_up = 0;
+    if (A.hold && blockIdx.x == 0) return;
+    if (tid >= T) {
+        // ------------------------------------------------ moments
+        // joins the third barrier (the older block is overwritten after it)
+        // and the fifth (the newer one is complete)
+        __syncthreads();
+        for (int app = 0; app < 2 * A.rounds; ++app) {
+            if (app > 0) add_moments(A, (app & 1) == 0, D.mod, tid - T);
+            if (!grid_barrier_join(&gave_up, all) || !grid_barrier_join(&gave_up, all)) return;
+        }
+        add_moments(A, true, D.mod, tid - T);
+        grid_barrier_join(&gave_up, all);
+        return;
+    }
+    const uint32_t id = blockIdx.x * static_cast<uint32_t>(T) + tid;
+    const bool has0 = id < D.n0, has1 = id < D.n1, has2 = id < D.n2;
+    const int c_dmf = (D.w_dmf + 3) / 4, c_d2f = (D.w_d2f + 3) / 4, c_d2t = (D.w_d2t + 3) / 4, c_dmt = (D.w_dmt + 3) / 4;
+    uint32_t* const w_dmf = reinterpret_cast<uint32_t*>(sm) + 2 * blob4 + tid;
+    uint32_t* const w_d2f = w_dmf + 4 * c_dmf * T;
+    uint32_t* const w_d2t = w_d2f + 4 * c_d2f * T;
+    uint32_t* const w_dmt = w_d2t + 4 * c_d2t * T;
+    uint32_t* const e_col = w_dmt + 4 * c_dmt * T;     // [12][T]: six slots of either row
+    int32_t* const e_val = reinterpret_cast<int32_t*>(e_col + 12 * T);
+    auto keep_words = [&](uint32_t* dst, const uint32_t* inc, bool has, uint32_t n, uint32_t width, uint32_t nin) {
+        for (uint32_t k = 0; k < (width + 3) / 4 * 4; ++k)
+            dst[k * T] = has && k < width ? __ldg(inc + static_cast<size_t>(k) * n + id) : nin;
+    };
+    keep_words(w_dmf, D.inc_dmf, has1, D.n1, D.w_dmf, D.n0);
+    keep_words(w_d2f, D.inc_d2f, has2, D.n2, D.w_d2f, D.n1);
+    keep_words(w_d2t, D.inc_d2t, has1, D.n1, D.w_d2t, D.n2);
+    keep_words(w_dmt, D.inc_dmt, has0, D.n0, D.w_dmt, D.n1);
+    for (int q = 0; q < 12; ++q) {
+        const long long at = (q % 6) * (2 * static_cast<long long>(D.n2)) + 2 * static_cast<long long>(id) + q / 6;
+        e_col[q * T] = has2 ? __ldg(D.e_col + at) : 0u;
+        e_val[q * T] = has2 ? __ldg(D.e_val + at) : 0;
+    }
+    __syncthreads();
+    const Tables F = views(D, sm), B = views(D, sm + blob4);
+
+    // (m-1)-subset: y = B z - R t forward, t_adj = R^t h and z = B^t h back, with
+    // zero coefficients where the block has fewer rows
+    int tch = 0, ych = 0, ny = 0, nt = 0, nz = 0;
+    long long zrow = 0;
+    int32_t cB[2][2] = {}, cR[2][2] = {}, dcz[2] = {};   // [y row][z or t row]
+    if (has1) {
+        const uint32_t d = __ldg(D.m1 + id);
+        tch = static_cast<int>(d >> 26);
+        ych = F.ych[tch];
+        zrow = d & kLow26;
+        ny = F.a0off[ych + 1] - F.a0off[ych];
+        nt = F.a1off[tch + 1] - F.a1off[tch];
+        nz = F.koff[ych + 1] - F.koff[ych];
+        for (int q = 0; q < ny; ++q) {
+            const int a = F.a0idx[F.a0off[ych] + q];
+            for (int j = 0; j < nz; ++j) cB[q][j] = F.B[a * D.kdim + F.kidx[F.koff[ych] + j]];
+            for (int j = 0; j < nt; ++j) cR[q][j] = F.R[a * D.n + F.a1idx[F.a1off[tch] + j]];
+        }
+        for (int j = 0; j < nz; ++j) dcz[j] = __ldg(A.dc + D.x_cols + zrow + j);
+    }
+    // (m-2)-subset: the positions of its u rows
+    int uch = 0, nu = 0;
+    uint32_t upos[2] = {};
+    if (has2) {
+        const uint32_t d = __ldg(D.m2 + id);
+        uch = static_cast<int>(d >> 26);
+        nu = F.a1off[uch + 1] - F.a1off[uch];
+        for (int q = 0; q < nu; ++q) upos[q] = __ldg(D.u_pos + (d & kLow26) + q);
+    }
+    // m-subset: its compact rows and their column preconditioner
+    int xch = 0, nx = 0;
+    long long xrow = 0;
+    int32_t dcx[2] = {};
+    if (has0) {
+        const uint32_t d = __ldg(D.m0 + id);
+        xch = static_cast<int>(d >> 26);
+        nx = F.a0off[xch + 1] - F.a0off[xch];
+        xrow = d & kLow26;
+        for (int q = 0; q < nx; ++q) dcx[q] = __ldg(A.dc + xrow + q);
+    }
+
+    const unsigned long long pos = *A.seq_index;
+    unsigned int met = 0;
+    // the sums of application `app`, complete after a barrier, to the sequence
+    auto write_moments = [&](int app) {
+        if (blockIdx.x == 0 && tid < 20) {
+            const int32_t total = atomicExch(A.sums + tid, 0);
+            A.seq[(pos + 2ull * app) * 10 + tid] = to_canonical(reduce_balanced(total, D.mod), D.mod);
+        }
+    };
+    const int4 zero = make_int4(0, 0, 0, 0);
+    // subset threads alone, or with the moments' threads
+    // (a give-up there lets the moments' threads out of the barrier they wait at)
+    auto subset_barrier = [&] {
+        if (grid_barrier(A, ++met, 1, T, &gave_up)) return true;
+        grid_barrier_join(&gave_up, all);
+        return false;
+    };
+    auto full_barrier = [&] { return grid_barrier(A, ++met, 0, all, &gave_up); };
+    for (int app = 0; app < 2 * A.rounds; ++app) {
+        int32_t* out = (app & 1) ? A.b : A.d;
+        if (has1) {
+            int4 z[2] = {zero, zero};
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if (j < nz) z[j] = __ldcg(reinterpret_cast<const int4*>(A.zs) + zrow + j);
+            Acc4<SMALL> t0, t1;
+            gather_resident<SMALL>(w_dmf, T, c_dmf, F.coef, D.r, tch, A.xs, t0, t1);
+            const int4 t[2] = {t0.reduce(D.mod), t1.reduce(D.mod)};
+            int4 y[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                Acc4<SMALL> acc;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    acc.mac(cB[q][j], z[j]);
+                    acc.mac(-cR[q][j], t[j]);
+                }
+                y[q] = acc.reduce(D.mod);
+            }
+            st_block(A.y, id, y[0], y[1]);
+        }
+        if (!subset_barrier()) return;
+        if (has2) {
+            Acc4<SMALL> u0, u1;
+            gather_resident<SMALL>(w_d2f, T, c_d2f, F.coef, D.r, uch, A.y, u0, u1);
+            if (nu > 0) A.u[upos[0]] = pack_row(u0.reduce(D.mod));
+            if (nu > 1) A.u[upos[1]] = pack_row(u1.reduce(D.mod));
+        }
+        if (!subset_barrier()) return;
+        if (has2) {
+            uint2 x[12];
+#pragma unroll
+            for (int q = 0; q < 12; ++q) x[q] = __ldcg(A.u + e_col[q * T]);
+            Acc4<SMALL> p[2];
+#pragma unroll
+            for (int q = 0; q < 12; ++q) p[q / 6].mac(e_val[q * T], unpack_row(x[q].x, x[q].y));
+            st_block(A.u2, id, p[0].reduce(D.mod), p[1].reduce(D.mod));
+        }
+        if (!full_barrier()) return;
+        if (app > 0) write_moments(app - 1);   // complete since the third barrier
+        if (has1) {
+            Acc4<SMALL> h0, h1;
+            gather_resident<SMALL>(w_d2t, T, c_d2t, B.coef, D.r, ych, A.u2, h0, h1);
+            const int4 h[2] = {ny > 0 ? h0.reduce(D.mod) : zero, ny > 1 ? h1.reduce(D.mod) : zero};
+            int4 t[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                Acc4<SMALL> acc, az;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    acc.mac(cR[q][j], h[q]);
+                    az.mac(cB[q][j], h[q]);
+                }
+                t[j] = acc.reduce(D.mod);
+                if (j < nz) {
+                    const int4 o = scale4(az.reduce(D.mod), dcz[j], D.mod);
+                    st4(out, static_cast<long long>(D.x_cols) + zrow + j, o);
+                    st4(A.zs, zrow + j, scale4(o, dcz[j], D.mod));   // next source row
+                }
+            }
+            st_block(A.t_adj, id, t[0], t[1]);
+        }
+        if (!subset_barrier()) return;
+        if (has0 && nx > 0) {
+            Acc4<SMALL> x0, x1;
+            gather_resident<SMALL>(w_dmt, T, c_dmt, B.coef, D.r, xch, A.t_adj, x0, x1);
+            int4 next[2] = {zero, zero};
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                if (q < nx) {
+                    const int4 o = scale4(neg4(q == 0 ? x0.reduce(D.mod) : x1.reduce(D.mod)), dcx[q], D.mod);
+                    st4(out, xrow + q, o);
+                    next[q] = scale4(o, dcx[q], D.mod);
+                }
+            st_block(A.xs, id, next[0], next[1]);   // next application's source block
+        }
+        if (!full_barrier()) return;
+    }
+    if (!full_barrier()) return;   // the last application's moments
+    write_moments(2 * A.rounds - 1);
+    if (blockIdx.x == 0 && tid == 0) *A.seq_index = pos + 4ull * A.rounds;
 }
 
 // Compact int32 rows <-> padded int16 blocks of the (m-2)-subsets: u2 in the
@@ -702,6 +1045,63 @@ void CyclicCtx::setup_subset_path() {
     BW_CUDA(cudaMemsetAsync(d_t16, 0, (D.n1 + 1) * sizeof(uint4), stream));
     BW_CUDA(cudaMemsetAsync(d_u2_16, 0, (D.n2 + 1) * sizeof(uint4), stream));
     subset_path = true;
+    setup_rounds();
+}
+
+// Whether generate() runs whole rounds in one cooperative launch
+// (sub_rounds_kernel): the eliminated operator with two row-mixing rounds,
+// every subset with a thread of its own in one CTA an SM, and the tables in
+// shared memory (the published genera up to 22).  BW_CYCLIC_PERSISTENT=0 turns
+// it off.
+void CyclicCtx::setup_rounds() {
+    if (const char* env = std::getenv("BW_CYCLIC_PERSISTENT"))
+        if (std::string(env) == "0") return;
+    if (S.n_extra != 0 || S.drop0 >= 0 || S.ell != 6) return;
+    auto chunks = [](uint32_t w) { return (w + 3) / 4; };
+    if (std::max({chunks(S.w_dmf), chunks(S.w_d2f), chunks(S.w_d2t), chunks(S.w_dmt)}) > kResidentChunks) return;
+    const uint32_t items = std::max({S.n0, S.n1, S.n2});
+    const uint32_t per_sm = (items + sms - 1) / sms, threads = std::max(64u, (per_sm + 31) / 32 * 32);
+    if (threads + kMomentThreads > kResidentThreads) return;
+    const uint32_t words = 4 * (chunks(S.w_dmf) + chunks(S.w_d2f) + chunks(S.w_d2t) + chunks(S.w_dmt)) + 24;
+    rounds_smem = (static_cast<size_t>(2 * ((S.blob_words + 3) / 4 * 4)) + static_cast<size_t>(words) * threads) * 4;
+    auto kern = small ? sub_rounds_kernel<true> : sub_rounds_kernel<false>;
+    if (rounds_smem > static_cast<size_t>(allow_dynamic_smem(kern, device))) return;
+    int coop = 0, occ = 0;
+    BW_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
+    BW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, static_cast<int>(threads) + kMomentThreads,
+                                                          rounds_smem));
+    if (!coop || occ < 1) return;
+    rounds_threads = static_cast<int>(threads) + kMomentThreads;
+    rounds_grid = (items + threads - 1) / threads;
+    d_barrier = alloc<uint32_t>(1);
+    void* word = nullptr;
+    BW_CUDA(cudaHostAlloc(&word, sizeof(int), cudaHostAllocMapped));
+    h_err = static_cast<volatile int*>(word);
+    *h_err = 0;
+    BW_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&d_err), word, 0));
+    if (const char* e = std::getenv("BW_TEST_WAIT_LIMIT")) {
+        const unsigned long v = std::strtoul(e, nullptr, 10);
+        if (v >= 1 && v < rounds_wait_limit) rounds_wait_limit = static_cast<uint32_t>(v);
+    }
+    if (const char* e = std::getenv("BW_TEST_HOLD_FIRST_STAGE")) rounds_hold = (*e && std::string(e) != "0") ? 1 : 0;
+    persistent = true;
+}
+
+void CyclicCtx::subset_rounds(size_t rounds) {
+    RoundsArgs A{d_xs16, d_y16, d_t16, d_u2_16, reinterpret_cast<uint2*>(d_u16), d_zs, d_b, d_d, d_dc,
+                 static_cast<long long>(op_cols), d_partials, d_seq, d_seq_index, d_barrier, d_err, rounds_wait_limit,
+                 rounds_hold, 0};
+    auto kern = small ? sub_rounds_kernel<true> : sub_rounds_kernel<false>;
+    for (size_t done = 0; done < rounds; done += A.rounds) {
+        // bounded launches: 10 barriers a round keep the arrival count far below 2^32
+        A.rounds = static_cast<int>(std::min<size_t>(rounds - done, 1024));
+        BW_CUDA(cudaMemsetAsync(d_barrier, 0, sizeof(uint32_t), stream));
+        void* args[] = {&S, &A};
+        BW_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), dim3(rounds_grid),
+                                            dim3(rounds_threads), args, rounds_smem, stream));
+        ++launches;
+    }
+    xs_for = d_b;
 }
 
 // Kernel template dispatch: SMALL (int32 sums exact) x STREAM (tables above L2).
@@ -744,7 +1144,11 @@ void CyclicCtx::subset_precondition16() {
     const uint2* u = reinterpret_cast<const uint2*>(d_u16);
     uint2* u2 = reinterpret_cast<uint2*>(d_u2_16);
     const unsigned grid = grid_for(2 * static_cast<size_t>(S.n2));
-#define BW_LAUNCH(A, B) launch_pdl(sub_ell_kernel<A, B>, grid, 0, S, u, u2)
+#define BW_LAUNCH(A, B)                                            \
+    if (S.ell == 6)                                                \
+        launch_pdl(sub_ell_kernel<A, B, true>, grid, 0, S, u, u2); \
+    else                                                           \
+        launch_pdl(sub_ell_kernel<A, B, false>, grid, 0, S, u, u2)
     BW_SUBSET_DISPATCH(BW_LAUNCH);
 #undef BW_LAUNCH
     BW_CHECK_LAUNCH();

@@ -962,7 +962,7 @@ std::string build_subset_tables(const Instance& inst, const EliminatedSector& es
     for (size_t q = 0; q < es.target_rows; ++q)
         widest = std::max<size_t>(widest, precond.row_ptr[q + 1] - precond.row_ptr[q]);
     if (widest > 64) return "preconditioner above 64 entries a row";
-    out.ell = (widest + 3) / 4 * 4;
+    out.ell = widest <= 6 && widest > 4 ? 6 : (widest + 3) / 4 * 4;   // six: two row-mixing rounds (see the kernel)
     const size_t rows = 2 * n2;
     if (rows * out.ell >= (1ull << 32)) return "preconditioner above 2^32 slots";
     out.e_col.assign(rows * out.ell, 0u);
