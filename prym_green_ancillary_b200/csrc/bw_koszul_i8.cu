@@ -1137,7 +1137,7 @@ struct KoszulCtx::I8State {
         std::vector<uint32_t> mask;      // [tile] union of its blocks' generators
         uint32_t* d_mask = nullptr;
         uint32_t *start = nullptr, *words = nullptr, *steps = nullptr;   // stage list of list_gs generators a stage
-        int list_gs = 0;
+        int list_gs = 0, list_issuers = 0;
     } fwd, bwd;
     // Y_a, Y_b, Z: lo, hi, -lo, -hi; each -plane directly follows its +plane in
     // memory, so that one tensor map covers both signs of a limb
@@ -1168,6 +1168,7 @@ struct TuneChoice {
     int pw = 8;             // cp.async producer warps
     int gps = 0;            // generators per stage (dense and union kernels)
     int t_tma = 0;          // hybrid: blocks of a tile gathered by TMA; union: producer groups
+    int issuers = 1;        // union: MMA warps
     double ms = 0;
 };
 std::mutex g_tune_mutex;
@@ -1358,12 +1359,13 @@ __global__ void union_mask_kernel(const uint32_t* __restrict__ inc, uint32_t* __
     mask[tile] = m;
 }
 
-// Plans one direction of the union kernel with gs generators a stage and pw
-// producer warps in groups; false when it does not fit (shared memory for the
-// resident maps and at least two slots, one table word and one step word a
-// lane, kUnionPasses passes).
-bool plan_union(KoszulCtx& c, KoszulCtx::I8State::Dir& D, int inner, int outer, bool transpose_dir, int gs, int pw,
-                int groups) {
+// Plans one direction of the union kernel with gs generators a stage, the
+// producer warps in so many groups and one or two MMA warps; false when it does
+// not fit (shared memory for the resident maps and at least two slots, one
+// table word and one step word a lane, kUnionPasses passes, a stage a tile for
+// either MMA warp).
+bool plan_union(KoszulCtx& c, KoszulCtx::I8State::Dir& D, int inner, int outer, bool transpose_dir, int gs, int groups,
+                int issuers) {
     I8Union& U = D.u;
     const int bt = 128 / c.nbi, run = (c.nbi / 16) * inner;
     U.r = c.r;
@@ -1373,6 +1375,7 @@ bool plan_union(KoszulCtx& c, KoszulCtx::I8State::Dir& D, int inner, int outer, 
     U.cpg = (2 * inner + 15) / 16;
     U.gs = gs;
     U.groups = groups;
+    U.issuers = issuers;
     U.row = ((gs * U.cpg + 1) / 2 + 3) / 4 * 4;
     // Without a reduction of hi on its own the epilogue's first sum is lo + 255
     // hi over at most n = incident generators x inner pairs of rows, each below
@@ -1382,7 +1385,7 @@ bool plan_union(KoszulCtx& c, KoszulCtx::I8State::Dir& D, int inner, int outer, 
     U.wide = (transpose_dir ? c.k : c.r - c.k + 1) * inner > 500;
     const bool odd = (U.cpg & 1) != 0;
     if (gs < 1 || (odd && gs % 2 != 0) || gs * bt > 32 || U.row > kUnionSteps) return false;
-    if (gs * bt * run > pw / groups * 32 * kUnionPasses) return false;
+    if (gs * bt * run > union_warps::producers / groups * 32 * kUnionPasses) return false;
     const size_t b = (static_cast<size_t>(c.r) * U.cpg + (odd ? 1 : 0)) * 2 * U.ho * 16;
     const size_t slot = static_cast<size_t>(gs) * U.cpg * 16 * 128;
     const size_t extra = (2 * 8 + 2 * 2 + 2) * 8 + 16;
@@ -1390,10 +1393,15 @@ bool plan_union(KoszulCtx& c, KoszulCtx::I8State::Dir& D, int inner, int outer, 
     U.b_bytes = static_cast<uint32_t>(b);
     U.slot_bytes = static_cast<uint32_t>(slot);
     U.slots = static_cast<int>(std::min<size_t>(8, (kMaxSmem - b - extra) / slot));
-    if (U.slots < groups) return false;
+    // Two MMA warps take the stages in turn: every tile has to have a stage for
+    // either (a block alone has so many generators), and a slot has to belong to
+    // one of them for good, or one could run a lap ahead of the other and take a
+    // barrier's phase for the next but one.
+    const int least = transpose_dir ? c.k : c.r - c.k + 1;
+    if (issuers == 2) U.slots &= ~1;
+    if (U.slots < std::max(2, groups) || (issuers == 2 && least <= gs)) return false;
     U.mod = c.mod;
     U.maps = D.maps;
-    D.pw = pw;
     D.smem = b + U.slots * slot + extra;
     return true;
 }
@@ -1425,7 +1433,7 @@ std::vector<int8_t> union_maps(const KoszulCtx& c, int inner, int outer, bool tr
 // c + grid, ..., their stages one after the other.
 void build_stage_list(KoszulCtx& c, KoszulCtx::I8State::Dir& D, uint64_t n_blk, uint64_t n_in, int inner) {
     I8Union& U = D.u;
-    if (D.list_gs != U.gs) {
+    if (D.list_gs != U.gs || D.list_issuers != U.issuers) {
         for (uint32_t** p : {&D.start, &D.words, &D.steps})
             if (*p) {
                 c.release(*p);
@@ -1452,11 +1460,12 @@ void build_stage_list(KoszulCtx& c, KoszulCtx::I8State::Dir& D, uint64_t n_blk, 
         const uint32_t run16 = static_cast<uint32_t>((c.nbi / 16) * inner);
         union_tables_kernel<<<blocks_of(tiles, 128), 128, 0, c.own_stream>>>(
             D.inc, D.d_mask, d_ts, D.words, D.steps, static_cast<long long>(tiles), static_cast<long long>(n_blk), c.r,
-            bt, U.gs, U.cpg, 2 * U.ho, U.row, run16, static_cast<uint32_t>(n_in * run16));
+            bt, U.gs, U.cpg, 2 * U.ho, U.row, U.issuers, run16, static_cast<uint32_t>(n_in * run16));
         BW_CHECK_LAUNCH();
         BW_CUDA(cudaStreamSynchronize(c.own_stream));
         c.release(d_ts);
         D.list_gs = U.gs;
+        D.list_issuers = U.issuers;
     }
     U.start = D.start;
     U.words = D.words;
@@ -1549,10 +1558,7 @@ void launch_i8(KoszulCtx& c, KoszulCtx::I8State::Dir& D, const CUtensorMap* maps
     if (D.use_union) {
         BW_REQUIRE(D.u.start != nullptr && D.u.words != nullptr && D.u.steps != nullptr && D.u.maps != nullptr,
                    "internal: INT8 stage list missing for the union kernel");
-        if (D.pw == 16)
-            launch_dependent(i8_union_gemm_kernel<NB, 16>, D.grid, GatherWarps<16>::threads, D.smem, st, D.u);
-        else
-            launch_dependent(i8_union_gemm_kernel<NB, 8>, D.grid, GatherWarps<8>::threads, D.smem, st, D.u);
+        launch_dependent(i8_union_gemm_kernel<NB>, D.grid, union_warps::threads, D.smem, st, D.u);
         BW_CHECK_LAUNCH();
         ++c.launches;
         return;
@@ -1626,11 +1632,11 @@ void KoszulCtx::i8_setup() {
     // producers' only where the union kernel's resident maps leave room for
     // fewer than eight generators in flight (maps of 2 r inner rows: r * inner
     // * outer above about 32,000).  With more room the union kernel won at every
-    // shape timed (us, dense against union: r=19 k=9 20->28 n=16 179/130 d and
-    // 228/156 d^T; r=21 k=10 32->40 n=32 1726/1190 and 2429/1411).
+    // shape timed (us, dense against union: r=19 k=9 20->28 n=16 179/92 d and
+    // 228/127 d^T; r=21 k=10 32->40 n=32 1726/1050 and 2429/1260).
     struct Cand {
-        int kind;               // 0 dense cp.async, 1 dense hybrid, 2 union
-        int gps, t_tma, pw;     // as in TuneChoice
+        int kind;                        // 0 dense cp.async, 1 dense hybrid, 2 union
+        int gps, t_tma, pw, issuers;     // as in TuneChoice
     };
     std::vector<Cand> cands[2];
     TuneKey keys[2];
@@ -1640,17 +1646,18 @@ void KoszulCtx::i8_setup() {
         const uint64_t n_out = dir == 0 ? n_t : n_s, n_in = dir == 0 ? n_s : n_t;
         const int inner = dir == 0 ? ci : co, outer = dir == 0 ? co : ci, bt = 128 / nbi;
         int in_flight = 0;      // generators, of the roomiest union plan
-        // four to eight generators a stage (fewer, where those do not fit, pay a
-        // hand-over between the roles for less work), warps in 2 or 4 groups
-        for (const auto& sizes : {std::vector<int>{4, 6, 8}, std::vector<int>{3, 2}})
-            for (int g : sizes)
-                for (int pw : pws)
-                    for (int groups : {2, 4}) {
-                        if (!allow_union || !plan_union(*this, D, inner, outer, dir == 1, g, pw, groups)) continue;
-                        if (g < 4 && !cands[dir].empty() && cands[dir][0].gps >= 4) continue;
-                        cands[dir].push_back({2, g, groups, pw});
+        // four generators a stage or near it (fewer leave room for more slots but
+        // pay a hand-over between the roles for less work), in 2 or 4 groups; two
+        // MMA warps where they fit (us at the two sizes of bw_koszul_i8_union.cuh,
+        // one warp / two: d 130/92 and 1190/1050, d^T 156/127 and 1410/1260)
+        for (int g : {4, 3, 6, 8, 2}) {
+            for (int groups : {2, 4})
+                for (int issuers : {2, 1})
+                    if (allow_union && plan_union(*this, D, inner, outer, dir == 1, g, groups, issuers)) {
+                        cands[dir].push_back({2, g, groups, 8, issuers});
                         in_flight = std::max(in_flight, D.u.slots * g);
                     }
+        }
         const bool dense = (allow_g4 || allow_cp) && in_flight < 8;
         BW_REQUIRE(!cands[dir].empty() || dense, "INT8 form: no union plan fits in shared memory");
         if (dense) {
@@ -1658,13 +1665,13 @@ void KoszulCtx::i8_setup() {
                 // the fill heuristic's stage, and fewer or more generators a stage
                 // (smaller stages leave room for more pipeline slots)
                 for (int pw : pws) {
-                    cands[dir].push_back({0, 0, 0, pw});
+                    cands[dir].push_back({0, 0, 0, pw, 1});
                     for (int g : {4, 6, 8, 12})
-                        if (g < r) cands[dir].push_back({0, g, 0, pw});
+                        if (g < r) cands[dir].push_back({0, g, 0, pw, 1});
                 }
             if (allow_g4)
                 for (int gs = 1; gs <= std::min(3, (r + 3) / 4); ++gs)
-                    for (int qt = 1; qt <= 3; ++qt) cands[dir].push_back({1, 4 * gs, qt * bt / 4, 8});
+                    for (int qt = 1; qt <= 3; ++qt) cands[dir].push_back({1, 4 * gs, qt * bt / 4, 8, 1});
         }
         keys[dir] = TuneKey{r, k, inner, outer, nbi, dir, sms,
                             (allow_g4 ? 1 : 0) | (allow_cp ? 2 : 0) | (pws.size() == 1 ? pws[0] * 4 : 0) |
@@ -1672,7 +1679,7 @@ void KoszulCtx::i8_setup() {
         TuneChoice known{};
         // a shape tuned earlier in this process: its choice alone
         if (tune && tune_lookup(keys[dir], known))
-            cands[dir] = {{known.kind, known.gps, known.t_tma, known.pw}};
+            cands[dir] = {{known.kind, known.gps, known.t_tma, known.pw, known.issuers}};
         // the tables that the candidates read
         bool any_union = false, any_rows = false;
         for (const Cand& c : cands[dir]) {
@@ -1726,8 +1733,7 @@ void KoszulCtx::i8_setup() {
     dispatch_i8_nb(nbi, [&](auto NBc) {
         cap_g = std::min(allow_dynamic_smem(i8_gather_gemm_kernel<decltype(NBc)::value, 8>, device),
                          allow_dynamic_smem(i8_gather_gemm_kernel<decltype(NBc)::value, 16>, device));
-        cap_u = std::min(allow_dynamic_smem(i8_union_gemm_kernel<decltype(NBc)::value, 8>, device),
-                         allow_dynamic_smem(i8_union_gemm_kernel<decltype(NBc)::value, 16>, device));
+        cap_u = allow_dynamic_smem(i8_union_gemm_kernel<decltype(NBc)::value>, device);
         cap_4 = allow_dynamic_smem(i8_gather_hybrid_kernel<decltype(NBc)::value>, device);
         const int cap_p = allow_dynamic_smem(i8_project_tc_kernel<decltype(NBc)::value>, device);
         BW_REQUIRE(static_cast<int>(S.proj_smem) <= cap_p, "INT8 form: shared-memory plan above the device limit");
@@ -1753,7 +1759,7 @@ void KoszulCtx::i8_setup() {
         auto plan = [&](const Cand& c) {
             D.use_union = c.kind == 2;
             if (D.use_union) {
-                if (!plan_union(*this, D, inner, outer, dir == 1, c.gps, c.pw, c.t_tma) ||
+                if (!plan_union(*this, D, inner, outer, dir == 1, c.gps, c.t_tma, c.issuers) ||
                     static_cast<int>(D.smem) > cap_u)
                     return false;
                 build_stage_list(*this, D, dir == 0 ? n_t : n_s, dir == 0 ? n_s : n_t, inner);
@@ -1792,8 +1798,8 @@ void KoszulCtx::i8_setup() {
                 char buf[96];
                 const char* sep = tried.empty() ? "" : ", ";
                 if (cand.kind == 2)
-                    std::snprintf(buf, sizeof buf, "%sunion stage=%d warps=%d/%d: %.4f ms", sep, cand.gps, cand.pw,
-                                  cand.t_tma, ms);
+                    std::snprintf(buf, sizeof buf, "%su%d/%d/%d %.4f", sep, cand.gps, cand.t_tma,
+                                  cand.issuers, ms);
                 else if (cand.kind == 1)
                     std::snprintf(buf, sizeof buf, "%shybrid stage=%d tma=%d/%d: %.4f ms", sep, D.p.gi, cand.t_tma, bt,
                                   ms);
@@ -1802,18 +1808,18 @@ void KoszulCtx::i8_setup() {
                 tried += buf;
                 if (ms < best) {
                     best = ms;
-                    choice = {cand.kind, cand.kind == 2 ? cand.gps : D.p.gi, cand.t_tma, cand.pw};
+                    choice = {cand.kind, cand.kind == 2 ? cand.gps : D.p.gi, cand.t_tma, cand.pw, cand.issuers};
                 }
             }
             BW_REQUIRE(best < 1e30, "INT8 form: no stage plan fits in shared memory");
-            tune_store(keys[dir], TuneChoice{choice.kind, choice.pw, choice.gps, choice.t_tma, best});
+            tune_store(keys[dir], TuneChoice{choice.kind, choice.pw, choice.gps, choice.t_tma, choice.issuers, best});
         }
         BW_REQUIRE(plan(choice), "INT8 form: maps too large for shared memory");
         D.gather4 = !D.use_union && D.gather4;
-        char buf[192];
+        char buf[256];
         if (D.use_union)
-            std::snprintf(buf, sizeof buf, "%s: union stage=%d generators, %d producer warps in %d groups, %d slots, "
-                          "%zu B shared", dir == 0 ? "d" : "d^T", D.u.gs, D.pw, D.u.groups, D.u.slots, D.smem);
+            std::snprintf(buf, sizeof buf, "%s: union stage=%d generators, %d producer groups, %d MMA warps, %d slots, "
+                          "%zu B shared", dir == 0 ? "d" : "d^T", D.u.gs, D.u.groups, D.u.issuers, D.u.slots, D.smem);
         else if (D.gather4)
             std::snprintf(buf, sizeof buf, "%s: hybrid (TMA gathers for %d of %d blocks) stage=%d generators, %d slots, "
                           "%zu B shared", dir == 0 ? "d" : "d^T", D.p.t_tma, bt, D.p.gi, D.p.slots, D.smem);

@@ -37,7 +37,10 @@
 // (its operands at 128 bytes a cycle from shared memory), but computing
 // descriptors in the issuing thread cost 135-150 cycles an MMA, and a stage's
 // hand-over between roles costs 200-400 cycles whatever the stage holds.  So
-//   * the MMA warp issues from the table (see its loop);
+//   * the MMA warps issue from the table, and there are two of them where
+//     every tile has two stages: a stage's hand-over (wait, proxy fence, commit)
+//     keeps its warp about as long as its MMAs take, and the tensor pipe's queue
+//     is too short to bridge it (see their loop);
 //   * the producer warps form groups that take the stages in turn, each warp
 //     with more copies a stage and fewer hand-overs;
 //   * every wait is made by all lanes of a warp (one lane and a shuffle took
@@ -46,14 +49,13 @@
 // every stage and stays in registers, so a pass is a shuffle of the run
 // offset, a compare, an add and the two limbs' cp.async.
 //
-// Measured on one B200 (1965 MHz), dense kernels -> this one: r = 19, k = 9,
-// dims 20 -> 28, 16 columns: d 179 -> 130 us, d^T 228 -> 156 us; r = 21, k = 10,
-// dims 32 -> 40, 32 columns: d 1726 -> 1190 us, d^T 2429 -> 1411 us.  With the
-// other roles' work switched off the copies alone take 81 / 86 us at the
-// first size and 688 / 786 at the second, the MMAs 110 / 122 and 699 / 827, the
-// epilogue 99 / 110 and 731 / 863: no role is far above the others, and the
-// second size, whose maps leave three to four slots, loses most to slots that
-// wait for their copies.
+// Measured on one B200 (1965 MHz), us, dense kernels -> one MMA warp -> two:
+// r = 19, k = 9, dims 20 -> 28, 16 columns: d 179 -> 130 -> 92, d^T 228 -> 156 ->
+// 127; r = 21, k = 10, dims 32 -> 40, 32 columns: d 1726 -> 1190 -> 1050, d^T
+// 2429 -> 1411 -> 1260.  With the other roles' work switched off the copies
+// alone take 60 / 76 us at the first size and 614 / 745 at the second, the MMAs
+// 74 / 78 and 555 / 591, the epilogue 73 / 95 and 728 / 859, and the hand-overs
+// without any of them 59 / 60 and 348 / 377: no role is far above the others.
 #pragma once
 
 #include "bw_common.cuh"
@@ -64,11 +66,24 @@ namespace bw {
 
 namespace {
 
+// Warp roles.  8 producer and 8 epilogue warps: every other split measured was
+// slower or within 2 % (d, d^T at (19,9,20,28,16) / (21,10,32,40,32), ms: 8+8
+// 0.092, 0.127 / 1.05, 1.26; 12+8 0.097, 0.129 / 1.04, 1.23; 8+12 0.098, 0.134 /
+// 1.06, 1.27; 8+16 in two teams 0.097, 0.133 / 1.09, 1.30; 4+12 0.124, 0.189 /
+// 1.45, 1.81).
+namespace union_warps {
+constexpr int producers = 8;
+constexpr int mma = 8;                        // two; the first also allocates TMEM
+constexpr int epilogue0 = 10;
+constexpr int epilogue = 8;
+constexpr int threads = (epilogue0 + epilogue) * 32;
+}  // namespace union_warps
+
 constexpr int kUnionPasses = 10;   // 32-unit passes a producer warp makes over a stage, at most
 constexpr int kUnionSteps = 16;    // K-steps of a stage, at most
 constexpr uint32_t kSkip = 0xFFFFFFFEu;      // table word of a generator slot past the tile's union
 constexpr uint32_t kStepValid = 1u << 14;    // step word: this K-step exists (a descriptor's free bits)
-constexpr uint32_t kStepLast = 1u << 15;     // step word 0: last stage of its tile
+constexpr uint32_t kStepLast = 1u << 15;     // step word 0: the issuing warp's last stage of its tile
 
 struct I8Union {
     const int8_t* in[2];           // input +planes lo and hi: [blk][h][inner][16]; the -planes follow them
@@ -85,6 +100,7 @@ struct I8Union {
     int cpg;                       // 16-row chunks of a generator's 2 * inner K' rows
     int gs;                        // generators a stage (even when cpg is odd)
     int row;                       // words of a stage in `steps`: its K-steps rounded up to 4
+    int issuers;                   // MMA warps: 2 where every tile has two stages or more, else 1
     int groups;                    // producer groups: group g fills the stages g, g + groups, ...
     int slots;
     uint32_t b_bytes, slot_bytes;
@@ -127,9 +143,9 @@ __device__ __forceinline__ void pack_limbs(const int32_t (&v)[4], const Mod& mod
     hi = pack_bytes(h[0], h[1], h[2], h[3]) ^ 0x80808080u;
 }
 
-template <int NB, int PW>
-__global__ void __launch_bounds__(GatherWarps<PW>::threads, 1) i8_union_gemm_kernel(I8Union P) {
-    using W = GatherWarps<PW>;
+template <int NB>
+__global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(I8Union P) {
+    namespace W = union_warps;
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int BT = 128 / NB;        // output blocks a tile
     constexpr int HG = NB / 16;         // 16-byte column groups a block row
@@ -157,16 +173,16 @@ __global__ void __launch_bounds__(GatherWarps<PW>::threads, 1) i8_union_gemm_ker
             tc::mbar_init(&empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
-            tc::mbar_init(&accfull[b], 1);
+            tc::mbar_init(&accfull[b], P.issuers);
             tc::mbar_init(&accempty[b], W::epilogue * 32);
         }
-        tc::mbar_init(drained, 1);
+        tc::mbar_init(drained, P.issuers);
         tc::mbar_init(maps_in, 1);
         tc::fence_mbar_init();
         *abort = 0;
     }
     uint32_t tmem_cols = 32;
-    while (tmem_cols < static_cast<uint32_t>(2 * N)) tmem_cols *= 2;
+    while (tmem_cols < static_cast<uint32_t>(2 * N * P.issuers)) tmem_cols *= 2;   // two buffers of an accumulator a warp
     if (warp == W::mma) {
         tc::tmem_alloc(tmem_slot, tmem_cols);
         tc::tmem_relinquish();
@@ -252,78 +268,93 @@ __global__ void __launch_bounds__(GatherWarps<PW>::threads, 1) i8_union_gemm_ker
             }
         }
         tc::cp_async_wait_all();   // no copy may still be landing when the CTA exits
-    } else if (warp == W::mma) {
-        // ------------------------------------------------------------ MMA issuer
-        // The whole warp waits and walks the stages, lane k holding K-step k's
-        // descriptor word (loaded two stages ahead), and one elected lane
-        // issues: an MMA costs a shuffle and no descriptor arithmetic.
-        // the maps, in pieces of at most 32 KB; nothing leaves this block before they have landed
-        if (lane == 0) {
-            tc::mbar_arrive_expect_tx(maps_in, P.b_bytes);
-            for (uint32_t off = 0; off < P.b_bytes; off += 32768u)
-                tc::bulk_g2s(sB + off, P.maps + off, min(32768u, P.b_bytes - off), maps_in);
-        }
-        __syncwarp();
-        const bool ok = tc::warp_wait(tc::smem_u32(maps_in), 0, nullptr, P.err, tc::ERR_WAIT_FINAL);
-        const uint32_t idesc = tc::idesc_i8(128, N, true, false);
-        const uint32_t a_hi = tc::desc_hi(static_cast<uint32_t>(KS) * 16u), b_hi = tc::desc_hi(128u);
-        const uint32_t a_slot0 = tc::desc_lo(tc::smem_u32(sA), 128u), b0 = tc::desc_lo(tc::smem_u32(sB), 0u);
-        const uint32_t slot_units = P.slot_bytes >> 4;
-        const bool has_word = lane < P.row;
-        const uint32_t* tab = P.steps + static_cast<size_t>(stage0) * P.row + lane;
-        uint32_t word0 = has_word && n_stages > 0 ? __ldg(tab) : 0u;
-        uint32_t word1 = has_word && n_stages > 1 ? __ldg(tab + P.row) : 0u;
-        tab += 2 * P.row;
-        uint32_t acc = 0, buf = 0, acc_parity = 1;   // acc = 0: the next stage begins a tile
-        int slot = 0;
-        uint32_t bar = full0, parity = 0, a_lo = a_slot0;
-        // failure tests: CTA 0 waits for its first stage on a barrier that
-        // nothing completes before the final drain, so the wait runs out
-        const bool held = P.hold_first_stage && blockIdx.x == 0 && ok &&
-                          !tc::warp_wait(tc::smem_u32(drained), 0, abort, P.err, tc::ERR_WAIT_FULL, P.wait_limit);
-        for (int left = ok && !held ? n_stages : 0; left > 0; --left) {
-            const uint32_t word = word0;
-            word0 = word1;
-            if (has_word && left > 2) word1 = __ldg(tab);
-            tab += P.row;
-            const int n = __popc(__ballot_sync(0xffffffffu, (word & kStepValid) != 0));
-            const bool last = __any_sync(0xffffffffu, (word & kStepLast) != 0);
-            const uint32_t bw = (word & 0x3FFF3FFFu) + b0;
-            if (acc == 0 && !tc::warp_wait(accempty0 + buf * 8u, acc_parity, abort, P.err, tc::ERR_WAIT_ACCUM_FREE,
-                                           P.wait_limit))
-                break;
-            if (!tc::warp_wait(bar, parity, abort, P.err, tc::ERR_WAIT_FULL, P.wait_limit)) break;
-            tc::fence_proxy_async_smem();
-            tc::tc_fence_after();
-            const uint32_t dcol = tmem + buf * static_cast<uint32_t>(N);
+    } else if (warp < W::epilogue0) {
+        // ------------------------------------------------------------ MMA issuers
+        // A whole warp waits and walks its stages, lane k holding K-step k's
+        // descriptor word (loaded four stages ahead), and one elected lane
+        // issues: an MMA costs a shuffle and no descriptor arithmetic.  The
+        // tensor pipe's queue is short, so while a warp waits for a stage, takes
+        // the proxy fence and commits (about 400 cycles) nothing runs behind the
+        // MMAs that it has issued (6 of 48 cycles a stage at the first size
+        // above): two warps take the stages in turn, each with an accumulator of
+        // its own.
+        const int issuer = warp - W::mma;
+        if (issuer < P.issuers) {
+            // the maps, in pieces of at most 32 KB; nothing leaves this block before they have landed
+            if (issuer == 0 && lane == 0) {
+                tc::mbar_arrive_expect_tx(maps_in, P.b_bytes);
+                for (uint32_t off = 0; off < P.b_bytes; off += 32768u)
+                    tc::bulk_g2s(sB + off, P.maps + off, min(32768u, P.b_bytes - off), maps_in);
+            }
+            __syncwarp();
+            const uint32_t idesc = tc::idesc_i8(128, N, true, false);
+            const uint32_t a_hi = tc::desc_hi(static_cast<uint32_t>(KS) * 16u), b_hi = tc::desc_hi(128u);
+            const uint32_t a_slot0 = tc::desc_lo(tc::smem_u32(sA), 128u), b0 = tc::desc_lo(tc::smem_u32(sB), 0u);
+            const uint32_t slot_units = P.slot_bytes >> 4, step_units = static_cast<uint32_t>(P.issuers) * slot_units;
+            const bool has_word = lane < P.row;
+            const int tab_step = P.issuers * P.row;
+            const uint32_t* tab = P.steps + static_cast<size_t>(stage0 + issuer) * P.row + lane;
+            uint32_t ahead[4];
 #pragma unroll
-            for (int k = 0; k < kUnionSteps; ++k) {
-                if (k >= n) break;
-                const uint32_t b = __shfl_sync(0xffffffffu, bw, k);
-                tc::mma_i8_elect(dcol, tc::desc_make(a_lo + static_cast<uint32_t>(k) * (512u >> 4), a_hi),
-                                 tc::desc_make(b, b_hi), idesc, acc);
-                acc = 1;
+            for (int q = 0; q < 4; ++q)
+                ahead[q] = has_word && issuer + q * P.issuers < n_stages ? __ldg(tab + q * tab_step) : 0u;
+            tab += 4 * tab_step;
+            const uint32_t acc0 = tmem + static_cast<uint32_t>(issuer * N), buf_cols = static_cast<uint32_t>(P.issuers * N);
+            uint32_t acc = 0, buf = 0, acc_parity = 1;   // acc = 0: the next stage is the warp's first of a tile
+            int slot = issuer % P.slots;
+            uint32_t bar = full0 + static_cast<uint32_t>(slot) * 8u, parity = static_cast<uint32_t>(issuer / P.slots) & 1u;
+            uint32_t a_lo = a_slot0 + static_cast<uint32_t>(slot) * slot_units;
+            const bool ok = tc::warp_wait(tc::smem_u32(maps_in), 0, nullptr, P.err, tc::ERR_WAIT_FINAL);
+            // failure tests: CTA 0 waits for its first stage on a barrier that
+            // nothing completes before the final drain, so the wait runs out
+            const bool held = P.hold_first_stage && blockIdx.x == 0 && issuer == 0 && ok &&
+                              !tc::warp_wait(tc::smem_u32(drained), 0, abort, P.err, tc::ERR_WAIT_FULL, P.wait_limit);
+            for (int left = ok && !held ? n_stages - issuer : 0; left > 0; left -= P.issuers) {
+                const uint32_t word = ahead[0];
+#pragma unroll
+                for (int q = 0; q < 3; ++q) ahead[q] = ahead[q + 1];
+                if (has_word && left > 4 * P.issuers) ahead[3] = __ldg(tab);
+                tab += tab_step;
+                const int n = __popc(__ballot_sync(0xffffffffu, (word & kStepValid) != 0));
+                const bool last = __any_sync(0xffffffffu, (word & kStepLast) != 0);
+                const uint32_t bw = (word & 0x3FFF3FFFu) + b0;
+                if (acc == 0 && !tc::warp_wait(accempty0 + buf * 8u, acc_parity, abort, P.err, tc::ERR_WAIT_ACCUM_FREE,
+                                               P.wait_limit))
+                    break;
+                if (!tc::warp_wait(bar, parity, abort, P.err, tc::ERR_WAIT_FULL, P.wait_limit)) break;
+                tc::fence_proxy_async_smem();
+                tc::tc_fence_after();
+                const uint32_t dcol = acc0 + buf * buf_cols;
+#pragma unroll
+                for (int k = 0; k < kUnionSteps; ++k) {
+                    if (k >= n) break;
+                    const uint32_t b = __shfl_sync(0xffffffffu, bw, k);
+                    tc::mma_i8_elect(dcol, tc::desc_make(a_lo + static_cast<uint32_t>(k) * (512u >> 4), a_hi),
+                                     tc::desc_make(b, b_hi), idesc, acc);
+                    acc = 1;
+                }
+                tc::mma_commit_elect(bar + static_cast<uint32_t>(P.slots) * 8u);   // empty[slot]
+                if (last) {
+                    tc::mma_commit_elect(accfull0 + buf * 8u);
+                    acc = 0;
+                    buf ^= 1u;
+                    acc_parity ^= buf == 0 ? 1u : 0u;
+                }
+                slot += P.issuers;
+                bar += static_cast<uint32_t>(P.issuers) * 8u;
+                a_lo += step_units;
+                if (slot >= P.slots) {   // at least two slots
+                    slot -= P.slots;
+                    bar -= static_cast<uint32_t>(P.slots) * 8u;
+                    a_lo -= static_cast<uint32_t>(P.slots) * slot_units;
+                    parity ^= 1u;
+                }
             }
-            tc::mma_commit_elect(bar + static_cast<uint32_t>(P.slots) * 8u);   // empty[slot]
-            if (last) {
-                tc::mma_commit_elect(accfull0 + buf * 8u);
-                acc = 0;
-                buf ^= 1u;
-                acc_parity ^= buf == 0 ? 1u : 0u;
-            }
-            bar += 8u;
-            a_lo += slot_units;
-            if (++slot == P.slots) {
-                slot = 0;
-                bar = full0;
-                a_lo = a_slot0;
-                parity ^= 1u;
-            }
+            // drain: every MMA issued above completes before TMEM is released
+            // (this wait ignores the give-up flag; issued MMAs always finish)
+            tc::mma_commit_elect(tc::smem_u32(drained));
+            tc::warp_wait(tc::smem_u32(drained), 0, nullptr, P.err, tc::ERR_WAIT_FINAL);
         }
-        // drain: every MMA issued above completes before TMEM is released
-        // (this wait ignores the give-up flag; issued MMAs always finish)
-        tc::mma_commit_elect(tc::smem_u32(drained));
-        tc::warp_wait(tc::smem_u32(drained), 0, nullptr, P.err, tc::ERR_WAIT_FINAL);
     } else {
         // ------------------------------------------------------------ epilogue
         // warp & 3 is the TMEM lane quadrant a warp may read; the warps of a
@@ -374,7 +405,7 @@ __global__ void __launch_bounds__(GatherWarps<PW>::threads, 1) i8_union_gemm_ker
             load_diag(dg_next, tile + gridDim.x, part);
             if (!tc::warp_wait(accfull0 + static_cast<uint32_t>(buf) * 8u, aph, abort, P.err, tc::ERR_WAIT_ACCUM, P.wait_limit)) break;
             tc::tc_fence_after();
-            const uint32_t col0 = tmem + lane_off + static_cast<uint32_t>(buf * N);
+            const uint32_t col0 = tmem + lane_off + static_cast<uint32_t>(buf * P.issuers * N);
             const long long base = blk * static_cast<long long>(NB) * P.outer + h_off;
             for (int c = part; c < chunks; c += EPQ) {
                 const int o0 = c * 16;
@@ -390,7 +421,19 @@ __global__ void __launch_bounds__(GatherWarps<PW>::threads, 1) i8_union_gemm_ker
                     const uint32_t cb = col0 + static_cast<uint32_t>(o0 + h8 * 8);
                     tc::tmem_ld8(cb, lo);
                     tc::tmem_ld8(cb + P.ho, hi);
-                    tc::tmem_ld_wait();
+                    if (P.issuers == 2) {   // the second warp's sums
+                        int32_t lo2[8], hi2[8];
+                        tc::tmem_ld8(cb + N, lo2);
+                        tc::tmem_ld8(cb + N + P.ho, hi2);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            lo[q] += lo2[q];
+                            hi[q] += hi2[q];
+                        }
+                    } else {
+                        tc::tmem_ld_wait();
+                    }
 #pragma unroll
                     for (int g4 = 0; g4 < 2; ++g4) {
                         if (h8 * 8 + g4 * 4 >= live) break;
@@ -437,7 +480,7 @@ __global__ void __launch_bounds__(GatherWarps<PW>::threads, 1) i8_union_gemm_ker
 __global__ void union_tables_kernel(const uint32_t* __restrict__ inc, const uint32_t* __restrict__ mask,
                                     const uint32_t* __restrict__ tile_stage, uint32_t* __restrict__ words,
                                     uint32_t* __restrict__ steps, long long n_tiles, long long n_blk, int r, int bt,
-                                    int gs, int cpg, int n_cols, int row, uint32_t run16, uint32_t neg16) {
+                                    int gs, int cpg, int n_cols, int row, int issuers, uint32_t run16, uint32_t neg16) {
     const long long tile = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (tile >= n_tiles) return;
     const uint32_t all = mask[tile];
@@ -471,7 +514,7 @@ __global__ void union_tables_kernel(const uint32_t* __restrict__ inc, const uint
                 if ((c & 1) || c == chunks - 1) {
                     if (!(c & 1)) at[1] = static_cast<uint32_t>(r * cpg) * n_cols;
                     out[c >> 1] = at[0] | ((at[1] - at[0]) << 16) | kStepValid |
-                                  (c <= 1 && s == stages - 1 ? kStepLast : 0u);
+                                  (c <= 1 && s + issuers >= stages ? kStepLast : 0u);
                 }
             }
         for (int k = (chunks + 1) / 2; k < row; ++k) out[k] = 0;
