@@ -870,8 +870,14 @@ __global__ void __launch_bounds__(256) from_limbs_kernel(const int8_t* __restric
 // int32 accumulation is exact for at most 2^31 / 127^2 > 131072 rows, so the
 // accumulator is drained (double-buffered) every `drain` stages.
 //
-// Warps: 0 producer (bulk copies: the stage's X tile and W block runs), 1 MMA
-// issuer (allocates TMEM), 2-5 epilogue (tcgen05.ld + reduction mod p).  The
+// Warps: 0 producer (the stage's X tile and W runs), 1 MMA issuer (allocates
+// TMEM), 2-5 epilogue (tcgen05.ld + reduction mod p).  The W runs of 16-column
+// blocks are back to back in a plane and take one bulk copy a limb.  Those of
+// 32-column blocks alternate between the two column groups: a box of a 3-D
+// tensor map (run, group, block) collects a group's runs of the whole stage.
+// (One bulk copy a run, 32 a stage, held the copies at half the rate: 427 us at
+// r = 21, k = 10, dim 32, 32 columns, 409 with warp-uniform MMA issue, 221 with
+// the boxes.)  The
 // CTA's combined sums are added into an m x n int32 accumulator; the last CTA
 // to finish writes them to the session's buffer, clears them and advances the
 // index.
@@ -895,7 +901,8 @@ struct I8Proj {
 };
 
 template <int NB>
-__global__ void __launch_bounds__(kProjThreads, 1) i8_project_tc_kernel(I8Proj P) {
+__global__ void __launch_bounds__(kProjThreads, 1)
+    i8_project_tc_kernel(const __grid_constant__ CUtensorMap w_lo, const __grid_constant__ CUtensorMap w_hi, I8Proj P) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int HG = NB / 16;
     constexpr int N = 2 * NB;
@@ -909,7 +916,7 @@ __global__ void __launch_bounds__(kProjThreads, 1) i8_project_tc_kernel(I8Proj P
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
     __shared__ bool am_last;
 
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0), lane = threadIdx.x % 32;
     const long long n_my = blockIdx.x < P.n_stages ? (P.n_stages - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const long long n_chunks = (n_my + P.drain - 1) / P.drain;
     const uint32_t tmem_cols = 2 * N;   // two accumulators (64 or 128 columns)
@@ -946,7 +953,8 @@ __global__ void __launch_bounds__(kProjThreads, 1) i8_project_tc_kernel(I8Proj P
             const uint32_t ph = ring.phase;
             const long long st = blockIdx.x + i * gridDim.x;
             const long long blk0 = st * P.sb;
-            const int nbh = static_cast<int>(min(static_cast<long long>(P.sb), P.n_blk - blk0));
+            // a box is copied whole (past the last block: zeros)
+            const int nbh = HG == 1 ? static_cast<int>(min(static_cast<long long>(P.sb), P.n_blk - blk0)) : P.sb;
             int got = 1;
             if (lane == 0) {
                 got = tc::mbar_wait(&empty[slot], ph ^ 1u, abort, P.err, tc::ERR_WAIT_EMPTY, P.wait_limit) ? 1 : 0;
@@ -964,53 +972,58 @@ __global__ void __launch_bounds__(kProjThreads, 1) i8_project_tc_kernel(I8Proj P
                 if (lane < 2)
                     tc::bulk_g2s(sB + lane * group_bytes, P.w[lane] + blk0 * run_bytes, nbh * run_bytes, &full[slot]);
             } else {
-                for (int q = lane; q < nbh * 2 * HG; q += 32) {
-                    const int b = q / (2 * HG), limb = (q / HG) % 2, h = q % HG;
-                    tc::bulk_g2s(sB + (limb * HG + h) * group_bytes + b * run_bytes,
-                                 P.w[limb] + ((blk0 + b) * HG + h) * static_cast<long long>(run_bytes), run_bytes,
-                                 &full[slot]);
-                }
+                if (lane < 2 * HG)
+                    tc::tma_load3(sB + lane * group_bytes, lane < HG ? &w_lo : &w_hi, 0, lane % HG,
+                                  static_cast<int32_t>(blk0), &full[slot]);
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc = tc::idesc_i8(128, N, true, true);
-            const uint32_t s0 = tc::smem_u32(smem);
-            const uint32_t gb = static_cast<uint32_t>(P.kp) * 16;
-            const int ksteps = P.kp / 32;
-            long long i = 0;
-            SlotRing ring(P.slots);
-            bool ok = true;
-            for (long long c = 0; c < n_chunks && ok; ++c) {
-                const int buf = static_cast<int>(c & 1);
-                const uint32_t aph = static_cast<uint32_t>((c >> 1) & 1);
-                if (!tc::mbar_wait(&accempty[buf], aph ^ 1u, abort, P.err, tc::ERR_WAIT_ACCUM_FREE, P.wait_limit)) break;
-                tc::tc_fence_after();
-                const uint32_t dcol = tmem + static_cast<uint32_t>(buf * N);
-                const long long i_end = min(n_my, (c + 1) * P.drain);
-                for (bool first = true; i < i_end; ++i, first = false, ring.next()) {
-                    const int slot = ring.slot;
-                    const uint32_t ph = ring.phase;
-                    if (!tc::mbar_wait(&full[slot], ph, abort, P.err, tc::ERR_WAIT_FULL, P.wait_limit)) {
-                        ok = false;
-                        break;
-                    }
-                    tc::tc_fence_after();
-                    const uint32_t a0 = s0 + static_cast<uint32_t>(slot) * P.slot_bytes;
-                    const uint32_t b0 = a0 + P.a_bytes;
-                    for (int ks = 0; ks < ksteps; ++ks)
-                        tc::mma_i8(dcol, tc::smem_desc(a0 + ks * 512u, 128u, gb), tc::smem_desc(b0 + ks * 512u, 128u, gb),
-                                   idesc, (!first || ks > 0) ? 1u : 0u);
-                    tc::mma_commit(&empty[slot]);
-                }
-                if (!ok) break;
-                tc::mma_commit(&accfull[buf]);
+        // A whole warp waits and walks the stages and one elected lane issues, so
+        // that descriptors are warp-uniform (issued by lane 0 in a branch of its
+        // own, each MMA took 140 cycles instead of its 40 to 48).
+        const uint32_t idesc = tc::idesc_i8(128, N, true, true);
+        const uint32_t gb = static_cast<uint32_t>(P.kp) * 16, d_hi = tc::desc_hi(gb);
+        const uint32_t a_first = tc::desc_lo(tc::smem_u32(smem), 128u), slot_units = P.slot_bytes >> 4;
+        const uint32_t b_off = P.a_bytes >> 4;
+        const uint32_t full0 = tc::smem_u32(full), empty0 = tc::smem_u32(empty);
+        const uint32_t accfull0 = tc::smem_u32(accfull), accempty0 = tc::smem_u32(accempty);
+        const int ksteps = P.kp / 32;
+        int slot = 0, left = 0;          // stages left of the accumulator's share
+        uint32_t parity = 0, buf = 0, acc_parity = 1, acc = 0;
+        for (int todo = static_cast<int>(n_my); todo > 0; --todo) {
+            if (left == 0) {
+                if (!tc::warp_wait(accempty0 + buf * 8u, acc_parity, abort, P.err, tc::ERR_WAIT_ACCUM_FREE, P.wait_limit))
+                    break;
+                left = min(todo, P.drain);
+                acc = 0;
             }
-            tc::mma_commit(drained);
-            tc::mbar_wait(drained, 0, nullptr, P.err, tc::ERR_WAIT_FINAL);
+            if (!tc::warp_wait(full0 + static_cast<uint32_t>(slot) * 8u, parity, abort, P.err, tc::ERR_WAIT_FULL,
+                               P.wait_limit))
+                break;
+            tc::tc_fence_after();
+            const uint32_t a_lo = a_first + static_cast<uint32_t>(slot) * slot_units;
+            const uint32_t dcol = tmem + buf * N;
+#pragma unroll 4
+            for (int ks = 0; ks < ksteps; ++ks) {
+                const uint32_t a = a_lo + static_cast<uint32_t>(ks) * 32u;
+                tc::mma_i8_elect(dcol, tc::desc_make(a, d_hi), tc::desc_make(a + b_off, d_hi), idesc, acc);
+                acc = 1;
+            }
+            tc::mma_commit_elect(empty0 + static_cast<uint32_t>(slot) * 8u);
+            if (--left == 0) {
+                tc::mma_commit_elect(accfull0 + buf * 8u);
+                buf ^= 1u;
+                acc_parity ^= buf == 0 ? 1u : 0u;
+            }
+            if (++slot == P.slots) {
+                slot = 0;
+                parity ^= 1u;
+            }
         }
-        __syncwarp();
+        // drain: every MMA issued above completes before TMEM is released
+        tc::mma_commit_elect(tc::smem_u32(drained));
+        tc::warp_wait(tc::smem_u32(drained), 0, nullptr, P.err, tc::ERR_WAIT_FINAL);
     } else {
         // ------------------------------------------------------------ epilogue
         const int q = warp & 3;                  // TMEM lane quadrant of this warp
@@ -1142,6 +1155,7 @@ struct KoszulCtx::I8State {
     // Y_a, Y_b, Z: lo, hi, -lo, -hi; each -plane directly follows its +plane in
     // memory, so that one tensor map covers both signs of a limb
     int8_t* planes[3][4] = {};
+    CUtensorMap runs[2][2] = {};       // Y_a, Y_b: [limb], the projection's boxes of 32-column blocks
     CUtensorMap maps[3][2];        // [block array][limb]: rows = (sign, block, h) runs
     std::string plan_text;         // the chosen stage plans and the autotuner's timings
     I8Proj proj{};             // projection plan (X tiles, stage shape, grid)
@@ -1476,10 +1490,7 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// One limb of a block array as a 2-D tensor for the gathers: rows = the
-// (sign, block, h) runs of dim * 16 bytes (the -plane's rows after the
-// +plane's), 8-byte elements; box = one run of dim_pad * 16 bytes.
-void encode_plane_map(CUtensorMap* map, const int8_t* base, uint64_t n_blk, int dim, int dim_pad, int hg) {
+EncodeTiledFn tensor_map_encoder() {
     static const EncodeTiledFn encode = [] {
         void* f = nullptr;
         cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
@@ -1490,14 +1501,37 @@ void encode_plane_map(CUtensorMap* map, const int8_t* base, uint64_t n_blk, int 
         return reinterpret_cast<EncodeTiledFn>(f);
     }();
     BW_REQUIRE(encode != nullptr, "INT8 form: cuTensorMapEncodeTiled is not available from the driver");
+    return encode;
+}
+
+// One limb of a block array as a 2-D tensor for the gathers: rows = the
+// (sign, block, h) runs of dim * 16 bytes (the -plane's rows after the
+// +plane's), 8-byte elements; box = one run of dim_pad * 16 bytes.
+void encode_plane_map(CUtensorMap* map, const int8_t* base, uint64_t n_blk, int dim, int dim_pad, int hg) {
     BW_REQUIRE(reinterpret_cast<uintptr_t>(base) % 16 == 0, "INT8 form: plane not 16-byte aligned");
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(2 * dim), static_cast<cuuint64_t>(2 * n_blk * hg)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(dim) * 16};
     const cuuint32_t box[2] = {static_cast<cuuint32_t>(2 * dim_pad), 1};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult rc = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<int8_t*>(base), dims, strides, box,
-                               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult rc = tensor_map_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<int8_t*>(base), dims,
+                                             strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    BW_REQUIRE(rc == CUDA_SUCCESS, "INT8 form: cuTensorMapEncodeTiled failed (code " + std::to_string(rc) + ")");
+}
+
+// One limb of a source block array as a 3-D tensor for the projection: (bytes of
+// a run, column group, block), 8-byte elements; box = one group's runs of sb
+// blocks (sb and 2 * dim are at most 256).
+void encode_run_map(CUtensorMap* map, const int8_t* base, uint64_t n_blk, int dim, int hg, int sb) {
+    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(2 * dim), static_cast<cuuint64_t>(hg), n_blk};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(dim) * 16, static_cast<cuuint64_t>(dim) * 16 * hg};
+    const cuuint32_t box[3] = {static_cast<cuuint32_t>(2 * dim), 1, static_cast<cuuint32_t>(sb)};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult rc = tensor_map_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<int8_t*>(base), dims,
+                                             strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     BW_REQUIRE(rc == CUDA_SUCCESS, "INT8 form: cuTensorMapEncodeTiled failed (code " + std::to_string(rc) + ")");
 }
 
@@ -1515,7 +1549,8 @@ void plan_projection(KoszulCtx& c, KoszulCtx::I8State& S) {
     const int row_bytes = (2 * P.mg + 2 * (c.nbi / 16)) * 16;
     int best_sb = 1;
     double best_fill = 0;
-    for (int sb = 1; sb <= 4096; ++sb) {
+    const int max_sb = c.nbi == 16 ? 4096 : 256;   // a box has at most 256 blocks
+    for (int sb = 1; sb <= max_sb; ++sb) {
         const int kp = (sb * P.dim + 31) / 32 * 32;
         if (sb > 1 && kp * row_bytes > kProjStageTarget) break;
         const double fill = static_cast<double>(sb * P.dim) / kp;
@@ -1715,6 +1750,8 @@ void KoszulCtx::i8_setup() {
         const int dim = b < 2 ? ci : co;
         for (int limb = 0; limb < 2; ++limb)
             encode_plane_map(&S.maps[b][limb], S.planes[b][limb], n_blk, dim, dim + (dim & 1), hg);
+        for (int limb = 0; limb < 2 && b < 2 && hg > 1; ++limb)
+            encode_run_map(&S.runs[b][limb], S.planes[b][limb], n_blk, dim, hg, S.proj.sb);
     }
     // Failure tests only (the environment of the creating process): a short
     // limit on every pipeline wait, and a first stage that CTA 0 of the d/d^T
@@ -1960,7 +1997,8 @@ void KoszulCtx::i8_project(int buf, cudaStream_t st) {
     P.counter = d_counter;
     P.state = d_seq_state;
     dispatch_i8_nb(nbi, [&](auto NBc) {
-        launch_dependent(i8_project_tc_kernel<decltype(NBc)::value>, i8->proj_grid, kProjThreads, i8->proj_smem, st, P);
+        launch_dependent(i8_project_tc_kernel<decltype(NBc)::value>, i8->proj_grid, kProjThreads, i8->proj_smem, st,
+                         i8->runs[buf][0], i8->runs[buf][1], P);
     });
     BW_CHECK_LAUNCH();
     ++launches;

@@ -110,6 +110,17 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                  : "memory");
 }
 
+// TMA load of a box of a 3-D tensor map (this GPU's memory, no multicast) to
+// shared memory (128-byte aligned), completing on `bar` with the bytes of the
+// whole box; what lies outside the tensor is filled with zeros.
+__device__ __forceinline__ void tma_load3(void* dst, const void* tmap, int32_t x, int32_t y, int32_t z, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        : "memory");
+}
+
 // TMA gather of four rows of a 2-D tensor map (sm_100 tile::gather4): rows
 // y0..y3 (any order; a row outside the tensor is filled with zeros and read
 // from nowhere), columns from x for the map's box width, written back to back
