@@ -415,9 +415,9 @@ void KoszulCtx::project(const int32_t* w, cudaStream_t st) {
 }
 
 // One step: cur -> other, append a_i.
-void KoszulCtx::step_once(cudaStream_t st) {
+void KoszulCtx::step_once(cudaStream_t st, bool after_step) {
     if (form == BW_FORM_INT8) {
-        i8_step_once(st);
+        i8_step_once(st, after_step);
         return;
     }
     int32_t* src = cur_is_a ? d_ya : d_yb;
@@ -719,7 +719,7 @@ void KoszulCtx::seq_step(uint64_t steps, cudaStream_t st) {
             const uint64_t launches0 = launches;   // captured launches do not execute
             BW_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
             try {
-                for (int s = 0; s < 2 * kGraphPairs; ++s) step_once(st);
+                for (int s = 0; s < 2 * kGraphPairs; ++s) step_once(st, s > 0);
             } catch (...) {
                 cudaStreamEndCapture(st, &graph);
                 throw;
@@ -736,10 +736,9 @@ void KoszulCtx::seq_step(uint64_t steps, cudaStream_t st) {
         seq_len += 2 * kGraphPairs;
         steps -= 2 * kGraphPairs;
     }
-    while (steps > 0) {
-        step_once(st);
+    for (bool after_step = false; steps > 0; after_step = true, --steps) {
+        step_once(st, after_step);
         ++seq_len;
-        --steps;
     }
 }
 

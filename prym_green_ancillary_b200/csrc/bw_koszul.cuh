@@ -81,7 +81,8 @@ struct KoszulCtx {
     void plain_forward(const int32_t* y, int32_t* z, cudaStream_t st);
     void plain_transpose(const int32_t* z, int32_t* w, bool scale, cudaStream_t st);
     void project(const int32_t* w, cudaStream_t st);
-    void step_once(cudaStream_t st);
+    // after_step: the kernel launched before on st is the last of this state's previous step
+    void step_once(cudaStream_t st, bool after_step = false);
 
     void seq_start(const uint32_t* x, const uint32_t* y0, uint32_t* seq, uint64_t capacity, cudaStream_t st);
     void seq_step(uint64_t steps, cudaStream_t st);
@@ -98,7 +99,7 @@ struct KoszulCtx {
     void i8_destroy();
     uint64_t i8_kernels_per_step() const;
     enum { I8_YA = 0, I8_YB = 1, I8_Z = 2 };   // limb-plane block arrays
-    void i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cudaStream_t st);
+    void i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cudaStream_t st, bool after_projection = false);
     void i8_check_error();
     double i8_time_direction(bool forward_dir, int in_buf, int out_buf);
     const std::string& i8_plan_text() const;
@@ -106,7 +107,7 @@ struct KoszulCtx {
     void i8_from_limbs(int buf, uint32_t* out, cudaStream_t st);
     void i8_load_x(const uint32_t* x, cudaStream_t st);
     void i8_project(int buf, cudaStream_t st);
-    void i8_step_once(cudaStream_t st);
+    void i8_step_once(cudaStream_t st, bool after_step);
     int i8_dim(int buf) const;
     uint64_t i8_rows(int buf) const;
 };

@@ -64,7 +64,7 @@ struct KoszulBatch {
                 BW_CUDA(cudaEventRecord(fork, st));
                 for (size_t i = 0; i < sectors.size(); ++i) {
                     BW_CUDA(cudaStreamWaitEvent(lanes[i], fork, 0));
-                    for (int k = 0; k < kGraphSteps; ++k) sectors[i]->step_once(lanes[i]);
+                    for (int k = 0; k < kGraphSteps; ++k) sectors[i]->step_once(lanes[i], k > 0);
                     BW_CUDA(cudaEventRecord(joins[i], lanes[i]));
                     BW_CUDA(cudaStreamWaitEvent(st, joins[i], 0));
                 }

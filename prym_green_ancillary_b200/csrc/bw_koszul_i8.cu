@@ -920,7 +920,6 @@ __global__ void __launch_bounds__(kProjThreads, 1)
     const long long n_my = blockIdx.x < P.n_stages ? (P.n_stages - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const long long n_chunks = (n_my + P.drain - 1) / P.drain;
     const uint32_t tmem_cols = 2 * N;   // two accumulators (64 or 128 columns)
-    pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.slots; ++s) {
             tc::mbar_init(&full[s], 1);
@@ -943,7 +942,10 @@ __global__ void __launch_bounds__(kProjThreads, 1)
     tc::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t run_bytes = static_cast<uint32_t>(P.dim) * 16;   // one (block, h) run of a plane
+    // In this order: when the next kernel begins, W is complete (see
+    // i8_step_once: the next step's d does not wait for this kernel).
     pdl_wait();
+    pdl_trigger();
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
@@ -1589,8 +1591,10 @@ void plan_projection(KoszulCtx& c, KoszulCtx::I8State& S) {
 }
 
 template <int NB>
-void launch_i8(KoszulCtx& c, KoszulCtx::I8State::Dir& D, const CUtensorMap* maps, cudaStream_t st) {
+void launch_i8(KoszulCtx& c, KoszulCtx::I8State::Dir& D, const CUtensorMap* maps, bool after_projection,
+               cudaStream_t st) {
     if (D.use_union) {
+        D.u.late_wait = after_projection ? 1 : 0;
         BW_REQUIRE(D.u.start != nullptr && D.u.words != nullptr && D.u.steps != nullptr && D.u.maps != nullptr,
                    "internal: INT8 stage list missing for the union kernel");
         launch_dependent(i8_union_gemm_kernel<NB>, D.grid, union_warps::threads, D.smem, st, D.u);
@@ -1919,7 +1923,7 @@ double KoszulCtx::i8_time_direction(bool forward_dir, int in_buf, int out_buf) {
 
 uint64_t KoszulCtx::i8_kernels_per_step() const { return 3; }
 
-void KoszulCtx::i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cudaStream_t st) {
+void KoszulCtx::i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cudaStream_t st, bool after_projection) {
     I8State::Dir& D = forward_dir ? i8->fwd : i8->bwd;
     if (D.use_union) {
         D.u.in[0] = i8->planes[in_buf][PL_LO];
@@ -1934,7 +1938,7 @@ void KoszulCtx::i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cu
     }
     D.p.in_neg_off = i8->planes[in_buf][PL_NLO] - i8->planes[in_buf][PL_LO];
     D.p.diag = (!forward_dir && scale) ? d_diag : nullptr;
-    dispatch_i8_nb(nbi, [&](auto NBc) { launch_i8<decltype(NBc)::value>(*this, D, i8->maps[in_buf], st); });
+    dispatch_i8_nb(nbi, [&](auto NBc) { launch_i8<decltype(NBc)::value>(*this, D, i8->maps[in_buf], after_projection, st); });
 }
 
 void KoszulCtx::i8_check_error() {
@@ -2005,9 +2009,19 @@ void KoszulCtx::i8_project(int buf, cudaStream_t st) {
 }
 
 // One INT8 step on the limb state: cur -> other, append a_i.
-void KoszulCtx::i8_step_once(cudaStream_t st) {
+//
+// d reads what the step before it wrote in d^T and writes Z, which that d^T
+// has read: it has nothing to do with the projection between them.  Where the
+// kernel launched before it on `st` is this state's projection, d therefore
+// runs without waiting for that kernel (it begins once every CTA of the
+// projection has seen d^T complete, and waits for it before it ends, so that a
+// completed kernel still implies all earlier ones).  A step takes, us, waiting
+// at the start / at the end: r = 10, k = 4, 16 -> 24, 8 columns 14.9 / 12.0;
+// r = 19, k = 9, 20 -> 28, 16 columns 236 / 235; r = 21, k = 10, 32 -> 40, 32
+// columns 3050 / 2930; r = 23, k = 11, 32 -> 40, 32 columns 13350 / 12900.
+void KoszulCtx::i8_step_once(cudaStream_t st, bool after_step) {
     const int src = cur_is_a ? I8_YA : I8_YB, dst = cur_is_a ? I8_YB : I8_YA;
-    i8_run(true, src, I8_Z, false, st);
+    i8_run(true, src, I8_Z, false, st, after_step);
     i8_run(false, I8_Z, dst, true, st);
     i8_project(dst, st);
     cur_is_a = !cur_is_a;

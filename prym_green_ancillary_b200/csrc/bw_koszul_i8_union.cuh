@@ -107,6 +107,7 @@ struct I8Union {
     int wide;                      // the epilogue reduces hi on its own (see plan_union)
     Mod mod;
     uint32_t wait_limit;           // tries of every pipeline wait (tc::kWaitLimit outside the failure tests)
+    int late_wait;                 // nothing here depends on the kernel before: wait for it at the end only
     int hold_first_stage;          // failure tests only: CTA 0's MMA warp never sees its first stage
 };
 
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
         uint32_t word0 = has_word && group < n_stages ? __ldg(tab) : kSkip;
         uint32_t word1 = has_word && group + P.groups < n_stages ? __ldg(tab + tab_step) : kSkip;
         tab += 2 * tab_step;
-        pdl_wait();   // the input planes; the maps and lists are constant
+        if (!P.late_wait) pdl_wait();   // the input planes; the maps and lists are constant
         for (int left = n_stages - group; left > 0; left -= P.groups) {
             const uint32_t word = word0;
             word0 = word1;
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
                 for (int oo = 0; oo < 16; ++oo) dg[oo] = any && c * 16 + oo < P.outer ? __ldg(src + oo) : 0;
             }
         };
-        pdl_wait();   // the output planes may still be read, and the diagonal be written, by earlier kernels
+        if (!P.late_wait) pdl_wait();   // the output planes may still be read by earlier kernels
         // a tile's first chunk is loaded one tile ahead (the diagonal streams from DRAM)
         int32_t dg_next[16];
         load_diag(dg_next, blockIdx.x, part);
@@ -472,6 +473,7 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
         tc::tc_fence_after();
         tc::tmem_dealloc(tmem, tmem_cols);
     }
+    if (P.late_wait) pdl_wait();   // this kernel's completion implies that of all kernels before it
 }
 
 // The union kernel's stage list (see I8Union): tile t's stages start at
