@@ -824,8 +824,7 @@ extern "C" int bw_koszul_forward(bw_koszul* ctx, const uint32_t* d_y, uint32_t* 
         cudaStream_t st = scope.st;
         if (c.form == BW_FORM_INT8) {
             c.i8_to_limbs(d_y, KoszulCtx::I8_YA, st);
-            c.i8_run(true, KoszulCtx::I8_YA, KoszulCtx::I8_Z, false, st);
-            c.i8_from_limbs(KoszulCtx::I8_Z, d_z, st);
+            c.i8_run_to(true, KoszulCtx::I8_YA, KoszulCtx::I8_Z, false, d_z, st);
             BW_CUDA(cudaStreamSynchronize(st));
             c.i8_check_error();
             return;
@@ -847,8 +846,7 @@ extern "C" int bw_koszul_transpose(bw_koszul* ctx, const uint32_t* d_z, uint32_t
         cudaStream_t st = scope.st;
         if (c.form == BW_FORM_INT8) {
             c.i8_to_limbs(d_z, KoszulCtx::I8_Z, st);
-            c.i8_run(false, KoszulCtx::I8_Z, KoszulCtx::I8_YA, scale_by_diag != 0, st);
-            c.i8_from_limbs(KoszulCtx::I8_YA, d_w, st);
+            c.i8_run_to(false, KoszulCtx::I8_Z, KoszulCtx::I8_YA, scale_by_diag != 0, d_w, st);
             BW_CUDA(cudaStreamSynchronize(st));
             c.i8_check_error();
             return;
@@ -870,8 +868,7 @@ extern "C" int bw_koszul_apply(bw_koszul* ctx, const uint32_t* d_y, uint32_t* d_
         if (c.form == BW_FORM_INT8) {
             c.i8_to_limbs(d_y, KoszulCtx::I8_YA, st);
             c.i8_run(true, KoszulCtx::I8_YA, KoszulCtx::I8_Z, false, st);
-            c.i8_run(false, KoszulCtx::I8_Z, KoszulCtx::I8_YB, true, st);
-            c.i8_from_limbs(KoszulCtx::I8_YB, d_out, st);
+            c.i8_run_to(false, KoszulCtx::I8_Z, KoszulCtx::I8_YB, true, d_out, st);
             BW_CUDA(cudaStreamSynchronize(st));
             c.i8_check_error();
             return;

@@ -99,7 +99,9 @@ struct KoszulCtx {
     void i8_destroy();
     uint64_t i8_kernels_per_step() const;
     enum { I8_YA = 0, I8_YB = 1, I8_Z = 2 };   // limb-plane block arrays
-    void i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cudaStream_t st, bool after_projection = false);
+    void i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cudaStream_t st, bool after_projection = false,
+                uint32_t* canon = nullptr);
+    void i8_run_to(bool forward_dir, int in_buf, int out_buf, bool scale, uint32_t* out, cudaStream_t st);
     void i8_check_error();
     double i8_time_direction(bool forward_dir, int in_buf, int out_buf);
     const std::string& i8_plan_text() const;

@@ -1597,7 +1597,8 @@ void launch_i8(KoszulCtx& c, KoszulCtx::I8State::Dir& D, const CUtensorMap* maps
         D.u.late_wait = after_projection ? 1 : 0;
         BW_REQUIRE(D.u.start != nullptr && D.u.words != nullptr && D.u.steps != nullptr && D.u.maps != nullptr,
                    "internal: INT8 stage list missing for the union kernel");
-        launch_dependent(i8_union_gemm_kernel<NB>, D.grid, union_warps::threads, D.smem, st, D.u);
+        launch_dependent(D.u.canon ? i8_union_gemm_kernel<NB, true> : i8_union_gemm_kernel<NB, false>, D.grid,
+                         union_warps::threads, D.smem, st, D.u);
         BW_CHECK_LAUNCH();
         ++c.launches;
         return;
@@ -1774,7 +1775,8 @@ void KoszulCtx::i8_setup() {
     dispatch_i8_nb(nbi, [&](auto NBc) {
         cap_g = std::min(allow_dynamic_smem(i8_gather_gemm_kernel<decltype(NBc)::value, 8>, device),
                          allow_dynamic_smem(i8_gather_gemm_kernel<decltype(NBc)::value, 16>, device));
-        cap_u = allow_dynamic_smem(i8_union_gemm_kernel<decltype(NBc)::value>, device);
+        cap_u = std::min(allow_dynamic_smem(i8_union_gemm_kernel<decltype(NBc)::value, false>, device),
+                         allow_dynamic_smem(i8_union_gemm_kernel<decltype(NBc)::value, true>, device));
         cap_4 = allow_dynamic_smem(i8_gather_hybrid_kernel<decltype(NBc)::value>, device);
         const int cap_p = allow_dynamic_smem(i8_project_tc_kernel<decltype(NBc)::value>, device);
         BW_REQUIRE(static_cast<int>(S.proj_smem) <= cap_p, "INT8 form: shared-memory plan above the device limit");
@@ -1923,7 +1925,8 @@ double KoszulCtx::i8_time_direction(bool forward_dir, int in_buf, int out_buf) {
 
 uint64_t KoszulCtx::i8_kernels_per_step() const { return 3; }
 
-void KoszulCtx::i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cudaStream_t st, bool after_projection) {
+void KoszulCtx::i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cudaStream_t st, bool after_projection,
+                       uint32_t* canon) {
     I8State::Dir& D = forward_dir ? i8->fwd : i8->bwd;
     if (D.use_union) {
         D.u.in[0] = i8->planes[in_buf][PL_LO];
@@ -1931,6 +1934,8 @@ void KoszulCtx::i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cu
         for (int pl = 0; pl < 4; ++pl) D.u.out[pl] = i8->planes[out_buf][pl];
         D.u.n_blk = D.p.n_blk;
         D.u.diag = (!forward_dir && scale) ? d_diag : nullptr;
+        D.u.canon = canon;
+        D.u.width = nb;
     }
     for (int pl = 0; pl < 4; ++pl) {
         D.p.in[pl] = i8->planes[in_buf][pl];
@@ -1939,6 +1944,15 @@ void KoszulCtx::i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cu
     D.p.in_neg_off = i8->planes[in_buf][PL_NLO] - i8->planes[in_buf][PL_LO];
     D.p.diag = (!forward_dir && scale) ? d_diag : nullptr;
     dispatch_i8_nb(nbi, [&](auto NBc) { launch_i8<decltype(NBc)::value>(*this, D, i8->maps[in_buf], after_projection, st); });
+}
+
+// d or d^T with its result as canonical residues in the caller's buffer.  The
+// union kernel's epilogue writes them (limb planes and a conversion kernel after
+// it: forward at r = 19, k = 9, 20 -> 28, 16 columns 197 us, now 169).
+void KoszulCtx::i8_run_to(bool forward_dir, int in_buf, int out_buf, bool scale, uint32_t* out, cudaStream_t st) {
+    const bool direct = (forward_dir ? i8->fwd : i8->bwd).use_union;
+    i8_run(forward_dir, in_buf, out_buf, scale, st, false, direct ? out : nullptr);
+    if (!direct) i8_from_limbs(out_buf, out, st);
 }
 
 void KoszulCtx::i8_check_error() {

@@ -88,6 +88,8 @@ constexpr uint32_t kStepLast = 1u << 15;     // step word 0: the issuing warp's 
 struct I8Union {
     const int8_t* in[2];           // input +planes lo and hi: [blk][h][inner][16]; the -planes follow them
     int8_t* out[4];                // output planes lo, hi, -lo, -hi
+    uint32_t* canon;               // CANON: the output as canonical residues, [n_blk * outer][width]
+    int width;                     // columns of the caller's block (the rest of NB are zero padding)
     const uint32_t* start;         // [grid + 1]: first stage of every CTA's list
     const uint32_t* words;         // [stage][gs * BT]: the neighbour run's 16-byte offset from the +plane,
                                    // kAbsent (rows of zeros) or kSkip (no rows)
@@ -144,7 +146,9 @@ __device__ __forceinline__ void pack_limbs(const int32_t (&v)[4], const Mod& mod
     hi = pack_bytes(h[0], h[1], h[2], h[3]) ^ 0x80808080u;
 }
 
-template <int NB>
+// CANON: the output goes to P.canon as canonical residues, else to the planes.
+// (As a branch inside the plane form it cost a step 10 % at r = 19.)
+template <int NB, bool CANON>
 __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(I8Union P) {
     namespace W = union_warps;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -445,9 +449,21 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
                             v[oi] = P.wide ? union_value<true>(lo[o], hi[o], P.mod, scale, dg[h8 * 8 + o])
                                            : union_value<false>(lo[o], hi[o], P.mod, scale, dg[h8 * 8 + o]);
                         }
-                        pack_limbs(v, P.mod, lw[h8 * 2 + g4], hw[h8 * 2 + g4]);
+                        if constexpr (CANON) {   // a row's columns are neighbouring lanes: whole sectors
+                            const int o = o0 + h8 * 8 + g4 * 4;
+                            uint32_t* at = P.canon + (blk * P.outer + o) * P.width + j;
+                            if (valid && j < P.width)
+#pragma unroll
+                                for (int oi = 0; oi < 4; ++oi)
+                                    if (o + oi < P.outer)
+                                        at[oi * P.width] =
+                                            to_canonical(reduce_balanced_fast(v[oi] - P.mod.half, P.mod), P.mod);
+                        } else {
+                            pack_limbs(v, P.mod, lw[h8 * 2 + g4], hw[h8 * 2 + g4]);
+                        }
                     }
                 }
+                if constexpr (CANON) continue;
                 // transposed, lane L of the half-warp holds output row o0 + L: 16 bytes, one per j
                 transpose16(lw, lane);
                 transpose16(hw, lane);
