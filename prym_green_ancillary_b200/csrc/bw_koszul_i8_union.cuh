@@ -62,6 +62,8 @@
 #include "bw_koszul_i8_dev.cuh"
 #include "tc_sm100.cuh"
 
+#include <type_traits>
+
 namespace bw {
 
 namespace {
@@ -187,7 +189,8 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
         *abort = 0;
     }
     uint32_t tmem_cols = 32;
-    while (tmem_cols < static_cast<uint32_t>(2 * N * P.issuers)) tmem_cols *= 2;   // two buffers of an accumulator a warp
+    // two buffers of an accumulator a warp
+    while (tmem_cols < static_cast<uint32_t>(2 * N * P.issuers)) tmem_cols *= 2;
     if (warp == W::mma) {
         tc::tmem_alloc(tmem_slot, tmem_cols);
         tc::tmem_relinquish();
@@ -304,10 +307,12 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
             for (int q = 0; q < 4; ++q)
                 ahead[q] = has_word && issuer + q * P.issuers < n_stages ? __ldg(tab + q * tab_step) : 0u;
             tab += 4 * tab_step;
-            const uint32_t acc0 = tmem + static_cast<uint32_t>(issuer * N), buf_cols = static_cast<uint32_t>(P.issuers * N);
+            const uint32_t acc0 = tmem + static_cast<uint32_t>(issuer * N);
+            const uint32_t buf_cols = static_cast<uint32_t>(P.issuers * N);
             uint32_t acc = 0, buf = 0, acc_parity = 1;   // acc = 0: the next stage is the warp's first of a tile
             int slot = issuer % P.slots;
-            uint32_t bar = full0 + static_cast<uint32_t>(slot) * 8u, parity = static_cast<uint32_t>(issuer / P.slots) & 1u;
+            uint32_t bar = full0 + static_cast<uint32_t>(slot) * 8u;
+            uint32_t parity = static_cast<uint32_t>(issuer / P.slots) & 1u;
             uint32_t a_lo = a_slot0 + static_cast<uint32_t>(slot) * slot_units;
             const bool ok = tc::warp_wait(tc::smem_u32(maps_in), 0, nullptr, P.err, tc::ERR_WAIT_FINAL);
             // failure tests: CTA 0 waits for its first stage on a barrier that
@@ -372,115 +377,126 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
         const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
         const int chunks = (P.outer + 15) / 16;
         const uint32_t h_off = static_cast<uint32_t>((j >> 4) * P.outer * 16);
-        const bool scale = P.diag != nullptr;
         const bool vec = (P.outer & 3) == 0;       // whole int4 of the diagonal (its base is 16-byte aligned)
-        // diagonal entries of chunk c of tile tl's block
-        auto load_diag = [&](int32_t (&dg)[16], long long tl, int c) {
-            const long long bk = tl * BT + t;
-            const bool any = scale && bk < P.n_blk;
-            const int32_t* src = P.diag + bk * P.outer + c * 16;
-            if (vec) {
+        // a loop for every case, so that each is short (one loop for all four: 235
+        // instead of 232 us a step at r = 19, k = 9, 20 -> 28, 16 columns)
+        auto epilogue = [&](auto wide_c, auto scale_c) {
+            constexpr bool WIDE = decltype(wide_c)::value, SCALE = decltype(scale_c)::value;
+            // diagonal entries of chunk c of tile tl's block
+            auto load_diag = [&](int32_t (&dg)[16], long long tl, int c) {
+                const long long bk = tl * BT + t;
+                const bool any = SCALE && bk < P.n_blk;
+                const int32_t* src = P.diag + bk * P.outer + c * 16;
+                if (vec) {
 #pragma unroll
-                for (int o4 = 0; o4 < 4; ++o4) {
-                    const int4 d4 = any && c * 16 + o4 * 4 < P.outer ? __ldg(reinterpret_cast<const int4*>(src) + o4)
-                                                                     : make_int4(0, 0, 0, 0);
-                    dg[o4 * 4] = d4.x;
-                    dg[o4 * 4 + 1] = d4.y;
-                    dg[o4 * 4 + 2] = d4.z;
-                    dg[o4 * 4 + 3] = d4.w;
+                    for (int o4 = 0; o4 < 4; ++o4) {
+                        const int4 d4 = any && c * 16 + o4 * 4 < P.outer ? __ldg(reinterpret_cast<const int4*>(src) + o4)
+                                                                         : make_int4(0, 0, 0, 0);
+                        dg[o4 * 4] = d4.x;
+                        dg[o4 * 4 + 1] = d4.y;
+                        dg[o4 * 4 + 2] = d4.z;
+                        dg[o4 * 4 + 3] = d4.w;
+                    }
+                } else {
+#pragma unroll
+                    for (int oo = 0; oo < 16; ++oo) dg[oo] = any && c * 16 + oo < P.outer ? __ldg(src + oo) : 0;
                 }
-            } else {
+            };
+            if (!P.late_wait) pdl_wait();   // the output planes may still be read by earlier kernels
+            // a tile's first chunk is loaded one tile ahead (the diagonal streams from DRAM)
+            int32_t dg_next[16];
+            load_diag(dg_next, blockIdx.x, part);
+            long long tcount = 0;
+            for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tcount) {
+                const int buf = static_cast<int>(tcount & 1);
+                const uint32_t aph = static_cast<uint32_t>((tcount >> 1) & 1);
+                const long long blk = tile * BT + t;
+                const bool valid = blk < P.n_blk;
+                int32_t dg[16];
 #pragma unroll
-                for (int oo = 0; oo < 16; ++oo) dg[oo] = any && c * 16 + oo < P.outer ? __ldg(src + oo) : 0;
+                for (int oo = 0; oo < 16; ++oo) dg[oo] = dg_next[oo];
+                load_diag(dg_next, tile + gridDim.x, part);
+                if (!tc::warp_wait(accfull0 + static_cast<uint32_t>(buf) * 8u, aph, abort, P.err, tc::ERR_WAIT_ACCUM,
+                                   P.wait_limit))
+                    break;
+                tc::tc_fence_after();
+                const uint32_t col0 = tmem + lane_off + static_cast<uint32_t>(buf * P.issuers * N);
+                const long long base = blk * static_cast<long long>(NB) * P.outer + h_off;
+                for (int c = part; c < chunks; c += EPQ) {
+                    const int o0 = c * 16;
+                    if (c != part) load_diag(dg, tile, c);
+                    // this lane's 16 outputs (o0..o0+15 of its column j) as limb bytes; only groups of
+                    // eight columns that reach below outer are read (the accumulator has ho of each limb)
+                    uint32_t lw[4] = {0, 0, 0, 0}, hw[4] = {0, 0, 0, 0};
+                    const int live = P.outer - o0;
+#pragma unroll
+                    for (int h8 = 0; h8 < 2; ++h8) {
+                        if (h8 * 8 >= live) break;
+                        int32_t lo[8], hi[8];
+                        const uint32_t cb = col0 + static_cast<uint32_t>(o0 + h8 * 8);
+                        tc::tmem_ld8(cb, lo);
+                        tc::tmem_ld8(cb + P.ho, hi);
+                        if (P.issuers == 2) {   // the second warp's sums
+                            int32_t lo2[8], hi2[8];
+                            tc::tmem_ld8(cb + N, lo2);
+                            tc::tmem_ld8(cb + N + P.ho, hi2);
+                            tc::tmem_ld_wait();
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) {
+                                lo[q] += lo2[q];
+                                hi[q] += hi2[q];
+                            }
+                        } else {
+                            tc::tmem_ld_wait();
+                        }
+#pragma unroll
+                        for (int g4 = 0; g4 < 2; ++g4) {
+                            if (h8 * 8 + g4 * 4 >= live) break;
+                            int32_t v[4];
+#pragma unroll
+                            for (int oi = 0; oi < 4; ++oi) {
+                                const int o = g4 * 4 + oi;
+                                v[oi] = union_value<WIDE>(lo[o], hi[o], P.mod, SCALE, dg[h8 * 8 + o]);
+                            }
+                            if constexpr (CANON) {   // a row's columns are neighbouring lanes: whole sectors
+                                const int o = o0 + h8 * 8 + g4 * 4;
+                                uint32_t* at = P.canon + (blk * P.outer + o) * P.width + j;
+                                if (valid && j < P.width)
+#pragma unroll
+                                    for (int oi = 0; oi < 4; ++oi)
+                                        if (o + oi < P.outer)
+                                            at[oi * P.width] =
+                                                to_canonical(reduce_balanced_fast(v[oi] - P.mod.half, P.mod), P.mod);
+                            } else {
+                                pack_limbs(v, P.mod, lw[h8 * 2 + g4], hw[h8 * 2 + g4]);
+                            }
+                        }
+                    }
+                    if constexpr (CANON) continue;
+                    // transposed, lane L of the half-warp holds output row o0 + L: 16 bytes, one per j
+                    transpose16(lw, lane);
+                    transpose16(hw, lane);
+                    const int o = o0 + (lane & 15);
+                    if (valid && o < P.outer) {
+                        const long long at = base + o * 16;
+                        *reinterpret_cast<uint4*>(P.out[PL_LO] + at) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+                        *reinterpret_cast<uint4*>(P.out[PL_HI] + at) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+                        *reinterpret_cast<uint4*>(P.out[PL_NLO] + at) =
+                            make_uint4(neg_bytes4(lw[0]), neg_bytes4(lw[1]), neg_bytes4(lw[2]), neg_bytes4(lw[3]));
+                        *reinterpret_cast<uint4*>(P.out[PL_NHI] + at) =
+                            make_uint4(neg_bytes4(hw[0]), neg_bytes4(hw[1]), neg_bytes4(hw[2]), neg_bytes4(hw[3]));
+                    }
+                }
+                tc::tc_fence_before();
+                tc::mbar_arrive(&accempty[buf]);
             }
         };
-        if (!P.late_wait) pdl_wait();   // the output planes may still be read by earlier kernels
-        // a tile's first chunk is loaded one tile ahead (the diagonal streams from DRAM)
-        int32_t dg_next[16];
-        load_diag(dg_next, blockIdx.x, part);
-        long long tcount = 0;
-        for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tcount) {
-            const int buf = static_cast<int>(tcount & 1);
-            const uint32_t aph = static_cast<uint32_t>((tcount >> 1) & 1);
-            const long long blk = tile * BT + t;
-            const bool valid = blk < P.n_blk;
-            int32_t dg[16];
-#pragma unroll
-            for (int oo = 0; oo < 16; ++oo) dg[oo] = dg_next[oo];
-            load_diag(dg_next, tile + gridDim.x, part);
-            if (!tc::warp_wait(accfull0 + static_cast<uint32_t>(buf) * 8u, aph, abort, P.err, tc::ERR_WAIT_ACCUM, P.wait_limit)) break;
-            tc::tc_fence_after();
-            const uint32_t col0 = tmem + lane_off + static_cast<uint32_t>(buf * P.issuers * N);
-            const long long base = blk * static_cast<long long>(NB) * P.outer + h_off;
-            for (int c = part; c < chunks; c += EPQ) {
-                const int o0 = c * 16;
-                if (c != part) load_diag(dg, tile, c);
-                // this lane's 16 outputs (o0..o0+15 of its column j) as limb bytes; only groups of
-                // eight columns that reach below outer are read (the accumulator has ho of each limb)
-                uint32_t lw[4] = {0, 0, 0, 0}, hw[4] = {0, 0, 0, 0};
-                const int live = P.outer - o0;
-#pragma unroll
-                for (int h8 = 0; h8 < 2; ++h8) {
-                    if (h8 * 8 >= live) break;
-                    int32_t lo[8], hi[8];
-                    const uint32_t cb = col0 + static_cast<uint32_t>(o0 + h8 * 8);
-                    tc::tmem_ld8(cb, lo);
-                    tc::tmem_ld8(cb + P.ho, hi);
-                    if (P.issuers == 2) {   // the second warp's sums
-                        int32_t lo2[8], hi2[8];
-                        tc::tmem_ld8(cb + N, lo2);
-                        tc::tmem_ld8(cb + N + P.ho, hi2);
-                        tc::tmem_ld_wait();
-#pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            lo[q] += lo2[q];
-                            hi[q] += hi2[q];
-                        }
-                    } else {
-                        tc::tmem_ld_wait();
-                    }
-#pragma unroll
-                    for (int g4 = 0; g4 < 2; ++g4) {
-                        if (h8 * 8 + g4 * 4 >= live) break;
-                        int32_t v[4];
-#pragma unroll
-                        for (int oi = 0; oi < 4; ++oi) {
-                            const int o = g4 * 4 + oi;
-                            v[oi] = P.wide ? union_value<true>(lo[o], hi[o], P.mod, scale, dg[h8 * 8 + o])
-                                           : union_value<false>(lo[o], hi[o], P.mod, scale, dg[h8 * 8 + o]);
-                        }
-                        if constexpr (CANON) {   // a row's columns are neighbouring lanes: whole sectors
-                            const int o = o0 + h8 * 8 + g4 * 4;
-                            uint32_t* at = P.canon + (blk * P.outer + o) * P.width + j;
-                            if (valid && j < P.width)
-#pragma unroll
-                                for (int oi = 0; oi < 4; ++oi)
-                                    if (o + oi < P.outer)
-                                        at[oi * P.width] =
-                                            to_canonical(reduce_balanced_fast(v[oi] - P.mod.half, P.mod), P.mod);
-                        } else {
-                            pack_limbs(v, P.mod, lw[h8 * 2 + g4], hw[h8 * 2 + g4]);
-                        }
-                    }
-                }
-                if constexpr (CANON) continue;
-                // transposed, lane L of the half-warp holds output row o0 + L: 16 bytes, one per j
-                transpose16(lw, lane);
-                transpose16(hw, lane);
-                const int o = o0 + (lane & 15);
-                if (valid && o < P.outer) {
-                    const long long at = base + o * 16;
-                    *reinterpret_cast<uint4*>(P.out[PL_LO] + at) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-                    *reinterpret_cast<uint4*>(P.out[PL_HI] + at) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-                    *reinterpret_cast<uint4*>(P.out[PL_NLO] + at) =
-                        make_uint4(neg_bytes4(lw[0]), neg_bytes4(lw[1]), neg_bytes4(lw[2]), neg_bytes4(lw[3]));
-                    *reinterpret_cast<uint4*>(P.out[PL_NHI] + at) =
-                        make_uint4(neg_bytes4(hw[0]), neg_bytes4(hw[1]), neg_bytes4(hw[2]), neg_bytes4(hw[3]));
-                }
-            }
-            tc::tc_fence_before();
-            tc::mbar_arrive(&accempty[buf]);
-        }
+        using Yes = std::true_type;
+        using No = std::false_type;
+        if (P.diag != nullptr)
+            P.wide ? epilogue(Yes{}, Yes{}) : epilogue(No{}, Yes{});
+        else
+            P.wide ? epilogue(Yes{}, No{}) : epilogue(No{}, No{});
     }
 
     tc::tc_fence_before();
