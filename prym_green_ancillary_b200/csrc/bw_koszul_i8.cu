@@ -1151,6 +1151,7 @@ struct KoszulCtx::I8State {
         int8_t* maps = nullptr;
         std::vector<uint32_t> mask;      // [tile] union of its blocks' generators
         uint32_t* d_mask = nullptr;
+        uint32_t* order = nullptr;       // [tile][BT] blocks (see I8Union)
         uint32_t *start = nullptr, *words = nullptr, *steps = nullptr;   // stage list of list_gs generators a stage
         int list_gs = 0, list_issuers = 0;
     } fwd, bwd;
@@ -1364,14 +1365,16 @@ __global__ void gather_rows_kernel(const uint32_t* __restrict__ inc, int4* __res
 }
 
 // Per tile of bt blocks, the generators that any of its blocks has.
-__global__ void union_mask_kernel(const uint32_t* __restrict__ inc, uint32_t* __restrict__ mask, long long n_tiles,
-                                  long long n_blk, int r, int bt) {
+__global__ void union_mask_kernel(const uint32_t* __restrict__ inc, const uint32_t* __restrict__ order,
+                                  uint32_t* __restrict__ mask, long long n_tiles, int r, int bt) {
     const long long tile = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (tile >= n_tiles) return;
     uint32_t m = 0;
-    for (long long blk = tile * bt; blk < min(n_blk, (tile + 1) * bt); ++blk)
-        for (int i = 0; i < r; ++i)
-            if (inc[blk * r + i] != kAbsent) m |= 1u << i;
+    for (int t = 0; t < bt; ++t) {
+        const uint32_t blk = order[tile * bt + t];
+        for (int i = 0; blk != kNoBlock && i < r; ++i)
+            if (inc[static_cast<size_t>(blk) * r + i] != kAbsent) m |= 1u << i;
+    }
     mask[tile] = m;
 }
 
@@ -1445,9 +1448,38 @@ std::vector<int8_t> union_maps(const KoszulCtx& c, int inner, int outer, bool tr
     return maps;
 }
 
+// D.order: the blocks of a direction in the order of star_quad(), n_order >=
+// n_blk entries, kNoBlock where the last four of a kind have no block.
+void build_order(KoszulCtx& c, KoszulCtx::I8State::Dir& D, uint64_t n_blk, uint64_t n_order, bool forward,
+                 const BinomTable& binoms) {
+    const int size = forward ? c.k - 1 : c.k;
+    const unsigned ctas = blocks_of(n_blk, kOrderThreads);
+    D.order = c.alloc<uint32_t>(n_order);
+    // With a tile a CTA at most, a kernel is one tile's latency whatever its
+    // generators: lexicographic (the order's set-up took 0.1 ms of 0.8).
+    if (n_order * c.nbi <= static_cast<uint64_t>(c.sms) * 128) {
+        order_plain_kernel<<<blocks_of(n_order, kOrderThreads), kOrderThreads, 0, c.own_stream>>>(
+            D.order, static_cast<uint32_t>(n_blk), static_cast<uint32_t>(n_order));
+        BW_CHECK_LAUNCH();
+        return;
+    }
+    uint32_t* tmp = c.alloc<uint32_t>(2 * (ctas + 1ull) + n_blk + n_blk / 4 + 1);
+    uint2* counts = reinterpret_cast<uint2*>(tmp);
+    uint32_t *rest = tmp + 2 * (ctas + 1ull), *four = rest + n_blk;
+    const long long n = static_cast<long long>(n_blk);
+    BW_CUDA(cudaMemsetAsync(D.order, 0xFF, n_order * 4, c.own_stream));
+    order_count_kernel<<<ctas, kOrderThreads, 0, c.own_stream>>>(counts, n, c.r, size, forward, binoms);
+    order_scan_kernel<<<1, 1024, 0, c.own_stream>>>(counts, static_cast<int>(ctas));
+    order_place_kernel<<<ctas, kOrderThreads, 0, c.own_stream>>>(counts, D.order, rest, four, n, c.r, size, forward,
+                                                                 binoms);
+    order_rest_kernel<<<ctas, kOrderThreads, 0, c.own_stream>>>(counts + ctas, rest, four, D.order);
+    BW_CHECK_LAUNCH();
+    c.release(tmp);   // cudaFree waits for the kernels
+}
+
 // Builds the stage list for D.u's generators a stage: CTA c's tiles are c,
 // c + grid, ..., their stages one after the other.
-void build_stage_list(KoszulCtx& c, KoszulCtx::I8State::Dir& D, uint64_t n_blk, uint64_t n_in, int inner) {
+void build_stage_list(KoszulCtx& c, KoszulCtx::I8State::Dir& D, uint64_t n_in, int inner) {
     I8Union& U = D.u;
     if (D.list_gs != U.gs || D.list_issuers != U.issuers) {
         for (uint32_t** p : {&D.start, &D.words, &D.steps})
@@ -1475,14 +1507,16 @@ void build_stage_list(KoszulCtx& c, KoszulCtx::I8State::Dir& D, uint64_t n_blk, 
         BW_CUDA(cudaMemcpyAsync(d_ts, tile_stage.data(), tiles * 4, cudaMemcpyHostToDevice, c.own_stream));
         const uint32_t run16 = static_cast<uint32_t>((c.nbi / 16) * inner);
         union_tables_kernel<<<blocks_of(tiles, 128), 128, 0, c.own_stream>>>(
-            D.inc, D.d_mask, d_ts, D.words, D.steps, static_cast<long long>(tiles), static_cast<long long>(n_blk), c.r,
-            bt, U.gs, U.cpg, 2 * U.ho, U.row, U.issuers, run16, static_cast<uint32_t>(n_in * run16));
+            D.inc, D.order, D.d_mask, d_ts, D.words, D.steps, static_cast<long long>(tiles), c.r, bt, U.gs, U.cpg,
+            2 * U.ho, U.row, U.issuers, run16, static_cast<uint32_t>(n_in * run16));
         BW_CHECK_LAUNCH();
         BW_CUDA(cudaStreamSynchronize(c.own_stream));
         c.release(d_ts);
         D.list_gs = U.gs;
         D.list_issuers = U.issuers;
     }
+    U.n_tiles = static_cast<long long>(D.mask.size());
+    U.order = D.order;
     U.start = D.start;
     U.words = D.words;
     U.steps = D.steps;
@@ -1739,8 +1773,9 @@ void KoszulCtx::i8_setup() {
         if (any_union) {
             const uint64_t tiles = (n_out + bt - 1) / bt;
             D.d_mask = alloc<uint32_t>(tiles);
-            union_mask_kernel<<<blocks_of(tiles, 128), 128, 0, own_stream>>>(
-                D.inc, D.d_mask, static_cast<long long>(tiles), static_cast<long long>(n_out), r, bt);
+            build_order(*this, D, n_out, tiles * bt, dir == 0, binoms);
+            union_mask_kernel<<<blocks_of(tiles, 128), 128, 0, own_stream>>>(D.inc, D.order, D.d_mask,
+                                                                             static_cast<long long>(tiles), r, bt);
             D.mask.resize(tiles);
             BW_CUDA(cudaMemcpyAsync(D.mask.data(), D.d_mask, tiles * 4, cudaMemcpyDeviceToHost, own_stream));
             const std::vector<int8_t> maps = union_maps(*this, inner, outer, dir == 1);
@@ -1805,7 +1840,7 @@ void KoszulCtx::i8_setup() {
                 if (!plan_union(*this, D, inner, outer, dir == 1, c.gps, c.t_tma, c.issuers) ||
                     static_cast<int>(D.smem) > cap_u)
                     return false;
-                build_stage_list(*this, D, dir == 0 ? n_t : n_s, dir == 0 ? n_s : n_t, inner);
+                build_stage_list(*this, D, dir == 0 ? n_s : n_t, inner);
                 D.u.err = S.err;
                 D.u.wait_limit = wait_limit;
                 D.u.hold_first_stage = 0;
@@ -1886,6 +1921,7 @@ void KoszulCtx::i8_setup() {
             drop(D->words);
             drop(D->steps);
             drop(D->maps);
+            drop(D->order);
         }
         if (!D->gather4) drop(D->rows4);
         drop(D->d_mask);
@@ -1932,7 +1968,6 @@ void KoszulCtx::i8_run(bool forward_dir, int in_buf, int out_buf, bool scale, cu
         D.u.in[0] = i8->planes[in_buf][PL_LO];
         D.u.in[1] = i8->planes[in_buf][PL_HI];
         for (int pl = 0; pl < 4; ++pl) D.u.out[pl] = i8->planes[out_buf][pl];
-        D.u.n_blk = D.p.n_blk;
         D.u.diag = (!forward_dir && scale) ? d_diag : nullptr;
         D.u.canon = canon;
         D.u.width = nb;

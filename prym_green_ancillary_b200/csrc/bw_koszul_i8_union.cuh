@@ -12,11 +12,10 @@
 //     to 8) holds  out = acc_lo + 255 acc_hi:  the epilogue reads two partial
 //     sums an output instead of four.  |acc| <= 2 * 1024 * 127^2 < 2^26.
 //   * K runs over the union of the tile's generators only.  A tile is BT =
-//     128 / NB consecutive blocks in lexicographic order; they share most of
-//     their subset (config sizes r = 19, k = 9: 14.0 of 19 generators a tile
-//     for d and 12.6 for d^T; r = 23, k = 11: 15.4 and 13.7 of 23).  A tile's
-//     generators come in ascending order; a host table holds, per tile and
-//     position in the union, the BT neighbours' run offsets.
+//     128 / NB blocks of an order that keeps blocks with nearly the same subset
+//     together (see star_quad(); r = 19, k = 9: 13.6 of 19 generators a tile for
+//     d and 12.0 for d^T).  A tile's generators come in ascending order; a table
+//     holds, per tile and position in the union, the BT neighbours' run offsets.
 //   * A generator's K' rows are padded to a multiple of 16, the width of a
 //     core matrix of the K-major B operand.  The maps stay resident in shared
 //     memory as [generator][16-row chunk][N][16 bytes]; a K-step of 32 rows
@@ -52,7 +51,8 @@
 // Measured on one B200 (1965 MHz), us, dense kernels -> one MMA warp -> two:
 // r = 19, k = 9, dims 20 -> 28, 16 columns: d 179 -> 130 -> 92, d^T 228 -> 156 ->
 // 127; r = 21, k = 10, dims 32 -> 40, 32 columns: d 1726 -> 1190 -> 1050, d^T
-// 2429 -> 1411 -> 1260.  With the other roles' work switched off the copies
+// 2429 -> 1411 -> 1260.  (With lexicographic tiles; the star order takes another 1
+// to 5 %.)  With the other roles' work switched off the copies
 // alone take 60 / 76 us at the first size and 614 / 745 at the second, the MMAs
 // 74 / 78 and 555 / 591, the epilogue 73 / 95 and 728 / 859, and the hand-overs
 // without any of them 59 / 60 and 348 / 377: no role is far above the others.
@@ -60,6 +60,7 @@
 
 #include "bw_common.cuh"
 #include "bw_koszul_i8_dev.cuh"
+#include "bw_koszul_tables.cuh"
 #include "tc_sm100.cuh"
 
 #include <type_traits>
@@ -83,6 +84,7 @@ constexpr int threads = (epilogue0 + epilogue) * 32;
 
 constexpr int kUnionPasses = 10;   // 32-unit passes a producer warp makes over a stage, at most
 constexpr int kUnionSteps = 16;    // K-steps of a stage, at most
+constexpr uint32_t kNoBlock = 0xFFFFFFFFu;
 constexpr uint32_t kSkip = 0xFFFFFFFEu;      // table word of a generator slot past the tile's union
 constexpr uint32_t kStepValid = 1u << 14;    // step word: this K-step exists (a descriptor's free bits)
 constexpr uint32_t kStepLast = 1u << 15;     // step word 0: the issuing warp's last stage of its tile
@@ -93,13 +95,14 @@ struct I8Union {
     uint32_t* canon;               // CANON: the output as canonical residues, [n_blk * outer][width]
     int width;                     // columns of the caller's block (the rest of NB are zero padding)
     const uint32_t* start;         // [grid + 1]: first stage of every CTA's list
+    const uint32_t* order;         // [tile][BT]: the tile's blocks, kNoBlock past the last one
     const uint32_t* words;         // [stage][gs * BT]: the neighbour run's 16-byte offset from the +plane,
                                    // kAbsent (rows of zeros) or kSkip (no rows)
     const uint32_t* steps;         // [stage][row]: low descriptor word of every K-step's maps, relative to them
     const int8_t* maps;            // B operand in its shared-memory layout, the zero chunk last
     const int32_t* diag;           // nullptr, or [n_blk * outer] balanced (scales the output)
     int* err;
-    long long n_blk;
+    long long n_tiles;
     int r, inner, outer, ho;       // N = 2 * ho, ho = outer rounded up to 8
     int cpg;                       // 16-row chunks of a generator's 2 * inner K' rows
     int gs;                        // generators a stage (even when cpg is odd)
@@ -172,7 +175,7 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
 
     // the warp index through a shuffle, so that role and pass branches are uniform
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0), lane = threadIdx.x % 32;
-    const long long n_tiles = (P.n_blk + BT - 1) / BT;
+    const long long n_tiles = P.n_tiles;
     pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.slots; ++s) {
@@ -382,11 +385,10 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
         // instead of 232 us a step at r = 19, k = 9, 20 -> 28, 16 columns)
         auto epilogue = [&](auto wide_c, auto scale_c) {
             constexpr bool WIDE = decltype(wide_c)::value, SCALE = decltype(scale_c)::value;
-            // diagonal entries of chunk c of tile tl's block
-            auto load_diag = [&](int32_t (&dg)[16], long long tl, int c) {
-                const long long bk = tl * BT + t;
-                const bool any = SCALE && bk < P.n_blk;
-                const int32_t* src = P.diag + bk * P.outer + c * 16;
+            // diagonal entries of chunk c of block bk
+            auto load_diag = [&](int32_t (&dg)[16], uint32_t bk, int c) {
+                const bool any = SCALE && bk != kNoBlock;
+                const int32_t* src = P.diag + static_cast<long long>(bk) * P.outer + c * 16;
                 if (vec) {
 #pragma unroll
                     for (int o4 = 0; o4 < 4; ++o4) {
@@ -405,17 +407,22 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
             if (!P.late_wait) pdl_wait();   // the output planes may still be read by earlier kernels
             // a tile's first chunk is loaded one tile ahead (the diagonal streams from DRAM)
             int32_t dg_next[16];
-            load_diag(dg_next, blockIdx.x, part);
+            auto block_of = [&](long long tl) { return tl < n_tiles ? __ldg(P.order + tl * BT + t) : kNoBlock; };
+            uint32_t blk_next = block_of(blockIdx.x), blk_after = block_of(blockIdx.x + gridDim.x);
+            load_diag(dg_next, blk_next, part);
             long long tcount = 0;
             for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tcount) {
                 const int buf = static_cast<int>(tcount & 1);
                 const uint32_t aph = static_cast<uint32_t>((tcount >> 1) & 1);
-                const long long blk = tile * BT + t;
-                const bool valid = blk < P.n_blk;
+                const uint32_t blk_now = blk_next;
+                const bool valid = blk_now != kNoBlock;
+                const long long blk = blk_now;
+                blk_next = blk_after;
+                blk_after = block_of(tile + 2ll * gridDim.x);
                 int32_t dg[16];
 #pragma unroll
                 for (int oo = 0; oo < 16; ++oo) dg[oo] = dg_next[oo];
-                load_diag(dg_next, tile + gridDim.x, part);
+                load_diag(dg_next, blk_next, part);
                 if (!tc::warp_wait(accfull0 + static_cast<uint32_t>(buf) * 8u, aph, abort, P.err, tc::ERR_WAIT_ACCUM,
                                    P.wait_limit))
                     break;
@@ -424,7 +431,7 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
                 const long long base = blk * static_cast<long long>(NB) * P.outer + h_off;
                 for (int c = part; c < chunks; c += EPQ) {
                     const int o0 = c * 16;
-                    if (c != part) load_diag(dg, tile, c);
+                    if (c != part) load_diag(dg, blk_now, c);
                     // this lane's 16 outputs (o0..o0+15 of its column j) as limb bytes; only groups of
                     // eight columns that reach below outer are read (the accumulator has ho of each limb)
                     uint32_t lw[4] = {0, 0, 0, 0}, hw[4] = {0, 0, 0, 0};
@@ -508,13 +515,133 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
     if (P.late_wait) pdl_wait();   // this kernel's completion implies that of all kernels before it
 }
 
+// ---- the order of the blocks
+//
+// The fewer generators the blocks of a tile have between them, the fewer rows
+// it gathers and multiplies.  Four blocks that agree but for the place of one
+// element have the least: d's T = C u {x} lack only C's generators in common,
+// d^T's S = Q \ {x} lie in one set Q of k + 1.  So the elements are cut into
+// quads (from the last element down); a block whose set meets some quad in one
+// element (d) or three (d^T), the last such quad, goes with the three blocks
+// that differ from it there (its star: they have the same last such quad, so
+// stars are disjoint).  The blocks without such a quad go four by four as they
+// come.  Both kinds follow the lexicographic order of their first block, which
+// keeps the gathered rows of neighbouring tiles close.  A tile is one such four
+// (32 columns) or two.  Generators of a tile, lexicographic tiles -> these: r = 21,
+// k = 10, tiles of four: d 14.4 -> 13.2, d^T 12.7 -> 11.4; r = 19, k = 9, tiles of
+// eight: d 14.0 -> 13.6, d^T 12.6 -> 11.9.  (us: d^T at r = 20,
+// k = 8, 21 -> 29, 32 columns and a step of r = 23, k = 11, 32 -> 40, 32 columns:
+// 552 -> 548 with its conversion, 13100 -> 12750.)
+
+// First element of the set's star quad, or -1.
+__device__ __forceinline__ int star_quad(uint32_t set, int r, bool forward) {
+    for (int base = r - 4; base >= 0; base -= 4)
+        if (__popc(set >> base & 15u) == (forward ? 1 : 3)) return base;
+    return -1;
+}
+
+constexpr int kOrderThreads = 256;
+
+// 0: no star; 1: first of its star (lexicographically); 2: another of it.
+__device__ __forceinline__ int star_role(uint32_t set, int base, bool forward) {
+    return base < 0 ? 0 : (set >> base & 15u) == (forward ? 1u : 7u) ? 1 : 2;
+}
+
+// counts[CTA] = its stars and its blocks without one.
+__global__ void __launch_bounds__(kOrderThreads) order_count_kernel(uint2* counts, long long n_blk, int r, int size,
+                                                                    bool forward,
+                                                                    const __grid_constant__ BinomTable B) {
+    const long long blk = blockIdx.x * static_cast<long long>(kOrderThreads) + threadIdx.x;
+    int role = 2;
+    if (blk < n_blk) {
+        const uint32_t set = subset_of(static_cast<uint32_t>(blk), r, size, B);
+        role = star_role(set, star_quad(set, r, forward), forward);
+    }
+    const unsigned stars = __syncthreads_count(role == 1), rest = __syncthreads_count(role == 0);
+    if (threadIdx.x == 0) counts[blockIdx.x] = make_uint2(stars, rest);
+}
+
+// Exclusive sums in place; the totals follow the last entry.  One CTA of 1024.
+__global__ void __launch_bounds__(1024) order_scan_kernel(uint2* counts, int n) {
+    __shared__ uint2 part[1024];
+    const int per = (n + 1023) / 1024, lo = min(n, static_cast<int>(threadIdx.x) * per), hi = min(n, lo + per);
+    uint2 sum = make_uint2(0, 0);
+    for (int i = lo; i < hi; ++i) sum = make_uint2(sum.x + counts[i].x, sum.y + counts[i].y);
+    part[threadIdx.x] = sum;
+    __syncthreads();
+    for (int d = 1; d < 1024; d *= 2) {
+        const uint2 v = static_cast<int>(threadIdx.x) >= d ? part[threadIdx.x - d] : make_uint2(0, 0);
+        __syncthreads();
+        part[threadIdx.x].x += v.x;
+        part[threadIdx.x].y += v.y;
+        __syncthreads();
+    }
+    uint2 at = make_uint2(part[threadIdx.x].x - sum.x, part[threadIdx.x].y - sum.y);
+    for (int i = lo; i < hi; ++i) {
+        const uint2 c = counts[i];
+        counts[i] = at;
+        at = make_uint2(at.x + c.x, at.y + c.y);
+    }
+    if (threadIdx.x == 1023) counts[n] = at;
+}
+
+// Writes the stars to order and the other blocks, in order, to rest; with l stars
+// and q other blocks before it, a star is the four number l + ceil(q / 4), and
+// the other blocks q .. q + 3 (4 | q) are the four number l + q / 4, kept in four[q / 4].
+__global__ void __launch_bounds__(kOrderThreads) order_place_kernel(const uint2* counts, uint32_t* order, uint32_t* rest,
+                                                                    uint32_t* four, long long n_blk, int r, int size,
+                                                                    bool forward,
+                                                                    const __grid_constant__ BinomTable B) {
+    __shared__ uint2 warps[kOrderThreads / 32];
+    const long long blk = blockIdx.x * static_cast<long long>(kOrderThreads) + threadIdx.x;
+    const unsigned warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    uint32_t set = 0;
+    int base = -1, role = 2;
+    if (blk < n_blk) {
+        set = subset_of(static_cast<uint32_t>(blk), r, size, B);
+        base = star_quad(set, r, forward);
+        role = star_role(set, base, forward);
+    }
+    const uint32_t stars = __ballot_sync(0xffffffffu, role == 1), others = __ballot_sync(0xffffffffu, role == 0);
+    if (lane == 0) warps[warp] = make_uint2(__popc(stars), __popc(others));
+    __syncthreads();
+    const uint32_t below = (1u << lane) - 1;
+    uint32_t l = counts[blockIdx.x].x + __popc(stars & below), q = counts[blockIdx.x].y + __popc(others & below);
+    for (unsigned w = 0; w < warp; ++w) {
+        l += warps[w].x;
+        q += warps[w].y;
+    }
+    if (role == 1) {
+        uint32_t* out = order + 4ull * (l + (q + 3) / 4);
+        const uint32_t rem = set & ~(15u << base);
+        for (int j = 0; j < 4; ++j)   // ascending ranks: d's one element rises, d^T's missing one falls
+            out[j] = rank_of(rem | (forward ? 1u << j : 15u & ~(8u >> j)) << base, r, size, B);
+    } else if (role == 0) {
+        rest[q] = static_cast<uint32_t>(blk);
+        if (q % 4 == 0) four[q / 4] = l + q / 4;
+    }
+}
+
+// Lexicographic order.
+__global__ void __launch_bounds__(kOrderThreads) order_plain_kernel(uint32_t* order, uint32_t n_blk, uint32_t n_order) {
+    const uint32_t i = blockIdx.x * kOrderThreads + threadIdx.x;
+    if (i < n_order) order[i] = i < n_blk ? i : kNoBlock;
+}
+
+__global__ void __launch_bounds__(kOrderThreads) order_rest_kernel(const uint2* total, const uint32_t* rest,
+                                                                   const uint32_t* four, uint32_t* order) {
+    const uint32_t q = blockIdx.x * kOrderThreads + threadIdx.x;
+    if (q < total->y) order[4ull * four[q / 4] + q % 4] = rest[q];
+}
+
 // The union kernel's stage list (see I8Union): tile t's stages start at
 // tile_stage[t]; mask[t] is its union, inc the dense [n_blk][r] table
 // (neighbour rank | negative << 31, or kAbsent).
-__global__ void union_tables_kernel(const uint32_t* __restrict__ inc, const uint32_t* __restrict__ mask,
-                                    const uint32_t* __restrict__ tile_stage, uint32_t* __restrict__ words,
-                                    uint32_t* __restrict__ steps, long long n_tiles, long long n_blk, int r, int bt,
-                                    int gs, int cpg, int n_cols, int row, int issuers, uint32_t run16, uint32_t neg16) {
+__global__ void union_tables_kernel(const uint32_t* __restrict__ inc, const uint32_t* __restrict__ order,
+                                    const uint32_t* __restrict__ mask, const uint32_t* __restrict__ tile_stage,
+                                    uint32_t* __restrict__ words, uint32_t* __restrict__ steps, long long n_tiles, int r,
+                                    int bt, int gs, int cpg, int n_cols, int row, int issuers, uint32_t run16,
+                                    uint32_t neg16) {
     const long long tile = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     if (tile >= n_tiles) return;
     const uint32_t all = mask[tile];
@@ -527,8 +654,8 @@ __global__ void union_tables_kernel(const uint32_t* __restrict__ inc, const uint
         for (int t = 0; t < bt; ++t) {
             uint32_t v = kSkip;
             if (i >= 0) {
-                const long long blk = tile * bt + t;
-                const uint32_t e = blk < n_blk ? inc[blk * r + i] : kAbsent;
+                const uint32_t blk = order[tile * bt + t];
+                const uint32_t e = blk != kNoBlock ? inc[static_cast<size_t>(blk) * r + i] : kAbsent;
                 v = e == kAbsent ? kAbsent : (e >> 31 ? neg16 : 0u) + (e & 0x7FFFFFFFu) * run16;
             }
             w[q * bt + t] = v;

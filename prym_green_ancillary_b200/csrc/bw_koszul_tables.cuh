@@ -17,6 +17,25 @@ inline BinomTable binom_table() {
     return t;
 }
 
+// The size-subset of 0..r-1 of lexicographic rank blk, as a bit mask.
+__device__ __forceinline__ uint32_t subset_of(uint32_t blk, int r, int size, const BinomTable& B) {
+    uint32_t set = 0, rem = B.c[r][size] - 1 - blk;
+    for (int pos = 0, v = 0; pos < size; ++pos, ++v) {
+        while (B.c[r - 1 - v][size - pos] > rem) ++v;
+        rem -= B.c[r - 1 - v][size - pos];
+        set |= 1u << v;
+    }
+    return set;
+}
+
+// Its inverse.
+__device__ __forceinline__ uint32_t rank_of(uint32_t set, int r, int size, const BinomTable& B) {
+    uint32_t rank = B.c[r][size] - 1;
+    for (int v = 0, left = size; left > 0; ++v)
+        if (set >> v & 1) rank -= B.c[r - 1 - v][left--];
+    return rank;
+}
+
 // Calls f(i, rank, negative) for every neighbour of block blk, i ascending:
 //   forward : blk = T, a (k-1)-subset; neighbour S = T u {i} for every i not in T
 //   backward: blk = S, a k-subset; neighbour T = S \ {i} for every i in S
@@ -28,12 +47,7 @@ template <class F>
 __device__ __forceinline__ void for_each_neighbour(uint32_t blk, int r, int k, bool forward, const BinomTable& B,
                                                    F&& f) {
     const int size = forward ? k - 1 : k, other = forward ? k : k - 1;   // of blk, of its neighbours
-    uint32_t set = 0, rem = B.c[r][size] - 1 - blk;
-    for (int pos = 0, v = 0; pos < size; ++pos, ++v) {
-        while (B.c[r - 1 - v][size - pos] > rem) ++v;
-        rem -= B.c[r - 1 - v][size - pos];
-        set |= 1u << v;
-    }
+    const uint32_t set = subset_of(blk, r, size, B);
     // an element at position j counts C(r-1-v, other - j) below i; above i its
     // position in the neighbour is j + 1 (forward) or j - 1 (backward)
     const int shift = forward ? 1 : -1;
