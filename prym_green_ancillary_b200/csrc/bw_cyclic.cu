@@ -441,7 +441,6 @@ CyclicCtx::~CyclicCtx() {
     for (auto& g : graphs)
         if (g) cudaGraphExecDestroy(g);
     for (void* p : allocations) cudaFree(p);
-    if (h_err) cudaFreeHost(const_cast<int*>(h_err));
     for (auto& lane : out_lanes) {
         cudaFreeHost(lane.pinned);
         cudaStreamDestroy(lane.stream);
@@ -898,10 +897,12 @@ void CyclicCtx::generate(size_t nlen_target, float* device_ms) {
         *device_ms = 0;
     }
     seq_len = 1 + 4 * rounds;
+    int err = 0;
+    if (persistent) BW_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
     BW_CUDA(cudaStreamSynchronize(stream));
-    if (persistent && *h_err != 0) {
-        *h_err = 0;
+    if (err != 0) {
         seq_len = 0;
+        BW_CUDA(cudaMemset(d_err, 0, sizeof(int)));
         BW_CUDA(cudaMemset(d_partials, 0, 20 * sizeof(int32_t)));
         throw Error("the sequence's kernel gave up waiting (grid barrier between its phases)", 2);
     }
@@ -917,7 +918,7 @@ uint32_t* CyclicCtx::scratch_canonical() {
 // writing (and first touching) the destination's pages, which the threads
 // share (18 MB: 12 ms by one copy call).
 void CyclicCtx::copy_out(void* dst, const void* src, size_t bytes) {
-    constexpr size_t kChunk = size_t{1} << 20;
+    constexpr size_t kChunk = size_t{1} << 18;
     const size_t chunks = (bytes + kChunk - 1) / kChunk;
     const size_t workers = std::min<size_t>({4, std::max(1u, std::thread::hardware_concurrency()), chunks / 2});
     if (workers < 2) {

@@ -149,8 +149,7 @@ struct CyclicCtx {
     size_t rounds_smem = 0;
     uint32_t rounds_wait_limit = 1u << 22;
     uint32_t* d_barrier = nullptr;
-    int* d_err = nullptr;                 // mapped host memory (h_err)
-    volatile int* h_err = nullptr;
+    int* d_err = nullptr;                 // set by a grid barrier that gave up
     // validation path (explicit rowmix rounds)
     uint32_t* d_pairs = nullptr;
     int32_t* d_dr = nullptr;

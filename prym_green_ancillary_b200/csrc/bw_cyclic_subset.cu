@@ -1074,11 +1074,8 @@ void CyclicCtx::setup_rounds() {
     rounds_threads = static_cast<int>(threads) + kMomentThreads;
     rounds_grid = (items + threads - 1) / threads;
     d_barrier = alloc<uint32_t>(1);
-    void* word = nullptr;
-    BW_CUDA(cudaHostAlloc(&word, sizeof(int), cudaHostAllocMapped));
-    h_err = static_cast<volatile int*>(word);
-    *h_err = 0;
-    BW_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&d_err), word, 0));
+    d_err = alloc<int>(1);
+    BW_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), stream));
     if (const char* e = std::getenv("BW_TEST_WAIT_LIMIT")) {
         const unsigned long v = std::strtoul(e, nullptr, 10);
         if (v >= 1 && v < rounds_wait_limit) rounds_wait_limit = static_cast<uint32_t>(v);
