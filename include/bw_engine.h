@@ -141,11 +141,12 @@ BW_API int bw_koszul_seq_step_timed(bw_koszul* ctx, uint64_t steps, float* ms_ou
 BW_API uint64_t bw_koszul_launch_count(const bw_koszul* ctx);
 
 /* The context's kernel plan as text: for the INT8 form, each direction's
- * producer (TMA gathers or 8 or 16 cp.async warps), generators per stage,
- * pipeline slots and shared memory, with the set-up autotuner's timing of
- * every candidate when it ran (a shape already tuned in this process reuses
- * the choice), and the projection's stage; for the plain form, the output
- * rows a thread of each direction's gathers (4 or 8, timed the same way).  No reference counterpart (the
+ * kernel (union, hybrid or cp.async), generators per stage, producer groups
+ * and MMA warps (union), pipeline slots and shared memory, with the set-up
+ * autotuner's timing of every candidate when it ran (a shape already tuned in
+ * this process reuses the choice), and the projection's stage; for the plain
+ * form, the output rows a thread of each direction's gathers (4 to 8, timed
+ * the same way).  No reference counterpart (the
  * reference has one fixed kernel configuration per block width,
  * cuda/cyclic_cuda_helpers.h:552-631). */
 BW_API int bw_koszul_plan(const bw_koszul* ctx, char* buf, size_t cap);
