@@ -176,7 +176,6 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
     // the warp index through a shuffle, so that role and pass branches are uniform
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0), lane = threadIdx.x % 32;
     const long long n_tiles = P.n_tiles;
-    pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.slots; ++s) {
             tc::mbar_init(&full[s], W::producers / P.groups * 32);   // per thread: its copies have landed
@@ -201,6 +200,9 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
+    // Only now may the next kernel begin: one that shares the SM could otherwise
+    // take TMEM that this CTA still waits for, and then wait for this kernel.
+    pdl_trigger();
     const uint32_t tmem = *tmem_slot;
     const uint32_t stage0 = __ldg(P.start + blockIdx.x);
     const int n_stages = static_cast<int>(__ldg(P.start + blockIdx.x + 1) - stage0);
