@@ -856,6 +856,10 @@ void CyclicCtx::generate(size_t nlen_target, float* device_ms) {
     // source is written by the backward kernels of the application before
     if (subset_path && rounds > 0) subset_source16(d_b, d_dc);
     if (rounds > 0) {
+        if (subset_path && !rounds_checked) {
+            rounds_checked = true;
+            setup_rounds();
+        }
         if (!persistent && !graphs[0]) {
             const uint64_t l0 = launches;
             cudaGraph_t graph;

@@ -143,7 +143,7 @@ struct CyclicCtx {
     size_t seq_alloc = 0, seq_capacity = 0, seq_len = 0;
     cudaGraphExec_t graphs[1] = {nullptr};
     // whole rounds in one cooperative launch (small sectors; bw_cyclic_subset.cu)
-    bool persistent = false;
+    bool rounds_checked = false, persistent = false;
     unsigned rounds_grid = 0;
     int rounds_threads = 0, rounds_hold = 0;
     size_t rounds_smem = 0;

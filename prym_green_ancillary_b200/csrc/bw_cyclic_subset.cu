@@ -1045,14 +1045,14 @@ void CyclicCtx::setup_subset_path() {
     BW_CUDA(cudaMemsetAsync(d_t16, 0, (D.n1 + 1) * sizeof(uint4), stream));
     BW_CUDA(cudaMemsetAsync(d_u2_16, 0, (D.n2 + 1) * sizeof(uint4), stream));
     subset_path = true;
-    setup_rounds();
 }
 
 // Whether generate() runs whole rounds in one cooperative launch
 // (sub_rounds_kernel): the eliminated operator with two row-mixing rounds,
 // every subset with a thread of its own in one CTA an SM, and the tables in
 // shared memory (the published genera up to 22).  BW_CYCLIC_PERSISTENT=0 turns
-// it off.
+// it off.  Settled by the first generate(): loading the kernel in open() made
+// that 3 ms longer.
 void CyclicCtx::setup_rounds() {
     if (const char* env = std::getenv("BW_CYCLIC_PERSISTENT"))
         if (std::string(env) == "0") return;
