@@ -1204,6 +1204,44 @@ void tune_store(const TuneKey& k, const TuneChoice& c) {
     g_tune_cache[k] = c;
 }
 
+// Error words: contexts alive at the same time share mapped allocations of 64
+// words each (allocating one took a small context a fifth of its set-up); one
+// goes back with its last word.
+struct ErrorPage {
+    int* words;
+    uint64_t used;
+};
+std::mutex g_error_mutex;
+std::vector<ErrorPage> g_error_pages;
+
+volatile int* error_word_acquire() {
+    std::lock_guard<std::mutex> lock(g_error_mutex);
+    auto at = std::find_if(g_error_pages.begin(), g_error_pages.end(), [](const ErrorPage& g) { return ~g.used != 0; });
+    if (at == g_error_pages.end()) {
+        void* p = nullptr;
+        g_error_pages.reserve(g_error_pages.size() + 1);
+        BW_CUDA(cudaHostAlloc(&p, 64 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+        g_error_pages.push_back({static_cast<int*>(p), 0});
+        at = g_error_pages.end() - 1;
+    }
+    const int bit = __builtin_ctzll(~at->used);
+    at->used |= 1ull << bit;
+    return at->words + bit;
+}
+
+void error_word_release(volatile int* word) {
+    std::lock_guard<std::mutex> lock(g_error_mutex);
+    for (auto at = g_error_pages.begin(); at != g_error_pages.end(); ++at) {
+        if (word < at->words || word >= at->words + 64) continue;
+        at->used &= ~(1ull << (word - at->words));
+        if (at->used == 0) {
+            cudaFreeHost(at->words);
+            g_error_pages.erase(at);
+        }
+        return;
+    }
+}
+
 // Plans one direction: stage size, pipeline depth, B operand (host layout).
 //
 // A generator spans `inner_pad` K' rows (inner, rounded up to even for the TMA
@@ -1652,7 +1690,7 @@ void launch_i8(KoszulCtx& c, KoszulCtx::I8State::Dir& D, const CUtensorMap* maps
 }  // namespace
 
 void KoszulCtx::i8_destroy() {
-    if (i8 != nullptr && i8->h_err != nullptr) cudaFreeHost(const_cast<int*>(i8->h_err));
+    if (i8 != nullptr && i8->h_err != nullptr) error_word_release(i8->h_err);
     delete i8;
     i8 = nullptr;
 }
@@ -1679,11 +1717,9 @@ void KoszulCtx::i8_setup() {
             S.planes[b][limb + 2] = pair + plane;
         }
     }
-    void* word = nullptr;
-    BW_CUDA(cudaHostAlloc(&word, sizeof(int), cudaHostAllocMapped));
-    S.h_err = static_cast<volatile int*>(word);
+    S.h_err = error_word_acquire();
     *S.h_err = 0;
-    BW_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&S.err), word, 0));
+    BW_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&S.err), const_cast<int*>(S.h_err), 0));
     plan_projection(*this, S);
     const int hg = nbi / 16;
     // The producers that may be used.  BW_I8_PRODUCER=union, =cpasync or
