@@ -5,8 +5,11 @@
 // hi in [-64, 64] (|x| <= 16383 = 255 * 64 + 63).  The symmetric range makes negation exact in int8, which
 // is how the Koszul signs are applied while operands are staged.
 //
-// One gather-GEMM kernel serves both d and d^T.  For a tile of 128/n output
-// blocks (n = block width) the output is
+// d and d^T are one gather-GEMM.  bw_koszul_i8_union.cuh has the kernel that runs
+// it wherever its resident maps leave room for stages; this file has the dense
+// kernels for the other sizes (described here), the conversions, the projection
+// and the host side of both.  For a tile of 128/n output blocks (n = block width)
+// the output is
 //   out[blk][o][j] = sum_{i < r} sum_{u < inner} A[(blk, j)][(i, u)] * Bm[o][(i, u)]
 // with A[(blk, j)][(i, u)] = sign * in[nbr(blk, i)][u][j] (zero when the
 // generator i is not incident to blk) and Bm = the r maps side by side.  The
