@@ -432,10 +432,10 @@ void KoszulCtx::step_once(cudaStream_t st, bool after_step) {
 
 KoszulCtx::~KoszulCtx() {
     cudaSetDevice(device);
-    i8_destroy();
     for (auto& g : graphs)
         if (g) cudaGraphExecDestroy(g);
-    for (auto& a : allocations) cudaFree(a.first);
+    for (auto& a : allocations) cudaFree(a.first);   // waits for the kernels that a session left in flight
+    i8_destroy();   // only then: the error word goes back to the pool, and such a kernel may still write it
     if (ev_join) cudaEventDestroy(ev_join);
     if (own_stream) cudaStreamDestroy(own_stream);
 }
