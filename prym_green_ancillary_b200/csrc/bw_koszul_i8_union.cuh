@@ -320,6 +320,9 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
             uint32_t parity = static_cast<uint32_t>(issuer / P.slots) & 1u;
             uint32_t a_lo = a_slot0 + static_cast<uint32_t>(slot) * slot_units;
             const bool ok = tc::warp_wait(tc::smem_u32(maps_in), 0, nullptr, P.err, tc::ERR_WAIT_FINAL);
+            // The producers fill nothing before the kernel before this one is done:
+            // the limit of the waits below is for this kernel's own work.
+            if (!P.late_wait) pdl_wait();
             // failure tests: CTA 0 waits for its first stage on a barrier that
             // nothing completes before the final drain, so the wait runs out
             const bool held = P.hold_first_stage && blockIdx.x == 0 && issuer == 0 && ok &&
