@@ -557,7 +557,7 @@ __device__ __forceinline__ void cta_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 __device__ __forceinline__ bool grid_barrier(const RoundsArgs& A, unsigned int count, int id, int threads,
-                                             volatile int* gave_up /* shared */) {
+                                             volatile unsigned int* gave_up) {
     cta_sync(id, threads);
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(A.arrivals) : "memory");
@@ -567,7 +567,7 @@ __device__ __forceinline__ bool grid_barrier(const RoundsArgs& A, unsigned int c
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(A.arrivals) : "memory");
         } while (v < target && ++tries < A.wait_limit);
         if (v < target) {
-            *gave_up = 1;
+            *gave_up = count;
             *reinterpret_cast<volatile int*>(A.err) = 1;
         }
     }
@@ -575,11 +575,16 @@ __device__ __forceinline__ bool grid_barrier(const RoundsArgs& A, unsigned int c
     return *gave_up == 0;
 }
 
-// The part in it of threads that only wait for the CTA's polling threads.
-__device__ __forceinline__ bool grid_barrier_join(volatile int* gave_up, int all) {
+// The part in the `count`-th of threads that only wait for the CTA's polling
+// thread.  That thread may have run into a later barrier, and given it up,
+// before they read the word: they take that for what it is then and go on to
+// the next barrier they join, where the CTA's other threads meet them.  (Were
+// some to leave at once and others not, those would wait there for good.)
+__device__ __forceinline__ bool grid_barrier_join(unsigned int count, volatile unsigned int* gave_up, int all) {
     cta_sync(0, all);
     cta_sync(0, all);
-    return *gave_up == 0;
+    const unsigned int at = *gave_up;
+    return at == 0 || at > count;
 }
 
 __device__ __forceinline__ int tri(int row, int col) { return row * (2 * 4 - row + 1) / 2 + (col - row); }
@@ -654,7 +659,7 @@ __device__ __forceinline__ void gather_resident(const uint32_t* words, int strid
 template <bool SMALL>
 __global__ void __launch_bounds__(kResidentThreads, 1) sub_rounds_kernel(SubsetDev D, RoundsArgs A) {
     extern __shared__ int32_t sm[];
-    __shared__ int gave_up;
+    __shared__ unsigned int gave_up;   // number of the barrier that the CTA gave up at, or 0
     const int all = blockDim.x, T = all - kMomentThreads, tid = threadIdx.x;
     const int blob4 = (D.blob_words + 3) / 4 * 4;
     for (int w = tid; w < D.blob_words; w += all) {
@@ -670,10 +675,10 @@ __global__ void __launch_bounds__(kResidentThreads, 1) sub_rounds_kernel(SubsetD
         __syncthreads();
         for (int app = 0; app < 2 * A.rounds; ++app) {
             if (app > 0) add_moments(A, (app & 1) == 0, D.mod, tid - T);
-            if (!grid_barrier_join(&gave_up, all) || !grid_barrier_join(&gave_up, all)) return;
+            if (!grid_barrier_join(5u * app + 3, &gave_up, all) || !grid_barrier_join(5u * app + 5, &gave_up, all)) return;
         }
         add_moments(A, true, D.mod, tid - T);
-        grid_barrier_join(&gave_up, all);
+        grid_barrier_join(10u * A.rounds + 1, &gave_up, all);
         return;
     }
     const uint32_t id = blockIdx.x * static_cast<uint32_t>(T) + tid;
@@ -756,7 +761,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) sub_rounds_kernel(SubsetD
     // (a give-up there lets the moments' threads out of the barrier they wait at)
     auto subset_barrier = [&] {
         if (grid_barrier(A, ++met, 1, T, &gave_up)) return true;
-        grid_barrier_join(&gave_up, all);
+        grid_barrier_join(met, &gave_up, all);
         return false;
     };
     auto full_barrier = [&] { return grid_barrier(A, ++met, 0, all, &gave_up); };
