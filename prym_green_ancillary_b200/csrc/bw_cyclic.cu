@@ -906,8 +906,9 @@ void CyclicCtx::generate(size_t nlen_target, float* device_ms) {
     BW_CUDA(cudaStreamSynchronize(stream));
     if (err != 0) {
         seq_len = 0;
-        BW_CUDA(cudaMemset(d_err, 0, sizeof(int)));
-        BW_CUDA(cudaMemset(d_partials, 0, 20 * sizeof(int32_t)));
+        // on the context's stream, which the legacy stream's work is not ordered with
+        BW_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), stream));
+        BW_CUDA(cudaMemsetAsync(d_partials, 0, 20 * sizeof(int32_t), stream));
         throw Error("the sequence's kernel gave up waiting (grid barrier between its phases)", 2);
     }
 }
