@@ -174,7 +174,7 @@ __device__ __forceinline__ void gather_block(const uint32_t* __restrict__ inc, u
 __global__ void __launch_bounds__(kThreads) sub_source_kernel(SubsetDev D, const int32_t* __restrict__ in,
                                                               const int32_t* __restrict__ dc, uint4* __restrict__ xs,
                                                               int32_t* __restrict__ zs) {
-    extern __shared__ int32_t sm[];
+    extern __shared__ __align__(16) int32_t sm[];
     const Tables T = stage(D, D.blob_f, sm);
     const long long n0 = D.n0, total = n0 + static_cast<long long>(D.z_cols) + D.n_extra;
     BW_ITEMS(item, total) {
@@ -211,7 +211,7 @@ template <bool SMALL, bool STREAM>
 __global__ void __launch_bounds__(kThreads) sub_dm_forward_elim_kernel(SubsetDev D, const uint4* __restrict__ xs,
                                                                        const int32_t* __restrict__ zs,
                                                                        uint4* __restrict__ y) {
-    extern __shared__ int32_t sm[];
+    extern __shared__ __align__(16) int32_t sm[];
     const Tables T = stage(D, D.blob_f, sm);
     BW_ITEMS(item, D.n1) {
         const uint32_t s = static_cast<uint32_t>(item);
@@ -258,7 +258,7 @@ template <bool SMALL, bool STREAM>
 __global__ void __launch_bounds__(kThreads) sub_d2_forward_kernel(SubsetDev D, const uint4* __restrict__ y,
                                                                   const int32_t* __restrict__ zs,
                                                                   uint2* __restrict__ u) {
-    extern __shared__ int32_t sm[];
+    extern __shared__ __align__(16) int32_t sm[];
     const Tables T = stage(D, D.blob_f, sm);
     BW_ITEMS(item, D.n2) {
         const uint32_t s = static_cast<uint32_t>(item);
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(kThreads) sub_d2_transpose_adjoint_kernel(Subs
                                                                             uint4* __restrict__ t_adj,
                                                                             int32_t* __restrict__ out,
                                                                             int32_t* __restrict__ next_zs) {
-    extern __shared__ int32_t sm[];
+    extern __shared__ __align__(16) int32_t sm[];
     const Tables T = stage(D, D.blob_t, sm);
     BW_ITEMS(item, D.n1) {
         const uint32_t s = static_cast<uint32_t>(item);
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kThreads) sub_dm_transpose_kernel(SubsetDev D,
                                                                     const int32_t* __restrict__ dc,
                                                                     int32_t* __restrict__ out,
                                                                     uint4* __restrict__ next_xs) {
-    extern __shared__ int32_t sm[];
+    extern __shared__ __align__(16) int32_t sm[];
     const Tables T = stage(D, D.blob_t, sm);
     BW_ITEMS(item, D.n0) {
         const uint32_t s = static_cast<uint32_t>(item);
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(kThreads) sub_dense_t_kernel(SubsetDev D, cons
                                                                int32_t* __restrict__ partials,
                                                                unsigned int* __restrict__ counter,
                                                                int32_t* __restrict__ next_zs) {
-    extern __shared__ int32_t sm[];
+    extern __shared__ __align__(16) int32_t sm[];
     const Tables T = stage(D, D.blob_f, sm);
     int32_t acc[8];
 #pragma unroll
@@ -658,7 +658,7 @@ __device__ __forceinline__ void gather_resident(const uint32_t* words, int strid
 // threads that took 3.5 us an application).
 template <bool SMALL>
 __global__ void __launch_bounds__(kResidentThreads, 1) sub_rounds_kernel(SubsetDev D, RoundsArgs A) {
-    extern __shared__ int32_t sm[];
+    extern __shared__ __align__(16) int32_t sm[];
     __shared__ unsigned int gave_up;   // number of the barrier that the CTA gave up at, or 0
     const int all = blockDim.x, T = all - kMomentThreads, tid = threadIdx.x;
     const int blob4 = (D.blob_words + 3) / 4 * 4;
@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) sub_rounds_kernel(SubsetD
 // non-hot entry points (backward / target_precondition on compact vectors).
 __global__ void __launch_bounds__(kThreads) sub_u_pack_kernel(SubsetDev D, const int32_t* __restrict__ u32,
                                                               uint4* __restrict__ u16) {
-    extern __shared__ int32_t sm[];
+    extern __shared__ __align__(16) int32_t sm[];
     const Tables T = stage(D, D.blob_f, sm);
     BW_ITEMS(item, D.n2) {
         const uint32_t d = __ldg(D.m2 + item);
@@ -868,7 +868,7 @@ __global__ void __launch_bounds__(kThreads) sub_u_pack_kernel(SubsetDev D, const
 }
 __global__ void __launch_bounds__(kThreads) sub_u_unpack_kernel(SubsetDev D, const uint4* __restrict__ u16,
                                                                 int32_t* __restrict__ u32) {
-    extern __shared__ int32_t sm[];
+    extern __shared__ __align__(16) int32_t sm[];
     const Tables T = stage(D, D.blob_f, sm);
     BW_ITEMS(item, D.n2) {
         const uint32_t d = __ldg(D.m2 + item);
