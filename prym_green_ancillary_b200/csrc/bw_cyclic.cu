@@ -19,7 +19,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <system_error>
 #include <thread>
 #include <iostream>
 
@@ -918,6 +917,25 @@ uint32_t* CyclicCtx::scratch_canonical() {
     return d_canon;
 }
 
+// Makes up to `count` lanes of copy_out; the number there are.
+size_t CyclicCtx::make_out_lanes(size_t count, size_t chunk) {
+    out_lanes.reserve(count);
+    while (out_lanes.size() < count) {
+        OutLane lane;
+        if (cudaHostAlloc(&lane.pinned, chunk, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();   // not an error of the call: fewer lanes, or none, do as well
+            break;
+        }
+        if (cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFreeHost(lane.pinned);
+            break;
+        }
+        out_lanes.push_back(lane);
+    }
+    return out_lanes.size();
+}
+
 // Device to pageable host memory.  A large block goes through a few pinned
 // chunks, each with a host thread and a stream of its own: the time is in
 // writing (and first touching) the destination's pages, which the threads
@@ -925,21 +943,14 @@ uint32_t* CyclicCtx::scratch_canonical() {
 void CyclicCtx::copy_out(void* dst, const void* src, size_t bytes) {
     constexpr size_t kChunk = size_t{1} << 18;
     const size_t chunks = (bytes + kChunk - 1) / kChunk;
-    const size_t workers = std::min<size_t>({4, std::max(1u, std::thread::hardware_concurrency()), chunks / 2});
-    if (workers < 2) {
+    size_t workers = std::min<size_t>({4, std::max(1u, std::thread::hardware_concurrency()), chunks / 2});
+    if (workers >= 2) workers = std::min(workers, make_out_lanes(workers, kChunk));
+    if (workers < 2) {   // a small block, or no pinned memory to be had
         BW_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream));
         BW_CUDA(cudaStreamSynchronize(stream));
         return;
     }
     BW_CUDA(cudaStreamSynchronize(stream));   // src is complete
-    while (out_lanes.size() < workers) {
-        OutLane lane;
-        BW_CUDA(cudaHostAlloc(&lane.pinned, kChunk, cudaHostAllocDefault));
-        const cudaError_t made = cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking);
-        if (made != cudaSuccess) cudaFreeHost(lane.pinned);
-        BW_CUDA(made);
-        out_lanes.push_back(lane);
-    }
     std::vector<cudaError_t> result(workers, cudaSuccess);
     auto run = [&](size_t w) {
         const OutLane& lane = out_lanes[w];
@@ -953,10 +964,11 @@ void CyclicCtx::copy_out(void* dst, const void* src, size_t bytes) {
         result[w] = e;
     };
     std::vector<std::thread> pool;
+    pool.reserve(workers);   // nothing but the start of a thread may fail below
     size_t started = 1;
     try {
         for (; started < workers; ++started) pool.emplace_back(run, started);
-    } catch (const std::system_error&) {   // no more threads: the caller does the rest
+    } catch (const std::exception&) {   // no more threads: the caller does the rest
     }
     run(0);
     for (size_t w = started; w < workers; ++w) run(w);

@@ -211,6 +211,7 @@ struct CyclicCtx {
         cudaStream_t stream = nullptr;
     };
     std::vector<OutLane> out_lanes;       // copy_out's pinned chunks and streams (first large download)
+    size_t make_out_lanes(size_t count, size_t chunk);
     void copy_out(void* dst, const void* src, size_t bytes);
     void download_into(uint32_t* current, uint32_t* packed);   // host buffers, either may be null
     void download_state(std::vector<uint32_t>& current, std::vector<uint32_t>& packed);
