@@ -1726,13 +1726,21 @@ void KoszulCtx::i8_setup() {
     plan_projection(*this, S);
     const int hg = nbi / 16;
     // The producers that may be used.  BW_I8_PRODUCER=union, =cpasync or
-    // =hybrid restricts the choice to one.
-    bool allow_union = true, allow_g4 = true, allow_cp = true, tune = true;
+    // =hybrid restricts the choice to one, two of them with a comma between d's
+    // and d^T's to one each.
+    struct {
+        bool uni = true, g4 = true, cp = true;
+    } allow[2];
+    bool tune = true;
     if (const char* e = std::getenv("BW_I8_PRODUCER")) {
-        const std::string want = e;
-        allow_union = want != "cpasync" && want != "hybrid";
-        allow_g4 = want != "cpasync" && want != "union";
-        allow_cp = want != "hybrid" && want != "union";
+        const std::string text = e;
+        const size_t comma = text.find(',');
+        for (int dir = 0; dir < 2; ++dir) {
+            const std::string want =
+                comma == std::string::npos ? text : dir == 0 ? text.substr(0, comma) : text.substr(comma + 1);
+            allow[dir] = {want != "cpasync" && want != "hybrid", want != "cpasync" && want != "union",
+                          want != "hybrid" && want != "union"};
+        }
     }
     if (const char* e = std::getenv("BW_I8_TUNE")) tune = std::string(e) != "0";
     // BW_I8_PRODUCER_WARPS=8 or =16 restricts the cp.async producers' warp count
@@ -1766,15 +1774,15 @@ void KoszulCtx::i8_setup() {
         for (int g : {4, 3, 6, 8, 2}) {
             for (int groups : {2, 4})
                 for (int issuers : {2, 1})
-                    if (allow_union && plan_union(*this, D, inner, outer, dir == 1, g, groups, issuers)) {
+                    if (allow[dir].uni && plan_union(*this, D, inner, outer, dir == 1, g, groups, issuers)) {
                         cands[dir].push_back({2, g, groups, 8, issuers});
                         in_flight = std::max(in_flight, D.u.slots * g);
                     }
         }
-        const bool dense = (allow_g4 || allow_cp) && in_flight < 8;
+        const bool dense = (allow[dir].g4 || allow[dir].cp) && in_flight < 8;
         BW_REQUIRE(!cands[dir].empty() || dense, "INT8 form: no union plan fits in shared memory");
         if (dense) {
-            if (allow_cp)
+            if (allow[dir].cp)
                 // the fill heuristic's stage, and fewer or more generators a stage
                 // (smaller stages leave room for more pipeline slots)
                 for (int pw : pws) {
@@ -1782,13 +1790,13 @@ void KoszulCtx::i8_setup() {
                     for (int g : {4, 6, 8, 12})
                         if (g < r) cands[dir].push_back({0, g, 0, pw, 1});
                 }
-            if (allow_g4)
+            if (allow[dir].g4)
                 for (int gs = 1; gs <= std::min(3, (r + 3) / 4); ++gs)
                     for (int qt = 1; qt <= 3; ++qt) cands[dir].push_back({1, 4 * gs, qt * bt / 4, 8, 1});
         }
         keys[dir] = TuneKey{r, k, inner, outer, nbi, dir, sms,
-                            (allow_g4 ? 1 : 0) | (allow_cp ? 2 : 0) | (pws.size() == 1 ? pws[0] * 4 : 0) |
-                                (allow_union ? 128 : 0)};
+                            (allow[dir].g4 ? 1 : 0) | (allow[dir].cp ? 2 : 0) | (pws.size() == 1 ? pws[0] * 4 : 0) |
+                                (allow[dir].uni ? 128 : 0)};
         TuneChoice known{};
         // a shape tuned earlier in this process: its choice alone
         if (tune && tune_lookup(keys[dir], known))
