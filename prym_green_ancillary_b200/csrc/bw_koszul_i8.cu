@@ -1170,6 +1170,7 @@ struct KoszulCtx::I8State {
     unsigned proj_grid = 0;
     int* err = nullptr;        // the kernels' error word (device address)
     volatile int* h_err = nullptr;   // the same word: mapped host memory, written only when a kernel gives up
+    unsigned long long err_context = 0;   // the CUDA context that the word's page belongs to
 };
 
 namespace {
@@ -1207,24 +1208,47 @@ void tune_store(const TuneKey& k, const TuneChoice& c) {
     g_tune_cache[k] = c;
 }
 
-// Error words: contexts alive at the same time share mapped allocations of 64
-// words each (allocating one took a small context a fifth of its set-up); one
-// goes back with its last word.
+// Error words: engine contexts alive at the same time share mapped allocations
+// of 64 words each (allocating one took a small context a fifth of its set-up);
+// one goes back with its last word.  A page belongs to the CUDA context that it
+// was allocated in and serves only that one: cudaDeviceReset, which an engine
+// context may outlive, takes the memory of the device's pages with it.
 struct ErrorPage {
+    unsigned long long context;   // id of the CUDA context (never used again in the process)
     int* words;
     uint64_t used;
 };
 std::mutex g_error_mutex;
 std::vector<ErrorPage> g_error_pages;
 
-volatile int* error_word_acquire() {
+// Id of the calling thread's current CUDA context, 0 without one.
+unsigned long long current_context_id() {
+    using GetIdFn = CUresult (*)(CUcontext, unsigned long long*);
+    static const GetIdFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<GetIdFn>(f);
+    }();
+    unsigned long long id = 0;
+    if (fn == nullptr || fn(nullptr, &id) != CUDA_SUCCESS) return 0;
+    return id;
+}
+
+// A word of the current CUDA context's pages; `context` receives its id.
+volatile int* error_word_acquire(unsigned long long& context) {
+    context = current_context_id();
+    BW_REQUIRE(context != 0, "INT8 form: no current CUDA context");
     std::lock_guard<std::mutex> lock(g_error_mutex);
-    auto at = std::find_if(g_error_pages.begin(), g_error_pages.end(), [](const ErrorPage& g) { return ~g.used != 0; });
+    auto at = std::find_if(g_error_pages.begin(), g_error_pages.end(),
+                           [&](const ErrorPage& g) { return g.context == context && ~g.used != 0; });
     if (at == g_error_pages.end()) {
         void* p = nullptr;
         g_error_pages.reserve(g_error_pages.size() + 1);
-        BW_CUDA(cudaHostAlloc(&p, 64 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
-        g_error_pages.push_back({static_cast<int*>(p), 0});
+        BW_CUDA(cudaHostAlloc(&p, 64 * sizeof(int), cudaHostAllocMapped));
+        g_error_pages.push_back({context, static_cast<int*>(p), 0});
         at = g_error_pages.end() - 1;
     }
     const int bit = __builtin_ctzll(~at->used);
@@ -1232,13 +1256,13 @@ volatile int* error_word_acquire() {
     return at->words + bit;
 }
 
-void error_word_release(volatile int* word) {
+void error_word_release(volatile int* word, unsigned long long context) {
     std::lock_guard<std::mutex> lock(g_error_mutex);
     for (auto at = g_error_pages.begin(); at != g_error_pages.end(); ++at) {
-        if (word < at->words || word >= at->words + 64) continue;
+        if (at->context != context || word < at->words || word >= at->words + 64) continue;
         at->used &= ~(1ull << (word - at->words));
         if (at->used == 0) {
-            cudaFreeHost(at->words);
+            if (current_context_id() == context) cudaFreeHost(at->words);   // else it went with its CUDA context
             g_error_pages.erase(at);
         }
         return;
@@ -1693,7 +1717,7 @@ void launch_i8(KoszulCtx& c, KoszulCtx::I8State::Dir& D, const CUtensorMap* maps
 }  // namespace
 
 void KoszulCtx::i8_destroy() {
-    if (i8 != nullptr && i8->h_err != nullptr) error_word_release(i8->h_err);
+    if (i8 != nullptr && i8->h_err != nullptr) error_word_release(i8->h_err, i8->err_context);
     delete i8;
     i8 = nullptr;
 }
@@ -1720,7 +1744,7 @@ void KoszulCtx::i8_setup() {
             S.planes[b][limb + 2] = pair + plane;
         }
     }
-    S.h_err = error_word_acquire();
+    S.h_err = error_word_acquire(S.err_context);
     *S.h_err = 0;
     BW_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&S.err), const_cast<int*>(S.h_err), 0));
     plan_projection(*this, S);
