@@ -32,28 +32,6 @@ uint64_t binom(int n, int k) {
     return binom_table().c[n][k];
 }
 
-uint64_t lex_rank(const int* s, int r, int k) {
-    uint64_t acc = 0;
-    for (int pos = 0; pos < k; ++pos) acc += binom(r - 1 - s[pos], k - pos);
-    return binom(r, k) - 1 - acc;
-}
-
-void lex_unrank(uint64_t rank, int r, int k, int* out) {
-    int start = 0;
-    for (int pos = 0; pos < k; ++pos) {
-        int remaining = k - pos - 1;
-        for (int v = start; v < r; ++v) {
-            uint64_t cnt = binom(r - v - 1, remaining);
-            if (rank < cnt) {
-                out[pos] = v;
-                start = v + 1;
-                break;
-            }
-            rank -= cnt;
-        }
-    }
-}
-
 int sm_count(int device) {
     int n = 0;
     BW_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device));

@@ -1,6 +1,6 @@
 // Shared helpers of the B200 block-Wiedemann engine: error plumbing, modular
-// arithmetic on balanced residues, the counter-based seeded stream and the
-// lexicographic subset ranking used by every Koszul table.
+// arithmetic on balanced residues, programmatic dependent launch, the
+// counter-based seeded stream and binomial coefficients.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -249,13 +249,6 @@ enum SeedTag : uint32_t { TAG_MAPS = 1, TAG_DIAG = 2, TAG_X = 3, TAG_Y = 4 };
 
 // Binomial coefficients C(n, k) for n, k <= 64 (host table).
 uint64_t binom(int n, int k);
-
-// Lexicographic rank of a sorted k-subset of {0..r-1}:
-// rank = C(r,k) - 1 - sum_pos C(r-1-s_pos, k-pos).
-uint64_t lex_rank(const int* s, int r, int k);
-
-// Unrank (lexicographic, itertools.combinations order).
-void lex_unrank(uint64_t rank, int r, int k, int* out);
 
 // ------------------------------------------------------------- device info
 

@@ -283,8 +283,6 @@ __global__ void cyc_rowmix_kernel(const uint32_t* __restrict__ pairs, long long 
     }
 }
 
-__device__ __forceinline__ int tri_index(int row, int col) { return row * (2 * 4 - row + 1) / 2 + (col - row); }
-
 // Gram moments of one half-round: B^t D and (count == 2) O^t O, where O is the
 // newer of the two, upper triangles packed into seq at positions *seq_index
 // (+1), canonical.
@@ -297,8 +295,8 @@ __global__ void __launch_bounds__(kThreads, 4) cyc_gram_kernel(
     const int32_t* __restrict__ B, const int32_t* __restrict__ D, int b_is_newer, int count, long long rows,
     int32_t* __restrict__ partials, unsigned int* __restrict__ counter, uint32_t* __restrict__ seq,
     unsigned long long* __restrict__ seq_index, Mod mod) {
-    cyc::pdl_trigger();
-    cyc::pdl_wait();
+    pdl_trigger();
+    pdl_wait();
     int32_t acc[20];
 #pragma unroll
     for (int e = 0; e < 20; ++e) acc[e] = 0;
@@ -309,8 +307,8 @@ __global__ void __launch_bounds__(kThreads, 4) cyc_gram_kernel(
         for (int r0 = 0; r0 < 4; ++r0)
 #pragma unroll
             for (int c0 = r0; c0 < 4; ++c0) {
-                acc[tri_index(r0, c0)] += bv[r0] * dv[c0];
-                acc[10 + tri_index(r0, c0)] += ov[r0] * ov[c0];
+                acc[cyc::tri_index(r0, c0)] += bv[r0] * dv[c0];
+                acc[10 + cyc::tri_index(r0, c0)] += ov[r0] * ov[c0];
             }
     };
     // four rows in flight, eight products beside a partially reduced sum

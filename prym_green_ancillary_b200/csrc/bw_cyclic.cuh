@@ -169,7 +169,7 @@ struct CyclicCtx {
 
     // Launches a kernel of 256-thread CTAs on the context's stream, as a
     // programmatic dependent launch when `pdl` is set (the kernel must call
-    // cyc::pdl_wait() before touching data of the kernels before it).
+    // pdl_wait() before touching data of the kernels before it).
     template <class... P, class... A>
     void launch_pdl(void (*kernel)(P...), unsigned grid, size_t smem, A&&... args) {
         cudaLaunchConfig_t cfg{};

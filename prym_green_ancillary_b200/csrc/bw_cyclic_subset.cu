@@ -89,10 +89,10 @@ __device__ __forceinline__ Tables views(const SubsetDev& D, const int32_t* sm) {
 // Staging reads only the constant tables, so it overlaps the end of the kernel
 // before (programmatic dependent launch); the wait follows it.
 __device__ __forceinline__ Tables stage(const SubsetDev& D, const int32_t* __restrict__ blob, int32_t* sm) {
-    cyc::pdl_trigger();
+    pdl_trigger();
     for (int w = threadIdx.x; w < D.blob_words; w += blockDim.x) sm[w] = __ldg(blob + w);
     __syncthreads();
-    cyc::pdl_wait();
+    pdl_wait();
     return views(D, sm);
 }
 
@@ -311,8 +311,8 @@ template <bool SMALL, bool STREAM, bool SIX>
 __global__ void __launch_bounds__(kThreads, 4) sub_ell_kernel(SubsetDev D, const uint2* __restrict__ u,
                                                            uint2* __restrict__ u2) {
     constexpr int U = SIX ? 6 : 4;
-    cyc::pdl_trigger();
-    cyc::pdl_wait();
+    pdl_trigger();
+    pdl_wait();
     const long long rows = 2 * static_cast<long long>(D.n2);
     BW_ITEMS(row, rows) {
         Acc4<SMALL> acc;
@@ -587,8 +587,6 @@ __device__ __forceinline__ bool grid_barrier_join(unsigned int count, volatile u
     return at == 0 || at > count;
 }
 
-__device__ __forceinline__ int tri(int row, int col) { return row * (2 * 4 - row + 1) / 2 + (col - row); }
-
 // Adds the packed upper triangles of B^t D and O^t O (O: the newer of the two)
 // over all rows to A.sums, by the kMomentThreads threads that call it in every
 // CTA (t: the thread's number among them).
@@ -606,8 +604,8 @@ __device__ __forceinline__ void add_moments(const RoundsArgs& A, bool b_is_newer
         for (int r0 = 0; r0 < 4; ++r0)
 #pragma unroll
             for (int c0 = r0; c0 < 4; ++c0) {
-                acc[tri(r0, c0)] += bv[r0] * dv[c0];
-                acc[10 + tri(r0, c0)] += ov[r0] * ov[c0];
+                acc[cyc::tri_index(r0, c0)] += bv[r0] * dv[c0];
+                acc[10 + cyc::tri_index(r0, c0)] += ov[r0] * ov[c0];
             }
         if (++cnt == 8) {
             cnt = 0;

@@ -98,11 +98,6 @@ __device__ __forceinline__ void transpose16(uint32_t (&w)[4], int lane) {
     }
 }
 
-// Byte offset of element (row = blk * dim + u, column j) in a plane of width NB.
-__host__ __device__ __forceinline__ long long plane_offset(long long blk, int u, int j, int dim, int NB) {
-    return blk * (static_cast<long long>(NB) * dim) + static_cast<long long>(j >> 4) * dim * 16 + u * 16 + (j & 15);
-}
-
 }  // namespace
 
 }  // namespace bw

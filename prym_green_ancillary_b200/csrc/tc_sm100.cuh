@@ -140,12 +140,8 @@ __device__ __forceinline__ void prefetch_tmap(const void* tmap) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }
 
-// 16-byte asynchronous copy global -> shared through L2 (cp.async.cg).
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
-// 16-byte cp.async that reads src_size (0 or 16) bytes and zero-fills the rest:
+// 16-byte asynchronous copy global -> shared through L2 (cp.async.cg) that reads
+// src_size (0 or 16) bytes and zero-fills the rest:
 // src_size 0 writes 16 zero bytes without reading global memory.
 __device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, uint32_t src_size) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(src_size)
@@ -191,19 +187,10 @@ __device__ __forceinline__ void tc_fence_after() {
 
 // ---- descriptors
 // Shared-memory matrix descriptor, no swizzle: start address, leading-dimension
-// byte offset (LBO) and stride-dimension byte offset (SBO), version 1.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFFu);
-    d |= static_cast<uint64_t>((lbo >> 4) & 0x3FFFu) << 16;
-    d |= static_cast<uint64_t>((sbo >> 4) & 0x3FFFu) << 32;
-    d |= static_cast<uint64_t>(1) << 46;
-    return d;
-}
-
-// The same descriptor as two 32-bit words, so that a loop can advance the start
-// address by adding to the low word (the address field holds addr >> 4 in 14
-// bits; shared-memory addresses stay below 2^18, so the sum never carries out).
+// byte offset (LBO) and stride-dimension byte offset (SBO), version 1.  Two
+// 32-bit words, so that a loop can advance the start address by adding to the
+// low word (the address field holds addr >> 4 in 14 bits; shared-memory
+// addresses stay below 2^18, so the sum never carries out).
 __device__ __forceinline__ uint32_t desc_lo(uint32_t saddr, uint32_t lbo) {
     return ((saddr >> 4) & 0x3FFFu) | (((lbo >> 4) & 0x3FFFu) << 16);
 }
@@ -276,16 +263,6 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, int32_t (&r)[8]) {
                  : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ bool elect_one() {
-    uint32_t pred = 0;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xffffffff;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(pred));
-    return pred != 0;
-}
 
 }  // namespace tc
 }  // namespace bw
