@@ -173,6 +173,14 @@ __host__ __device__ __forceinline__ uint32_t to_canonical(int32_t balanced, cons
 // early.  Every kernel launched this way calls pdl_wait(), so a kernel's
 // completion implies that of all kernels before it.  Without the attribute
 // both are no-ops.
+//
+// One exception to the first access: the INT8 form's d inside a run of steps
+// (I8Union::late_wait) gathers what the kernel before the projection before it
+// wrote, and waits only at its end.  It begins once every CTA of the projection
+// has returned from its own pdl_wait(), hence after that writer's completion,
+// when the data is in L2; as it has not waited itself, nothing has been made
+// visible to it beyond L2, so it has to read that data there (cp.async.cg), not
+// through L1.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

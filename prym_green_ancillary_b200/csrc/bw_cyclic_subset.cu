@@ -540,7 +540,7 @@ struct RoundsArgs {
     uint32_t* seq;
     unsigned long long* seq_index;
     unsigned int* arrivals;       // of all CTAs at all barriers (zero at launch)
-    int* err;                     // mapped host memory, written only on a give-up
+    int* err;                     // written only on a give-up
     unsigned int wait_limit;
     int hold;                     // failure test: CTA 0 never arrives
     int rounds;

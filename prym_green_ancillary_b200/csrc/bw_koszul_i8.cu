@@ -1,9 +1,12 @@
 // INT8-limb tensor-core form of the synthetic Koszul operator (tcgen05 kind::i8).
 //
-// Every residue x (balanced, |x| <= (p-1)/2 < 2^14) is stored in HBM as two
-// signed 8-bit limbs in base 255:  x = 255*hi + lo,  lo in [-127, 127],
-// hi in [-64, 64] (|x| <= 16383 = 255 * 64 + 63).  The symmetric range makes negation exact in int8, which
-// is how the Koszul signs are applied while operands are staged.
+// Every residue x is stored in HBM as two signed 8-bit limbs in base 255:
+// x = 255*hi + lo, both in [-127, 127].  Inputs and maps are split from the
+// balanced residue (|x| <= (p-1)/2 <= 16383 = 255 * 64 + 63: hi in [-64, 64]);
+// the union kernel stores any representative that two limbs hold (|x| <= 255 *
+// 127 + 127), so what reads a stored block relies on 127 for either limb.  The
+// symmetric range makes negation exact in int8, which is how the Koszul signs
+// are applied while operands are staged.
 //
 // d and d^T are one gather-GEMM.  bw_koszul_i8_union.cuh has the kernel that runs
 // it wherever its resident maps leave room for stages; this file has the dense
@@ -1778,7 +1781,11 @@ void KoszulCtx::i8_setup() {
     // fewer than eight generators in flight (maps of 2 r inner rows: r * inner
     // * outer above about 32,000).  With more room the union kernel won at every
     // shape timed (us, dense against union: r=19 k=9 20->28 n=16 179/92 d and
-    // 228/127 d^T; r=21 k=10 32->40 n=32 1726/1050 and 2429/1260).
+    // 228/127 d^T; r=21 k=10 32->40 n=32 1726/1050 and 2429/1260), also where it
+    // pads most, at dims 1 to 16 (a step, dense / union: r=20 k=10 1->1 n=32
+    // 683/398, 4->5 921/448; r=16 k=8 1->1 n=16 34.6/27.4; r=31 k=5 1->1 n=16
+    // 158/149; r=31 k=28 1->1 n=16 40.4/35.7; 150 shapes, 1.06 to 2.0 times).  Its
+    // kernels alone are there within 15 % of the dense ones or faster.
     struct Cand {
         int kind;                        // 0 dense cp.async, 1 dense hybrid, 2 union
         int gps, t_tma, pw, issuers;     // as in TuneChoice

@@ -115,6 +115,7 @@ struct I8Union {
     Mod mod;
     uint32_t wait_limit;           // tries of every pipeline wait (tc::kWaitLimit outside the failure tests)
     int late_wait;                 // nothing here depends on the kernel before: wait for it at the end only
+                                   // (the input is then read at L2 alone, see pdl_wait())
     int hold_first_stage;          // failure tests only: CTA 0's MMA warp never sees its first stage
 };
 
@@ -265,6 +266,7 @@ __global__ void __launch_bounds__(union_warps::threads, 1) i8_union_gemm_kernel(
                     const uint32_t src16 = (present ? o16 : 0u) + (unit[j] & 127u);
                     const uint32_t nbytes = present ? 16u : 0u;
                     const uint32_t dst = slotA + (unit[j] >> 12) * 16u;
+                    // .cg: late_wait allows no read of the input through L1
                     tc::cp_async16_zfill(dst, P.in[0] + static_cast<size_t>(src16) * 16u, nbytes);
                     tc::cp_async16_zfill(dst + hi_rows, P.in[1] + static_cast<size_t>(src16) * 16u, nbytes);
                 }
