@@ -469,6 +469,8 @@ Fold plan_fold(uint32_t p) {
     return best;
 }
 
+constexpr size_t kPlainMapBytes = 200 * 1024;   // shared memory for the plain gathers' maps
+
 KoszulCtx* KoszulCtx::create(const bw_koszul_desc& d, int dev) {
     BW_REQUIRE(d.r >= 2 && d.r <= 31, "r must be in 2..31");
     BW_REQUIRE(d.k >= 1 && d.k <= d.r, "k must be in 1..r");
@@ -508,7 +510,7 @@ KoszulCtx* KoszulCtx::create(const bw_koszul_desc& d, int dev) {
 
     const size_t smem_fwd = static_cast<size_t>(c->r) * c->ci * ((c->co + 7) / 8 * 8) * sizeof(int32_t);
     const size_t smem_bwd = static_cast<size_t>(c->r) * c->co * ((c->ci + 7) / 8 * 8) * sizeof(int32_t);
-    BW_REQUIRE(smem_fwd <= 200 * 1024 && smem_bwd <= 200 * 1024,
+    BW_REQUIRE(smem_fwd <= kPlainMapBytes && smem_bwd <= kPlainMapBytes,
                "maps too large for shared memory staging (r * dim_in * dim_out * 4 > 200 KiB)");
 
     c->maps_canonical.assign(d.maps, d.maps + static_cast<size_t>(c->r) * c->co * c->ci);
@@ -593,11 +595,16 @@ void KoszulCtx::plain_coefficients(bool transpose_dir, int rows) {
 // Output rows a thread of each direction's gathers: 4, 8 or the even height
 // (5 to 7, see even_rows), timed at set-up on the context's own buffers (one
 // warm-up and two launches; the kernels' work does not depend on the values),
-// the fastest kept; BW_PLAIN_TILE=4 to =8 forces one height.
+// the fastest kept; BW_PLAIN_TILE=4 to =8 forces one height where it fits.
 void KoszulCtx::plain_setup() {
     int forced = 0;
     if (const char* e = std::getenv("BW_PLAIN_TILE")) forced = std::atoi(e);
-    if (forced >= 4 && forced <= 8) {
+    // (heights that are no multiple of four pad a tile's coefficients: a forced one may not fit)
+    auto fits = [&](int inner, int outer, int rows) {
+        return static_cast<size_t>(r) * inner * ((outer + rows - 1) / rows) * ((rows + 3) / 4 * 4) * sizeof(int32_t) <=
+               kPlainMapBytes;
+    };
+    if (forced >= 4 && forced <= 8 && fits(ci, co, forced) && fits(co, ci, forced)) {
         plain_coefficients(false, forced);
         plain_coefficients(true, forced);
         plain_plan = "plain: " + std::to_string(forced) + " output rows a thread (forced)";
